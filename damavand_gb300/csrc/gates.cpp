@@ -191,6 +191,100 @@ Op make_op(const PGate& g, int32_t target_pos, int32_t ctrl, int32_t ctrl_kind) 
 
 inline uint64_t qbit(int32_t q) { return q >= 0 ? (uint64_t(1) << q) : 0; }
 
+// Depth of a gate in its window: the number of non-exchange gates on the
+// longest chain of taken gates that ends with it. `depth` holds it per qubit.
+inline bool is_exchange(const PGate& g) { return g.m[2] == 1. && g.m[4] == 1. && classify(g.m) == OP_SWAP; }
+inline int32_t gate_depth(const PGate& g, const int32_t* depth) {
+  const int32_t d = g.control >= 0 ? std::max(depth[g.target], depth[g.control]) : depth[g.target];
+  return is_exchange(g) ? d : d + 1;
+}
+inline void raise_depth(const PGate& g, int32_t* depth) {
+  const int32_t d = gate_depth(g, depth);
+  depth[g.target] = d;
+  if (g.control >= 0) depth[g.control] = d;
+}
+
+struct Window {
+  uint64_t local;
+  int32_t max_depth;  // gates deeper than this stay for a later window
+};
+
+// The next window's local qubits. Without `search`: the `low` lowest qubits
+// and the first other targets met in the pending list. With it, that window
+// and every run of k - low consecutive qubits are tried, each with every
+// depth limit, and the one that does the most work per unit of its cost is
+// taken, in FP64 multiply-adds per amplitude: 2 per non-exchange gate (a
+// rotation), 3 per level of depth (each level of rotations has to apply the
+// diagonal factors left by the one before: one phase table), and kPassCost
+// for the pass itself (the state read and written once; about 2.5 in FP64 at
+// HBM's rate, far more where the arithmetic is faster). A deep window saves
+// passes and a shallow one phase tables, because a window's edge loses a
+// qubit per level: kPassCost 8 is near both optima. On the 28-qubit, 20-layer
+// ladder the search takes 78 passes (6 low qubits, first targets met: those
+// scatter the window over the qubits, where few gates meet) to 27 with 4 low
+// qubits. Measured forwards, before and after: 28 qubits in FP64 1041 and 879
+// ms, 26 in FP32 pairs 183 and 128 ms, 25 on the tensor cores 80 and 56 ms, 27
+// in complex64 67 and 62 ms. The search takes 2 ms of host time there.
+constexpr double kPassCost = 8.0;
+
+Window next_window(const std::vector<PGate>& fg, const std::vector<int64_t>& pending, int32_t n, int32_t k,
+                   int32_t low, bool search) {
+  Window first;
+  first.local = (uint64_t(1) << low) - 1;
+  first.max_depth = INT32_MAX;
+  int32_t nlocal = low;
+  for (int64_t gi : pending) {
+    if (nlocal >= k) break;
+    const int32_t t = fg[(size_t)gi].target;
+    if (!(first.local & qbit(t))) { first.local |= qbit(t); ++nlocal; }
+  }
+  for (int32_t q = 0; q < n && nlocal < k; ++q)
+    if (!(first.local & qbit(q))) { first.local |= qbit(q); ++nlocal; }
+  if (!search || k >= n) return first;
+
+  Window best = first;
+  double best_score = -1.0;
+  std::vector<int32_t> work, moves;  // non-exchange and exchange gates taken, per depth
+  for (int32_t a = low - 1; a + (k - low) <= n; ++a) {
+    const uint64_t run = ((uint64_t(1) << (k - low)) - 1) << a;
+    const uint64_t local = a < low ? first.local : (((uint64_t(1) << low) - 1) | run);
+    if (a >= low && local == first.local) continue;
+    work.assign(1, 0);
+    moves.assign(1, 0);
+    uint64_t blocked = 0;
+    int32_t depth[64] = {};
+    for (int64_t gi : pending) {
+      if (!(local & ~blocked)) break;  // every local qubit blocked
+      const PGate& g = fg[(size_t)gi];
+      const uint64_t qs = qbit(g.target) | qbit(g.control);
+      if ((qs & blocked) || !(local & qbit(g.target))) {
+        blocked |= qs;
+        continue;
+      }
+      const int32_t d = gate_depth(g, depth);
+      raise_depth(g, depth);
+      if ((size_t)d >= work.size()) {
+        work.resize((size_t)d + 1, 0);
+        moves.resize((size_t)d + 1, 0);
+      }
+      if (is_exchange(g)) ++moves[(size_t)d];
+      else ++work[(size_t)d];
+    }
+    double w = 0.0, x = 0.0;
+    for (size_t d = 0; d < work.size(); ++d) {
+      w += 2.0 * work[d];
+      x += 0.2 * moves[d];
+      const double score = (w + x) / (w + 3.0 * (double)d + kPassCost);
+      if (score > best_score && w + x > 0.0) {
+        best_score = score;
+        best.local = local;
+        best.max_depth = d + 1 == work.size() ? INT32_MAX : (int32_t)d;
+      }
+    }
+  }
+  return best;
+}
+
 }  // namespace
 
 int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
@@ -248,36 +342,31 @@ int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
   (void)precision;
 
   // 2. Qubit-window passes. Each pass keeps `k` qubits local to a tile: the
-  //    `low` lowest ones (contiguous chunks in HBM) and the first other
-  //    targets met in the pending list. A list-order sweep then takes every
-  //    gate whose target is local and none of whose qubits is blocked by an
-  //    earlier gate left pending; a gate left pending blocks its qubits.
+  //    `low` lowest ones (contiguous chunks in HBM) and others chosen by
+  //    next_window. A list-order sweep then takes every gate whose target is
+  //    local and none of whose qubits is blocked by an earlier gate left
+  //    pending; a gate left pending blocks its qubits.
   std::vector<int64_t> pending(fg.size());
   for (size_t i = 0; i < fg.size(); ++i) pending[i] = (int64_t)i;
   std::vector<int64_t> keep, take;
   while (!pending.empty()) {
-    uint64_t local = (uint64_t(1) << low) - 1;
-    int32_t nlocal = low;
-    for (int64_t gi : pending) {
-      if (nlocal >= k) break;
-      const int32_t t = fg[(size_t)gi].target;
-      if (!(local & qbit(t))) { local |= qbit(t); ++nlocal; }
-    }
-    for (int32_t q = 0; q < n && nlocal < k; ++q)
-      if (!(local & qbit(q))) { local |= qbit(q); ++nlocal; }
+    const Window win = next_window(fg, pending, n, k, low, opt.search_windows);
+    const uint64_t local = win.local;
 
     keep.clear();
     take.clear();
     uint64_t blocked = 0;
+    int32_t depth[64] = {};
     for (size_t idx = 0; idx < pending.size(); ++idx) {
       const int64_t gi = pending[idx];
       const PGate& g = fg[(size_t)gi];
       const uint64_t qs = qbit(g.target) | qbit(g.control);
       if (blocked == all_mask) { keep.insert(keep.end(), pending.begin() + (int64_t)idx, pending.end()); break; }
-      if ((qs & blocked) || !(local & qbit(g.target))) {
+      if ((qs & blocked) || !(local & qbit(g.target)) || gate_depth(g, depth) > win.max_depth) {
         blocked |= qs;
         keep.push_back(gi);
       } else {
+        raise_depth(g, depth);
         take.push_back(gi);
       }
     }

@@ -251,6 +251,7 @@ struct PlanOptions {
   int32_t fusion = DMV_FUSE_WINDOW;
   int32_t tile_bits = 12;  // log2 amplitudes per tile
   int32_t low_bits = 6;    // always-local low qubits (coalesced chunks)
+  bool search_windows = false;  // choose each window by a search (next_window) instead of the first targets met
   bool windows_only = false;  // every pass a window pass (the batched kernel runs only those)
   // Adjoint sweeps: when set, no gates are merged and the op made from
   // gates[i] carries param_of[i] / generator_of[i] (Op::param, Op::generator).
@@ -385,6 +386,8 @@ inline PlanOptions plan_options_for(const dmv_state_s* s, int32_t fusion) {
   PlanOptions opt;
   opt.fusion = fusion;
   opt.tile_bits = 12;
+  opt.low_bits = 4;  // a 128-byte row of complex64, two of complex128
+  opt.search_windows = true;
   return opt;
 }
 
