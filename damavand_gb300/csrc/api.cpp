@@ -423,6 +423,13 @@ extern "C" int dmv_state_destroy(dmv_state_t s) {
   s->amps = nullptr;
   s->ops_dev.release();
   s->phase_ops_dev.release();
+  s->phase_src_dev.release();
+  s->phase_tab_dev.release();
+  s->phase_tab2_dev.release();
+  s->fix_ops_dev.release();
+  s->phase_tab_fix_dev.release();
+  s->tc_stages_dev.release();
+  s->tc_u_dev.release();
   s->reduce_dev.release();
   s->chunk_dev.release();
   if (s->pinned) cudaFreeHost(s->pinned);

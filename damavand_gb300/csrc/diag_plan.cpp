@@ -11,9 +11,9 @@
 //    product is checked against U entry by entry; an op it does not
 //    reproduce to 4e-15 stays as it was. R acts on the real parts and the
 //    imaginary parts of a pair as the same real rotation, applied as f M with
-//    M = [[1, -w], [w, 1]] (w = tan t, f = cos t) when cos t >= sin t, else
-//    M = [[w, -1], [1, w]] (w = cot t, f = sin t): each output is one
-//    multiply-add, 2 per amplitude instead of 8. The kernels apply M only; the
+//    M = [[1, -w], [w, 1]] (w = tan t, f = cos t): each output is one
+//    multiply-add, 2 per amplitude instead of 8. For t > pi/4,
+//    R(t) = X R(pi/2 - t) Z with Z a diagonal factor and X an exchange. The kernels apply M only; the
 //    product of the factors f (each >= 1/sqrt 2) is multiplied back into the
 //    state once, by the caller (three shears, x0 += T x1, x1 += S x0,
 //    x0 += T x1, keep the norm but cost 3 multiply-adds per amplitude).
@@ -25,7 +25,11 @@
 //    factors collect into tables of one phase per amplitude, applied as one
 //    op ("flush") where a rotation needs a bit the pending table depends on,
 //    and at the end of the pass. A factor whose bits nothing has touched
-//    since the last table joins that table instead of the pending one. An
+//    since the last table joins that table instead of the pending one. A
+//    table is held as terms, an angle times the parity of a set of bits (an
+//    exchange maps each onto one again), and a kernel makes its entries
+//    (k_phase_tables): per amplitude on the host that took 5.8 ms of the
+//    24-qubit, 10-layer forward and 4 MB of upload, as terms 0.3 ms. An
 //    exchange controlled from outside the tile re-indexes only the tiles
 //    whose control bit is 1, so a table may depend on up to three global
 //    bits (then it holds 2^(k+g) phases and each tile reads its slice).
@@ -39,91 +43,99 @@
 #include <cmath>
 #include <algorithm>
 #include <cstring>
-#include <atomic>
-#include <thread>
 
 #include "internal.h"
 
 namespace dmv {
 namespace {
 
-constexpr double kTwoPi = 6.283185307179586476925286766559;
-constexpr double kHalfPi = 1.5707963267948966192313216916398;
 constexpr double kZyzTol = 4e-15;  // per entry, about 18 ulp of 1
 
-constexpr double kPi = 3.1415926535897932384626433832795;
+// 1 / (2 pi) as an unevaluated sum of two doubles.
+constexpr double kInvTwoPiHi = 0x1.45f306dc9c883p-3, kInvTwoPiLo = -0x1.6b01ec5417056p-57;
 
-inline double wrap(double a) { return std::remainder(a, kTwoPi); }
-
-// x + a reduced to [-pi, pi] for x, a in [-pi, pi] (every term angle is).
-inline double add_angle(double x, double a) {
-  x += a;
-  if (x > kPi) x -= kTwoPi;
-  else if (x < -kPi) x += kTwoPi;
-  return x;
+// The argument of re + i im as a fraction of a turn in units of 2^-64: sums
+// of them are exact and wrap by themselves. Taken from the nearest axis, so
+// that i^q is exactly q quarter turns and the rounding is that of an angle of
+// at most pi/4.
+int64_t arg_turns(double re, double im) {
+  uint64_t q = 0;
+  double x = re, y = im;
+  if (std::fabs(im) > std::fabs(re)) {  // i^-1 (re + i im)
+    x = im;
+    y = -re;
+    q = 1;
+  }
+  if (x < 0.0) {
+    x = -x;
+    y = -y;
+    q += 2;
+  }
+  const double a = std::atan2(y, x);
+  const double p = a * kInvTwoPiHi;
+  const double e = std::fma(a, kInvTwoPiHi, -p) + a * kInvTwoPiLo;
+  return (int64_t)((q << 62) + (uint64_t)(int64_t)std::ldexp(p, 64) + (uint64_t)(int64_t)std::llrint(std::ldexp(e, 64)));
 }
+constexpr int64_t kHalfTurn = INT64_MIN;
+
+inline int64_t add_turns(int64_t a, int64_t b) { return (int64_t)((uint64_t)a + (uint64_t)b); }
+inline int64_t sub_turns(int64_t a, int64_t b) { return (int64_t)((uint64_t)a - (uint64_t)b); }
 
 // A diagonal phase over the tile (2^k amplitudes) and up to kMaxPhaseGlobals
-// global bits: angle of amplitude l on tiles with global-bit pattern gsel at
-// index (gsel << k) | l.
+// global bits, as parity terms: the angle of amplitude l is c plus every
+// term's turn whose mask meets an odd number of set bits.
 struct DiagTable {
   int g = 0;
   int gq[kMaxPhaseGlobals] = {0, 0, 0};
   uint32_t supp = 0;  // local bits it depends on
   bool used = false;
-  std::vector<double> ang;
-  void reset(int T) {
+  int64_t c = 0;
+  std::vector<PhaseTerm> terms;
+  void reset() {
     g = 0;
     supp = 0;
     used = false;
-    ang.assign((size_t)T, 0.0);
+    c = 0;
+    terms.clear();
+  }
+  void add(uint32_t mask, int64_t turn) {
+    for (PhaseTerm& t : terms)
+      if (t.mask == mask) {
+        t.turn = add_turns(t.turn, turn);
+        return;
+      }
+    terms.push_back(PhaseTerm{mask, 0u, turn});
   }
 };
 
-// Adds the phase f(l) of one diagonal factor (local bits only, |f| <= pi) to every slice.
-template <typename F>
-void add_term(DiagTable& d, int k, uint32_t bits, F f) {
-  const size_t T = size_t(1) << k;
-  double* a = d.ang.data();
-  for (size_t idx = 0; idx < d.ang.size(); ++idx) {
-    const double v = f((uint32_t)(idx & (T - 1)));
-    if (v != 0.0) a[idx] = add_angle(a[idx], v);
-  }
-  d.supp |= bits;
+// A factor on one bit t: angle p0 where the bit is clear, p1 where it is set.
+void add_bit_term(DiagTable& d, int t, int64_t p0, int64_t p1) {
+  d.c = add_turns(d.c, p0);
+  d.add(1u << t, sub_turns(p1, p0));
+  d.supp |= 1u << t;
   d.used = true;
 }
 
-// The same for a factor on one bit t: p0 where the bit is clear, p1 where it is set.
-void add_bit_term(DiagTable& d, int t, double p0, double p1) {
-  const size_t n = d.ang.size(), tb = size_t(1) << t;
-  double* a = d.ang.data();
-  for (size_t base = 0; base < n; base += 2 * tb) {
-    if (p0 != 0.0)
-      for (size_t i = base; i < base + tb; ++i) a[i] = add_angle(a[i], p0);
-    if (p1 != 0.0)
-      for (size_t i = base + tb; i < base + 2 * tb; ++i) a[i] = add_angle(a[i], p1);
-  }
-  d.supp |= 1u << t;
+// A factor on bit t where bit ctrl is set: with h half the difference,
+// (p1 - p0) ctrl t = h ctrl + h t - h (ctrl xor t).
+void add_controlled_term(DiagTable& d, int ctrl, int t, int64_t p0, int64_t p1) {
+  const int64_t h = sub_turns(p1, p0) >> 1;
+  d.add(1u << ctrl, add_turns(p0, h));
+  d.add(1u << t, h);
+  d.add((1u << ctrl) | (1u << t), sub_turns(0, h));
+  d.supp |= (1u << ctrl) | (1u << t);
   d.used = true;
 }
 
 // D o P for the exchange `op` (X or CNOT on tile bit op.target). Returns false,
 // changing nothing, when the table would need a fourth global bit.
-bool permute(DiagTable& d, int k, const Op& op) {
+bool permute(DiagTable& d, const Op& op) {
   const uint32_t tb = 1u << op.target;
   if (!(d.supp & tb)) return true;  // does not depend on the target: unchanged
-  // the exchange is an involution: swap the entries of each pair it maps onto each other
-  double* a = d.ang.data();
-  const size_t n = d.ang.size();
-  if (op.ctrl_kind == CTRL_NONE) {
-    for (size_t idx = 0; idx < n; ++idx)
-      if (!(idx & tb)) std::swap(a[idx], a[idx | tb]);
-  } else if (op.ctrl_kind == CTRL_LOCAL) {
-    const size_t cb = size_t(1) << op.ctrl;
-    for (size_t idx = 0; idx < n; ++idx)
-      if (!(idx & tb) && (idx & cb)) std::swap(a[idx], a[idx | tb]);
-    d.supp |= 1u << op.ctrl;
-  } else {
+  uint32_t flip = 0;  // P adds this bit's value to the target's
+  if (op.ctrl_kind == CTRL_LOCAL) {
+    flip = 1u << op.ctrl;
+  } else if (op.ctrl_kind == CTRL_GLOBAL) {
     int j = -1;
     for (int i = 0; i < d.g; ++i)
       if (d.gq[i] == op.ctrl) j = i;
@@ -131,14 +143,26 @@ bool permute(DiagTable& d, int k, const Op& op) {
       if (d.g == kMaxPhaseGlobals) return false;
       j = d.g++;
       d.gq[j] = op.ctrl;
-      const size_t old = d.ang.size();
-      d.ang.resize(old * 2);
-      std::memcpy(d.ang.data() + old, d.ang.data(), old * sizeof(double));
     }
-    a = d.ang.data();
-    const size_t on = size_t(1) << (k + j);
-    for (size_t idx = 0; idx < d.ang.size(); ++idx)
-      if ((idx & on) && !(idx & tb)) std::swap(a[idx], a[idx | tb]);
+    flip = 1u << (kPhaseGlobalBit + j);
+  }
+  for (PhaseTerm& t : d.terms) {
+    if (!(t.mask & tb)) continue;
+    if (op.ctrl_kind == CTRL_NONE) {  // the parity is complemented
+      d.c = add_turns(d.c, t.turn);
+      t.turn = sub_turns(0, t.turn);
+    } else {
+      t.mask ^= flip;
+    }
+  }
+  // terms whose masks became equal are one term
+  std::vector<PhaseTerm> old;
+  old.swap(d.terms);
+  d.supp = 0;
+  for (const PhaseTerm& t : old) {
+    if (t.turn == 0) continue;
+    d.add(t.mask, t.turn);
+    d.supp |= t.mask & ((1u << kPhaseGlobalBit) - 1u);
   }
   return true;
 }
@@ -147,7 +171,7 @@ inline double cabs(double re, double im) { return std::hypot(re, im); }
 
 // U = D1 R D2 (see the file comment). Returns false when the product does not
 // reproduce U to kZyzTol in every entry.
-bool zyz(const double m[8], double& T, double& S, double& C, double& a1, double& a2, double& g2) {
+bool zyz(const double m[8], double& T, double& S, double& C, int64_t& t1, int64_t& t2, int64_t& tg) {
   const double ra = cabs(m[0], m[1]), rb = cabs(m[2], m[3]);
   // c and s each rounded once from a wider quotient: dividing both by one
   // rounded double r biased c^2 + s^2 (by about 3e-17 per rotation on the
@@ -155,15 +179,17 @@ bool zyz(const double m[8], double& T, double& S, double& C, double& a1, double&
   const long double rl = std::hypot((long double)ra, (long double)rb);
   if (!(rl > 0.0L)) return false;
   const double c = (double)((long double)ra / rl), s = (double)((long double)rb / rl);
-  a1 = std::atan2(m[1], m[0]);
-  a2 = std::atan2(m[5], m[4]);
-  g2 = wrap(std::atan2(m[3], m[2]) + M_PI - a1);
+  const double a1 = std::atan2(m[1], m[0]), a2 = std::atan2(m[5], m[4]);
+  const double g2 = std::atan2(m[3], m[2]) + M_PI - a1;
   const double e[8] = {c * std::cos(a1),        c * std::sin(a1),
                        -s * std::cos(a1 + g2),  -s * std::sin(a1 + g2),
                        s * std::cos(a2),        s * std::sin(a2),
                        c * std::cos(a2 + g2),   c * std::sin(a2 + g2)};
   for (int i = 0; i < 8; ++i)
     if (!(std::fabs(e[i] - m[i]) <= kZyzTol)) return false;
+  t1 = arg_turns(m[0], m[1]);
+  t2 = arg_turns(m[4], m[5]);
+  tg = sub_turns(add_turns(arg_turns(m[2], m[3]), kHalfTurn), t1);
   T = -s / (1.0 + c);  // -tan(t/2), t = atan2(s, c) in [0, pi/2]
   S = s;
   C = c;
@@ -173,11 +199,10 @@ bool zyz(const double m[8], double& T, double& S, double& C, double& a1, double&
 // |z| = 1 to kZyzTol: a diagonal entry that is a pure phase.
 inline bool unit(double re, double im) { return std::fabs(cabs(re, im) - 1.0) <= kZyzTol; }
 
-PhaseEntry entry_of(double phi) {
+PhaseEntry entry_of(int64_t turn) {
   // phi = q pi/2 + phi', |phi'| <= pi/4
-  const double qf = std::nearbyint(phi / kHalfPi);
-  const double p = phi - qf * kHalfPi;
-  const int q = (((int)qf % 4) + 4) % 4;
+  const uint64_t q = ((uint64_t)turn + (uint64_t(1) << 61)) >> 62;
+  const double p = (double)(int64_t)((uint64_t)turn - (q << 62)) * (M_PI * 0x1p-63);
   PhaseEntry e;
   double sh, ch;
   sincos(0.5 * p, &sh, &ch);  // t = -tan(p/2), s = sin p = 2 sin(p/2) cos(p/2)
@@ -219,40 +244,31 @@ void phase_entry_value(const PhaseEntry& e, double& re, double& im) {
   }
 }
 
-void phase_tables_df(const std::vector<PhaseEntry>& in, std::vector<float4>& out) {
-  out.resize(in.size());
-  for (size_t i = 0; i < in.size(); ++i) {
-    double re, im;
-    phase_entry_value(in[i], re, im);
-    const float rh = (float)re, ih = (float)im;
-    out[i] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
-  }
+void phase_entries(const PhaseTables& tabs, std::vector<PhaseEntry>& out) {
+  out.resize((size_t)tabs.entries);
+  for (const PhaseTable& d : tabs.tables)
+    for (uint32_t i = 0; i < (1u << (d.k + d.g)); ++i) {
+      const uint32_t at = (i & ((1u << d.k) - 1u)) | (i >> d.k) << kPhaseGlobalBit;
+      int64_t a = d.c;
+      for (int32_t j = 0; j < d.num_terms; ++j) {
+        const PhaseTerm& t = tabs.terms[(size_t)(d.first_term + j)];
+        if (__builtin_parity(t.mask & at)) a = add_turns(a, t.turn);
+      }
+      out[(size_t)d.entry + i] = entry_of(a);
+    }
 }
 
 void rewrite_passes(const Plan& plan, const std::vector<int64_t>& which, bool rot_ops,
                     std::vector<RewrittenPass>& out) {
   out.assign(which.size(), RewrittenPass());
-  auto work = [&](size_t j) {
+  for (size_t j = 0; j < which.size(); ++j) {
     const Pass& ps = plan.passes[(size_t)which[j]];
     rewrite_pass_rotations(plan.ops.data() + ps.op_begin, ps.op_count, ps.low_bits + ps.num_high, rot_ops,
                            out[j].ops, out[j].tab, &out[j].scale);
-  };
-  const size_t nt = std::min<size_t>(std::min<size_t>(std::max(1u, std::thread::hardware_concurrency()), 16),
-                                     which.size());
-  if (nt <= 1) {
-    for (size_t j = 0; j < which.size(); ++j) work(j);
-    return;
   }
-  std::atomic<size_t> next{0};
-  std::vector<std::thread> pool;
-  pool.reserve(nt);
-  for (size_t t = 0; t < nt; ++t)
-    pool.emplace_back([&]() {
-      for (size_t j = next.fetch_add(1); j < which.size(); j = next.fetch_add(1)) work(j);
-    });
-  for (std::thread& th : pool) th.join();
 }
 
+// The FP64 kernels' form of the entries, as k_phase_tables writes it.
 void phase_tables_f64(const std::vector<PhaseEntry>& in, std::vector<double2>& out) {
   out.resize(in.size());
   for (size_t i = 0; i < in.size(); ++i) {
@@ -272,26 +288,14 @@ void phase_tables_f64(const std::vector<PhaseEntry>& in, std::vector<double2>& o
   }
 }
 
-void phase_tables_fx(const std::vector<PhaseEntry>& in, std::vector<int4>& out) {
-  out.resize(in.size());
-  for (size_t i = 0; i < in.size(); ++i) {
-    double re, im;
-    phase_entry_value(in[i], re, im);
-    const long long fr = std::llround(std::ldexp(re, 54)), fi = std::llround(std::ldexp(im, 54));
-    out[i] = make_int4((int)(fr >> 31), (int)(fr & 0x7FFFFFFFll), (int)(fi >> 31), (int)(fi & 0x7FFFFFFFll));
-  }
-}
-
 int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot_ops, std::vector<Op>& dst,
-                               std::vector<PhaseEntry>& tab, ScaleDD* scale) {
-  const int T = 1 << k;
+                               PhaseTables& tab, ScaleDD* scale) {
   std::vector<DiagTable> tables;  // flushes in time order; tables[0] may sit at the pass start
   bool start_table = false;
   std::vector<Item> items;
   int last = -1;          // table the next factor may join, -1: none yet
   uint32_t touched = 0;   // target bits of the ops emitted after `last` (after the pass start if none)
   DiagTable pend;
-  pend.reset(T);
   ScaleDD acc;  // OP_ROT factors not yet in the state (rot_ops)
 
   auto flush = [&]() {
@@ -300,71 +304,71 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
     items.push_back(Item{true, (int)tables.size() - 1, Op()});
     last = (int)tables.size() - 1;
     touched = 0;
-    pend.reset(T);
+    pend.reset();
   };
-  // A diagonal factor on `bits` with phase f(l): into the last table when
-  // nothing emitted since touches its bits, else pending.
-  auto diag = [&](uint32_t bits, auto f) {
-    if (!(bits & touched)) {
-      if (last < 0) {
-        DiagTable d;
-        d.reset(T);
-        tables.insert(tables.begin(), d);
-        for (Item& it : items)
-          if (it.flush) ++it.table;
-        start_table = true;
-        last = 0;
-      }
-      add_term(tables[(size_t)last], k, bits, f);
-    } else {
-      add_term(pend, k, bits, f);
+  // Where a diagonal factor on `bits` goes: the last table when nothing emitted
+  // since touches its bits, else the pending one.
+  auto home = [&](uint32_t bits) {
+    if (bits & touched) return &pend;
+    if (last < 0) {
+      tables.insert(tables.begin(), DiagTable());
+      for (Item& it : items)
+        if (it.flush) ++it.table;
+      start_table = true;
+      last = 0;
     }
-  };
-  // The same for a factor on one bit t (p0 where clear, p1 where set).
-  auto diag_bit = [&](int t, double p0, double p1) {
-    const uint32_t bits = 1u << t;
-    if (!(bits & touched)) {
-      if (last < 0) {
-        DiagTable d;
-        d.reset(T);
-        tables.insert(tables.begin(), d);
-        start_table = true;
-        last = 0;
-      }
-      add_bit_term(tables[(size_t)last], t, p0, p1);
-    } else {
-      add_bit_term(pend, t, p0, p1);
-    }
+    return &tables[(size_t)last];
   };
   auto emit = [&](const Op& op) {
     items.push_back(Item{false, -1, op});
     touched |= 1u << op.target;
   };
 
+  // An uncontrolled exchange, after the pending factors have moved past it.
+  auto emit_x = [&](int t) {
+    Op x = blank_op();
+    x.cls = OP_SWAP;
+    x.target = t;
+    x.ctrl = -1;
+    x.ctrl_kind = CTRL_NONE;
+    x.m[2] = 1.0;
+    x.m[4] = 1.0;
+    permute(pend, x);  // never needs another global bit
+    emit(x);
+  };
+
   for (int64_t i = 0; i < count; ++i) {
     const Op& op = src[i];
     const uint32_t tb = 1u << op.target;
     if (op.cls == OP_SWAP) {
-      if (!permute(pend, k, op)) {
+      if (!permute(pend, op)) {
         flush();
-        permute(pend, k, op);
+        permute(pend, op);
       }
       emit(op);
       continue;
     }
     if (op.unitary && op.ctrl_kind == CTRL_NONE &&
         (op.cls == OP_GENERAL || op.cls == OP_REAL || op.cls == OP_RXLIKE)) {
-      double Tq, Sq, Cq, a1, a2, g2;
+      double Tq, Sq, Cq;
+      int64_t a1, a2, g2;
       if (zyz(op.m, Tq, Sq, Cq, a1, a2, g2)) {
         const int t = op.target;
-        if (g2 != 0.0) diag_bit(t, 0.0, g2);  // D2
+        // FP64: t > pi/4 as R(t) = X R(pi/2 - t) Z, so every rotation has
+        // tan t <= 1; Z joins D2 and X is an exchange.
+        const bool flip = rot_ops && Cq < Sq;
+        if (flip) {
+          std::swap(Cq, Sq);
+          g2 = add_turns(g2, kHalfTurn);
+        }
+        if (g2 != 0) add_bit_term(*home(tb), t, 0, g2);  // D2
         if (pend.supp & tb) flush();
         Op r = blank_op();
         r.target = t;
         r.ctrl = -1;
         r.ctrl_kind = CTRL_NONE;
         if (rot_ops) {
-          // R = f M with one entry pair of M exactly 1: two multiply-adds per
+          // R = f M with M's diagonal exactly 1: two multiply-adds per
           // component instead of three shears; f (>= 1/sqrt 2) goes to *scale.
           // f = 1 / sqrt(1 + w^2), rounded once from a wider result, so that
           // f M is orthogonal to within that rounding (no norm drift).
@@ -373,23 +377,21 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
           // as the real 2x2 acc f M instead (8 multiply-adds per pair), which
           // gives the state its true scale back.
           (void)Tq;
-          const bool form_b = Cq < Sq;
-          const double w = form_b ? Cq / Sq : Sq / Cq;
+          const double w = Sq / Cq;
           const long double wl = w;
           const double f = (double)(1.0L / std::sqrt(1.0L + wl * wl));
           if (acc.hi * f >= 0x1p-200) {
             r.cls = OP_ROT;
             r.m[0] = w;
-            r.m[1] = form_b ? 1.0 : 0.0;
             acc.mul(f);
           } else {
             const long double F = ((long double)acc.hi + (long double)acc.lo) * (long double)f;
             const double one = (double)F, ww = (double)(F * wl);
             r.cls = OP_REAL;
-            r.m[0] = form_b ? ww : one;
-            r.m[2] = form_b ? -one : -ww;
-            r.m[4] = form_b ? one : ww;
-            r.m[6] = form_b ? ww : one;
+            r.m[0] = one;
+            r.m[2] = -ww;
+            r.m[4] = ww;
+            r.m[6] = one;
             acc = ScaleDD();
           }
         } else {  // the rotation as a real 2x2 in the arithmetic's own form
@@ -401,6 +403,7 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
           split_matrix(r);
         }
         emit(r);
+        if (flip) emit_x(t);
         // D1: after the rotation on its own bit, so it cannot join an earlier table
         add_bit_term(pend, t, a1, a2);
         continue;
@@ -409,33 +412,18 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
     if (op.unitary && op.cls == OP_DIAG && unit(op.m[0], op.m[1]) && unit(op.m[6], op.m[7]) &&
         op.ctrl_kind != CTRL_GLOBAL) {
       const int t = op.target;
-      const double p0 = std::atan2(op.m[1], op.m[0]), p1 = std::atan2(op.m[7], op.m[6]);
-      if (op.ctrl_kind == CTRL_NONE) {
-        diag_bit(t, p0, p1);
-      } else {
-        const int c = op.ctrl;
-        diag(tb | (1u << c), [=](uint32_t l) { return ((l >> c) & 1u) ? (((l >> t) & 1u) ? p1 : p0) : 0.0; });
-      }
+      const int64_t p0 = arg_turns(op.m[0], op.m[1]), p1 = arg_turns(op.m[6], op.m[7]);
+      if (op.ctrl_kind == CTRL_NONE) add_bit_term(*home(tb), t, p0, p1);
+      else add_controlled_term(*home(tb | (1u << op.ctrl)), op.ctrl, t, p0, p1);
       continue;
     }
     if (op.unitary && op.cls == OP_ANTI && op.ctrl_kind == CTRL_NONE && unit(op.m[2], op.m[3]) &&
         unit(op.m[4], op.m[5])) {
       // [[0, b], [c, 0]] = X diag(c, b)
       const int t = op.target;
-      const double pc = std::atan2(op.m[5], op.m[4]), pb = std::atan2(op.m[3], op.m[2]);
-      diag_bit(t, pc, pb);
-      Op x = blank_op();
-      x.cls = OP_SWAP;
-      x.target = t;
-      x.ctrl = -1;
-      x.ctrl_kind = CTRL_NONE;
-      x.m[2] = 1.0;
-      x.m[4] = 1.0;
-      if (!permute(pend, k, x)) {
-        flush();
-        permute(pend, k, x);
-      }
-      emit(x);
+      const int64_t pc = arg_turns(op.m[4], op.m[5]), pb = arg_turns(op.m[2], op.m[3]);
+      add_bit_term(*home(tb), t, pc, pb);
+      emit_x(t);
       continue;
     }
     // Anything else runs as it is, after the pending factors on its target.
@@ -446,23 +434,27 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
 
   const int64_t before = (int64_t)dst.size();
   auto put_table = [&](const DiagTable& d) {
-    bool trivial = true;
-    for (double a : d.ang)
-      if (a != 0.0) {
-        trivial = false;
-        break;
-      }
-    if (trivial) return;
+    PhaseTable pt;
+    pt.entry = tab.entries;
+    pt.c = d.c;
+    pt.first_term = (int32_t)tab.terms.size();
+    pt.g = d.g;
+    pt.k = k;
+    for (const PhaseTerm& t : d.terms)
+      if (t.turn != 0) tab.terms.push_back(t);
+    pt.num_terms = (int32_t)tab.terms.size() - pt.first_term;
+    if (pt.num_terms == 0 && d.c == 0) return;  // the identity
+    tab.tables.push_back(pt);
+    tab.entries += int64_t(1) << (k + d.g);
     Op p = blank_op();
     p.cls = OP_PHASE;
     p.target = 0;
     p.ctrl = -1;
     p.ctrl_kind = CTRL_NONE;
-    p.fh[0] = (int32_t)tab.size();
+    p.fh[0] = (int32_t)pt.entry;
     p.fh[1] = d.g;
     for (int j = 0; j < d.g; ++j) p.fh[2 + j] = d.gq[j];
-    if (tab.capacity() < tab.size() + d.ang.size()) tab.reserve(2 * (tab.size() + d.ang.size()));
-    for (double a : d.ang) tab.push_back(entry_of(a));
+    p.fh[5] = (int32_t)d.supp;
     dst.push_back(p);
   };
   if (start_table) put_table(tables[0]);
@@ -544,13 +536,8 @@ void host_op(std::vector<Cx>& tile, int k, const Op& op, const std::vector<Phase
     if (op.cls == OP_ROT) {
       const double w = op.m[0];
       const double x0 = a0.re, x1 = a1.re, y0 = a0.im, y1 = a1.im;
-      if (op.m[1] == 0.0) {
-        tile[l0] = Cx{std::fma(-w, x1, x0), std::fma(-w, y1, y0)};
-        tile[l1] = Cx{std::fma(w, x0, x1), std::fma(w, y0, y1)};
-      } else {
-        tile[l0] = Cx{std::fma(w, x0, -x1), std::fma(w, y0, -y1)};
-        tile[l1] = Cx{std::fma(w, x1, x0), std::fma(w, y1, y0)};
-      }
+      tile[l0] = Cx{std::fma(-w, x1, x0), std::fma(-w, y1, y0)};
+      tile[l1] = Cx{std::fma(w, x0, x1), std::fma(w, y0, y1)};
     } else {
       const double* m = op.m;
       tile[l0] = Cx{m[0] * a0.re - m[1] * a0.im + m[2] * a1.re - m[3] * a1.im,
@@ -586,14 +573,14 @@ extern "C" int dmv_debug_check_fp64_rewrite(const dmv_gate_t* gates, int64_t num
   };
   double worst = 0.0;
   int64_t n_rot = 0, n_phase = 0, n_general = 0, n_passes = 0;
-  // the threaded rewrite (what launch_plan runs) must give every pass exactly
-  // the sequential result
+  // rewrite_passes (what launch_plan runs) must give every pass exactly what
+  // the pass gives alone
   std::vector<int64_t> which;
   for (size_t i = 0; i < plan.passes.size(); ++i)
     if (plan.passes[i].kind == 1) which.push_back((int64_t)i);
-  std::vector<RewrittenPass> threaded[2];
-  rewrite_passes(plan, which, true, threaded[0]);
-  rewrite_passes(plan, which, false, threaded[1]);
+  std::vector<RewrittenPass> together[2];
+  rewrite_passes(plan, which, true, together[0]);
+  rewrite_passes(plan, which, false, together[1]);
   size_t wi = 0;
   for (const Pass& ps : plan.passes) {
     if (ps.kind != 1) continue;
@@ -601,22 +588,25 @@ extern "C" int dmv_debug_check_fp64_rewrite(const dmv_gate_t* gates, int64_t num
     const int k = ps.low_bits + ps.num_high;
     for (int form = 0; form < 2; ++form) {
       std::vector<Op> rw;
-      std::vector<PhaseEntry> tab;
+      PhaseTables tab;
       ScaleDD scale;
       rewrite_pass_rotations(plan.ops.data() + ps.op_begin, ps.op_count, k, form == 0, rw, tab, &scale);
-      const RewrittenPass& t = threaded[form][j];
-      if (t.ops.size() != rw.size() || t.tab.size() != tab.size() || t.scale.hi != scale.hi ||
-          t.scale.lo != scale.lo || (!rw.empty() && std::memcmp(t.ops.data(), rw.data(), rw.size() * sizeof(Op))) ||
-          (!tab.empty() && std::memcmp(t.tab.data(), tab.data(), tab.size() * sizeof(PhaseEntry))))
-        return set_error(DMV_ERR_INVALID, "threaded rewrite of pass %zu differs from the sequential one", j);
+      const RewrittenPass& t = together[form][j];
+      if (t.ops.size() != rw.size() || t.tab.entries != tab.entries || t.tab.terms.size() != tab.terms.size() ||
+          t.scale.hi != scale.hi || t.scale.lo != scale.lo ||
+          (!rw.empty() && std::memcmp(t.ops.data(), rw.data(), rw.size() * sizeof(Op))) ||
+          (!tab.terms.empty() && std::memcmp(t.tab.terms.data(), tab.terms.data(), tab.terms.size() * sizeof(PhaseTerm))))
+        return set_error(DMV_ERR_INVALID, "the plan's rewrite of pass %zu differs from the pass rewritten alone", j);
     }
     if (k != 12 || ps.num_high < 3) continue;
     ++n_passes;
     for (int form = 0; form < 2; ++form) {  // rotations as OP_ROT (FP64), then as real 2x2 ops
     std::vector<Op> rw;
+    PhaseTables tabs;
     std::vector<PhaseEntry> tab;
     ScaleDD scale;
-    rewrite_pass_rotations(plan.ops.data() + ps.op_begin, ps.op_count, k, form == 0, rw, tab, &scale);
+    rewrite_pass_rotations(plan.ops.data() + ps.op_begin, ps.op_count, k, form == 0, rw, tabs, &scale);
+    phase_entries(tabs, tab);
     std::vector<double2> packed;
     phase_tables_f64(tab, packed);
     if (form == 0)

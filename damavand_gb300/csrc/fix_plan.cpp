@@ -1,0 +1,229 @@
+// Fixed-point window passes (host C++): a rewritten pass's ops scheduled into
+// register phases (fix_window.cuh has the kernel).
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "internal.h"
+
+namespace dmv {
+namespace {
+
+constexpr int kFixTileBits = 12;
+constexpr int kFixRegBits = 4;
+
+// The linear map l -> fix_slot(A l): images of the tile bits.
+struct SlotMap {
+  int32_t img[kFixTileBits];
+};
+
+int rank3(const int32_t* v, int n) {
+  int32_t basis[3] = {0, 0, 0};
+  int r = 0;
+  for (int i = 0; i < n; ++i) {
+    int32_t x = v[i] & 7;
+    for (int b = 2; b >= 0; --b)
+      if ((x >> b) & 1) {
+        if (basis[b]) x ^= basis[b];
+        else {
+          basis[b] = x;
+          ++r;
+          break;
+        }
+      }
+  }
+  return r;
+}
+
+void pack_images(FixOp& op, const int32_t* slot12) {
+  for (int i = 0; i < 6; ++i) op.a[i] = slot12[2 * i] | (slot12[2 * i + 1] << 16);
+}
+
+// Thread bits of a phase: the tile bits outside `regs`, the first three chosen
+// so that eight consecutive lanes' 16-byte accesses meet all 32 banks (their
+// slots differ in three independent ways modulo 8), low bits first: those also
+// read consecutive table entries.
+void thread_bits(const SlotMap& m, uint32_t regs, int32_t* bits) {
+  int n = 0;
+  uint32_t used = regs;
+  int32_t pick[3];
+  for (int b = 0; b < kFixTileBits && n < 3; ++b) {
+    if ((used >> b) & 1u) continue;
+    pick[n] = m.img[b];
+    if (rank3(pick, n + 1) != n + 1) continue;
+    bits[n++] = b;
+    used |= 1u << b;
+  }
+  for (int b = 0; b < kFixTileBits; ++b)
+    if (!((used >> b) & 1u)) bits[n++] = b;
+}
+
+// w 2^64 as signed words hi 2^32 + lo; false when hi would not fit 31 bits
+// (w within 2^-32 of 1/2 from below, or w >= 1/2).
+bool split_multiplier(double w, int32_t& hi, int32_t& lo) {
+  if (!(w >= 0.0) || w >= 0.5) return false;
+  const uint64_t W = (uint64_t)std::nearbyint(std::ldexp(w, 64));
+  const uint64_t h = (W >> 32) + ((W >> 31) & 1u);
+  if (h >= 0x80000000ull) return false;
+  hi = (int32_t)h;
+  lo = (int32_t)(uint32_t)W;
+  return true;
+}
+
+}  // namespace
+
+bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32_t* shifts) {
+  const size_t mark = out.size();
+  *shifts = 0;
+  SlotMap m;
+  for (int b = 0; b < kFixTileBits; ++b) m.img[b] = fix_slot_host(1 << b);
+  auto blank = [](int32_t kind) {
+    FixOp f;
+    std::memset(&f, 0, sizeof(f));
+    f.kind = kind;
+    return f;
+  };
+  int32_t flip = 0;  // offset the next FIX_PHASE or FIX_END adds on every tile
+  // An exchange takes effect at the front of the phase being built.
+  auto exchange = [&](const Op& op) {
+    if (op.ctrl_kind == CTRL_LOCAL) {
+      m.img[op.ctrl] ^= m.img[op.target];
+      return;
+    }
+    if (op.ctrl_kind == CTRL_NONE) {
+      flip ^= m.img[op.target];
+      return;
+    }
+    FixOp f = blank(FIX_XOR);
+    f.a[0] = op.ctrl;
+    f.a[1] = m.img[op.target];
+    out.push_back(f);
+  };
+  // The stored state is the true one times `grown`, kept in (1/sqrt 2, sqrt 2].
+  double grown = 1.0;
+  std::vector<char> done((size_t)count, 0);
+  std::vector<FixOp> taken;
+  int64_t left = count, first = 0;
+  while (left > 0) {
+    while (done[(size_t)first]) ++first;
+    int32_t reg[kFixRegBits];
+    int nr = 0;
+    uint32_t regs = 0, blocked = 0, used = 0;
+    taken.clear();
+    for (int64_t i = first; i < count && blocked != 0xfffu; ++i) {
+      if (done[(size_t)i]) continue;
+      const Op& op = ops[i];
+      const uint32_t tb = 1u << op.target;
+      if (op.cls == OP_SWAP) {
+        const uint32_t qs = tb | (op.ctrl_kind == CTRL_LOCAL ? 1u << op.ctrl : 0u);
+        if (qs & (blocked | used)) {
+          blocked |= qs;
+          continue;
+        }
+        exchange(op);
+      } else if (op.cls == OP_PHASE) {
+        const uint32_t qs = (uint32_t)op.fh[5];
+        if (qs & blocked) {
+          blocked |= qs;
+          continue;
+        }
+        FixOp f = blank(FIX_TABLE);
+        f.a[0] = op.fh[0];
+        f.a[1] = op.fh[1];
+        for (int j = 0; j < op.fh[1]; ++j) f.a[2 + j] = op.fh[2 + j];
+        used |= qs;
+        taken.push_back(f);
+      } else if (op.cls == OP_ROT && op.ctrl_kind == CTRL_NONE) {
+        if (tb & blocked) continue;
+        if (!(regs & tb)) {
+          if (nr == kFixRegBits) {
+            blocked |= tb;
+            continue;
+          }
+          reg[nr++] = op.target;
+          regs |= tb;
+        }
+        used |= tb;
+        FixOp f = blank(FIX_ROT);
+        f.a[0] = op.target;  // the register bit once the phase is complete
+        const double w = op.m[0];
+        if (!split_multiplier(w, f.a[1], f.a[2])) {
+          f.a[0] |= kFixComplement << 8;
+          if (!split_multiplier(1.0 - w, f.a[1], f.a[2])) {
+            out.resize(mark);
+            return false;
+          }
+        }
+        grown *= std::sqrt(1.0 + w * w);
+        if (grown > 1.4142135623730951) {
+          f.a[0] |= kFixShift << 8;
+          grown *= 0.5;
+          ++*shifts;
+        }
+        taken.push_back(f);
+      } else {
+        out.resize(mark);
+        return false;
+      }
+      done[(size_t)i] = 1;
+      --left;
+    }
+    if (taken.empty()) continue;
+    // unused register bits from the top: the low ones serve the lanes
+    for (int b = kFixTileBits - 1; nr < kFixRegBits; --b)
+      if (!((regs >> b) & 1u)) {
+        reg[nr++] = b;
+        regs |= 1u << b;
+      }
+    int32_t tbits[8], slots[12];
+    thread_bits(m, regs, tbits);
+    FixOp ph = blank(FIX_PHASE);
+    for (int i = 0; i < kFixRegBits; ++i) slots[i] = m.img[reg[i]];
+    for (int i = 0; i < 8; ++i) slots[kFixRegBits + i] = m.img[tbits[i]];
+    pack_images(ph, slots);
+    uint32_t tpos = 0, rpos = 0;
+    for (int i = 0; i < 8; ++i) tpos |= (uint32_t)tbits[i] << (4 * i);
+    for (int i = 0; i < kFixRegBits; ++i) rpos |= (uint32_t)reg[i] << (4 * i);
+    ph.a[6] = (int32_t)tpos;
+    ph.a[7] = (int32_t)rpos;
+    ph.a[8] = flip;
+    flip = 0;
+    out.push_back(ph);
+    for (FixOp& f : taken) {
+      if (f.kind == FIX_ROT) {
+        const int32_t t = f.a[0] & 15, flags = f.a[0] >> 8;
+        int32_t b = 0;
+        while (reg[b] != t) ++b;
+        f.a[0] = b | flags;
+      }
+      out.push_back(f);
+    }
+  }
+  FixOp end = blank(FIX_END);
+  int32_t slots[12];
+  for (int i = 0; i < 4; ++i) slots[i] = m.img[8 + i];
+  for (int i = 0; i < 8; ++i) slots[4 + i] = m.img[i];
+  pack_images(end, slots);
+  end.a[8] = flip;
+  out.push_back(end);
+  // Each table's first entries load from the moment the one before it is done.
+  std::vector<FixOp> body(out.begin() + (std::ptrdiff_t)mark, out.end());
+  out.resize(mark);
+  auto fetch = [&](size_t from) {
+    for (size_t i = from; i < body.size(); ++i)
+      if (body[i].kind == FIX_TABLE) {
+        FixOp f = body[i];
+        f.kind = FIX_FETCH;
+        out.push_back(f);
+        return;
+      }
+  };
+  fetch(0);
+  for (size_t i = 0; i < body.size(); ++i) {
+    out.push_back(body[i]);
+    if (body[i].kind == FIX_TABLE) fetch(i + 1);
+  }
+  return true;
+}
+
+}  // namespace dmv

@@ -1,0 +1,399 @@
+// Fixed-point window pass (complex128 storage): the FP64 pass's rotations and
+// phase tables (rewrite_pass_rotations) as 64-bit integer arithmetic.
+//
+// GB300 issues an FP64 multiply-add from one warp every ~77 cycles per SM
+// quarter, a 32 x 32 -> 64-bit integer one every few. So a tile of 2^12
+// amplitudes is turned into integers under one exponent: the largest
+// component gets 56 bits, and a rotation output x0 - w x1 (the same f M form
+// as OP_ROT) is three integer multiply-adds and one rounding to the last bit,
+// 2^-56 of the tile's largest component: less than FP64 rounds a component of
+// the tile's average size by. The ops run in register phases (build_fix_pass):
+// 256 threads hold 16 amplitudes each, the tile crosses shared memory once per
+// phase, exchanges cost nothing (they re-index the tile).
+//
+// Which tiles. Fixed point keeps less of a component the smaller it is, so a
+// tile runs in it only when every amplitude is within 2^kFixRange of its
+// largest one (entangled states: all but one tile in a few hundred). Any
+// other tile (product states, exact zeros, infinities, NaN) takes the FP64
+// ops in shared memory. A tile of zeros is left as it is.
+//
+// Headroom. A component of the tile can grow: every phase checks that each is
+// below 2^58 when it is written back. 16 amplitudes of that size have a norm
+// below 2^60.5, and inside a phase the stored norm grows at most 2 sqrt 2 times
+// (kFixShift halves it), so no sum leaves 63 bits. A tile that fails the check
+// is loaded again and runs in FP64.
+
+constexpr int kFixThreads = 256;
+constexpr int kFixThreadBits = 8;
+constexpr int kFixAmps = 16;       // amplitudes per thread: (2^12 tile) / 256
+constexpr int kFixRange = 12;      // binary orders between a tile's largest and smallest amplitude
+constexpr int kFixLimitBits = 58;  // components checked below 2^58 between phases
+
+struct FixPassParams {
+  TmaPassParams t;
+  const FixOp* fix_ops;
+  const longlong2* fix_tab;
+  int32_t num_fix_ops;
+  int32_t shifts;  // halvings over the whole pass
+};
+
+__device__ __forceinline__ uint32_t fix_slot(uint32_t l) { return l ^ (((l >> 3) ^ (l >> 6) ^ (l >> 9)) & 7u); }
+
+__device__ __forceinline__ long long fix_wide(int a, int b) {
+  long long p;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(p) : "r"(a), "r"(b));
+  return p;
+}
+
+// x m / 2^64 = high + low for |x| < 2^62 and the multiplier m = mh 2^32 + ml
+// (0 <= mh < 2^31, ml signed). x's low word is taken as signed too, so low
+// stays within 2^30 + 2^29; the two truncated middle products average to the
+// 1 that is added. Three bare products: with the sums inside the 64-bit
+// multiply-adds a rotation took 24 cycles per warp output and SM quarter, so
+// 20; volatile keeps the compiler from hoisting products of other pairs,
+// which spills (23 without it).
+__device__ __forceinline__ void fix_mul(long long x, int mh, int ml, long long& high, int& low) {
+  const int xl = (int)x, xh = (int)(x >> 32) + (int)((unsigned)xl >> 31);
+  int q1, q2;
+  asm volatile("mul.hi.s32 %0, %1, %2;" : "=r"(q1) : "r"(xl), "r"(mh));
+  asm volatile("mul.hi.s32 %0, %1, %2;" : "=r"(q2) : "r"(xh), "r"(ml));
+  asm volatile("mul.wide.s32 %0, %1, %2;" : "=l"(high) : "r"(xh), "r"(mh));
+  low = q1 + q2 + 1;
+}
+
+// x + q and x - q for a 32-bit q.
+__device__ __forceinline__ long long fix_add(long long x, int q) {
+  unsigned l = (unsigned)x, h = (unsigned)(x >> 32);
+  asm("{add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;}" : "+r"(l), "+r"(h) : "r"(q), "r"(q >> 31));
+  return (long long)((unsigned long long)h << 32 | l);
+}
+__device__ __forceinline__ long long fix_sub(long long x, int q) {
+  unsigned l = (unsigned)x, h = (unsigned)(x >> 32);
+  asm("{sub.cc.u32 %0, %0, %2;\n\tsubc.u32 %1, %1, %3;}" : "+r"(l), "+r"(h) : "r"(q), "r"(q >> 31));
+  return (long long)((unsigned long long)h << 32 | l);
+}
+
+// x in double -> round(x 2^(1078 - emax)) for |x| < 2^(emax - 1022): below 2^56.
+__device__ __forceinline__ long long fix_from_double(double x, int emax) {
+  const int hi = __double2hiint(x);
+  const int E = (hi >> 20) & 0x7FF;
+  const unsigned long long M =
+      ((unsigned long long)(unsigned)((hi & 0xFFFFF) | 0x100000) << 32 | (unsigned)__double2loint(x)) << 11;
+  const int s = 7 + emax - E;  // the leading one goes from bit 63 to bit 56 - (emax - E), one bit kept to round
+  unsigned long long X = E > 0 && s < 64 ? M >> s : 0ull;
+  X = (X + 1) >> 1;
+  const long long sg = (long long)(hi >> 31);
+  return ((long long)X ^ sg) - sg;
+}
+
+// round(x) 2^(e - 1075) as a double (e: the biased exponent of 2^52 in x's
+// units, the result normal), ties away from zero. Integer operations only: the
+// conversion instruction runs at the FP64 rate, 75 cycles per warp.
+__device__ __forceinline__ double fix_to_double(long long x, int e) {
+  const unsigned sign = (unsigned)(x >> 32) & 0x80000000u;
+  const unsigned long long a = x < 0 ? 0ull - (unsigned long long)x : (unsigned long long)x;
+  const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
+  const int lz = ah ? __clz((int)ah) : 32 + __clz((int)al);
+  const unsigned long long m = (((a << (lz & 63)) >> 1) + 0x200ull) >> 10;  // 53 bits, or 2^53
+  const unsigned long long r =
+      m + ((unsigned long long)(unsigned)(e + 10 - lz) << 52);  // the leading one adds 1 to the exponent
+  return a == 0 ? 0.0 : __longlong_as_double((long long)(r | (unsigned long long)sign << 32));
+}
+
+// The rotation [[1, -w], [w, 1]] of every register pair along bit TP; the
+// multiplier is w, or 1 - w (COMP: w >= 1/2).
+template <int TP, bool COMP>
+__device__ __forceinline__ void fix_rot(long long (&r)[2 * kFixAmps], int mh, int ml) {
+#pragma unroll
+  for (int j = 0; j < kFixAmps; ++j) {
+    if (j & (1 << TP)) continue;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      long long& a = r[2 * j + k];
+      long long& b = r[2 * (j | (1 << TP)) + k];
+      const long long x0 = a, x1 = b;
+      long long h0, h1;
+      int q0, q1;
+      fix_mul(x0, mh, ml, h0, q0);
+      fix_mul(x1, mh, ml, h1, q1);
+      if constexpr (COMP) {
+        a = fix_add(x0 - x1 + h1, q1);
+        b = fix_sub(x1 + x0 - h0, q0);
+      } else {
+        a = fix_sub(x0 - h1, q1);
+        b = fix_add(x1 + h0, q0);
+      }
+    }
+  }
+}
+
+template <int TP>
+__device__ __forceinline__ void fix_rot_form(long long (&r)[2 * kFixAmps], int flags, int mh, int ml) {
+  if (flags & kFixComplement) fix_rot<TP, true>(r, mh, ml);
+  else fix_rot<TP, false>(r, mh, ml);
+}
+
+// (x, y) times the Q.62 phase w = (cos, sin) (words hi 2^32 + lo with lo
+// signed), one rounding per component.
+__device__ __forceinline__ void fix_phase(long long& x, long long& y, const longlong2 w) {
+  const int cl = (int)w.x, ch = (int)(w.x >> 32), sl = (int)w.y, sh = (int)(w.y >> 32);
+  const int xl = (int)x, xh = (int)(x >> 32) + (int)((unsigned)xl >> 31);
+  const int yl = (int)y, yh = (int)(y >> 32) + (int)((unsigned)yl >> 31);
+  const long long b0 = fix_wide(xh, cl) + fix_wide(xl, ch) - fix_wide(yh, sl) - fix_wide(yl, sh) + (1ll << 29);
+  const long long b1 = fix_wide(yh, cl) + fix_wide(yl, ch) + fix_wide(xh, sl) + fix_wide(xl, sh) + (1ll << 29);
+  const long long a0 = fix_wide(xh, ch) - fix_wide(yh, sh), a1 = fix_wide(yh, ch) + fix_wide(xh, sh);
+  x = (a0 << 2) + (b0 >> 30);
+  y = (a1 << 2) + (b1 >> 30);
+}
+
+// First entry of a table's slice for the tile at `base`.
+__device__ __forceinline__ int64_t fix_slice(const FixOp* op, int64_t base) {
+  const int4 w0 = *reinterpret_cast<const int4*>(op);
+  const int4 w1 = *(reinterpret_cast<const int4*>(op) + 1);
+  int gsel = 0;
+  if (w0.z > 0) gsel |= (int)((base >> w0.w) & 1);
+  if (w0.z > 1) gsel |= (int)((base >> w1.x) & 1) << 1;
+  if (w0.z > 2) gsel |= (int)((base >> w1.y) & 1) << 2;
+  return (int64_t)w0.y + ((int64_t)gsel << 12);
+}
+
+// Asynchronous copy of 16 bytes (L2 -> shared memory) by this thread.
+__device__ __forceinline__ void fix_copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void fix_copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void fix_copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Slot of register j.
+__device__ __forceinline__ uint32_t fix_reg(uint32_t base, const uint32_t (&pr)[4], int j) {
+  uint32_t s = base;
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+    if ((j >> b) & 1) s ^= pr[b];
+  return s;
+}
+
+template <typename FB>
+__global__ void __launch_bounds__(kFixThreads, 2)
+k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ FixPassParams fp) {
+  constexpr int NT = kFixThreads;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ uint32_t s_mx[NT / 32], s_mn[NT / 32], s_any[NT / 32];
+  __shared__ int s_high[16];
+  __shared__ int64_t s_slot[kFixAmps];
+  __shared__ int s_grown;
+  const TmaPassParams& p = fp.t;
+  unsigned char* tile =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int k = 12, T = 1 << k;
+  constexpr uint32_t tile_bytes = (uint32_t)T * 16u;
+  const int low = p.low, nh = p.nh, boxes = p.boxes;
+  const int64_t num_tiles = p.num_tiles;
+  const int tid = (int)threadIdx.x;
+  if (tid < 16) s_high[tid] = p.high[tid];
+  if (tid == 0) {
+    s_grown = 0;
+    mbar_init(&s_bar, 1);
+    fence_mbar_init();
+    tma_prefetch_map(&tmap);
+  }
+  // offset in HBM of element tid + 256 u: the thread's part and the slots' parts
+  int64_t t_off = (int64_t)(tid & ((1 << low) - 1));
+  const int from_tid = min(nh, kFixThreadBits - low);
+  for (int i = 0; i < from_tid; ++i) t_off |= (int64_t)((tid >> (low + i)) & 1) << p.high[i];
+  if (tid < kFixAmps) {
+    int64_t off = 0;
+    for (int i = from_tid; i < nh; ++i) off |= (int64_t)((tid >> (i - from_tid)) & 1) << p.high[i];
+    s_slot[tid] = off;
+  }
+  __syncthreads();
+  const TileGeom<16> geom{low, nh, s_high};
+  const int lane = tid & 31;
+  const bool mover = tid < 32;  // warp 0 issues the loads
+  double2* amps = static_cast<double2*>(p.amps);
+  longlong2* ti = reinterpret_cast<longlong2*>(tile);
+  // Table entries on their way: two groups of four per thread, its own slots.
+  longlong2* stage = ti + T + tid;
+  const FixOp* ops = fp.fix_ops;
+  if (fp.num_fix_ops <= kFixSmemOps) {
+    int4* dst = reinterpret_cast<int4*>(ti + T + 8 * NT);
+    const int4* src = reinterpret_cast<const int4*>(fp.fix_ops);
+    for (int i = tid; i < fp.num_fix_ops * 3; i += NT) dst[i] = src[i];
+    ops = reinterpret_cast<const FixOp*>(dst);
+  }
+
+  int64_t tix = blockIdx.x;
+  bool plain = false;  // this tile's fixed-point run failed its headroom check
+  uint32_t parity = 0;
+  if (mover && tix < num_tiles) geom.load(&tmap, &s_bar, tile, tix, boxes, tile_bytes, lane);
+  while (tix < num_tiles) {
+    const bool ok = mbar_wait(&s_bar, parity, p.wait_limit);
+    if (__syncthreads_or(!ok)) {
+      if (mover) {
+        if (lane == 0) atomicExch(p.status, 1);
+        mbar_wait(&s_bar, parity, kTmaDrainLimit);  // drain the one load in flight
+      }
+      return;
+    }
+    parity ^= 1u;
+    const int64_t base = geom.base(tix);
+    int64_t next = tix + gridDim.x;
+    long long r[2 * kFixAmps];
+    // largest and smallest amplitude (top words of their larger component)
+    uint32_t mx = 0, mn = ~0u, any = 0;
+#pragma unroll
+    for (int u = 0; u < kFixAmps; ++u) {
+      const longlong2 v = ti[tid + NT * u];
+      r[2 * u] = v.x;
+      r[2 * u + 1] = v.y;
+      const uint32_t h = max((uint32_t)(v.x >> 32) & 0x7FFFFFFFu, (uint32_t)(v.y >> 32) & 0x7FFFFFFFu);
+      mx = max(mx, h);
+      mn = min(mn, h);
+      any |= (uint32_t)v.x | (uint32_t)v.y;
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    any = __reduce_or_sync(0xffffffffu, any);
+    if (lane == 0) {
+      s_mx[tid >> 5] = mx;
+      s_mn[tid >> 5] = mn;
+      s_any[tid >> 5] = any;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+      mx = max(mx, s_mx[w]);
+      mn = min(mn, s_mn[w]);
+      any |= s_any[w];
+    }
+    const int emax = (int)(mx >> 20);
+    const bool zero = mx == 0 && any == 0;
+    const bool fixed = !plain && emax - (int)(mn >> 20) <= kFixRange && emax > 200 && emax < 1800;
+    int e_out = 0;
+    bool store = !zero;
+    plain = false;
+    if (fixed) {
+#pragma unroll
+      for (int u = 0; u < kFixAmps; ++u)
+        ti[fix_slot((uint32_t)(tid + NT * u))] =
+            make_longlong2(fix_from_double(__longlong_as_double(r[2 * u]), emax),
+                           fix_from_double(__longlong_as_double(r[2 * u + 1]), emax));
+      uint32_t pr[4] = {0, 0, 0, 0};
+      uint32_t pbase = 0, cx = 0;
+      bool loaded = false;
+      const longlong2* ahead = nullptr;  // the entries of the table being fetched
+      int4 nxt = *reinterpret_cast<const int4*>(ops);
+      for (int o = 0; o < fp.num_fix_ops; ++o) {
+        const FixOp* op = ops + o;
+        const int4 w0 = nxt;
+        if (o + 1 < fp.num_fix_ops) nxt = *reinterpret_cast<const int4*>(op + 1);
+        if (w0.x == FIX_ROT) {
+          switch (w0.y & 3) {
+            case 0: fix_rot_form<0>(r, w0.y, w0.z, w0.w); break;
+            case 1: fix_rot_form<1>(r, w0.y, w0.z, w0.w); break;
+            case 2: fix_rot_form<2>(r, w0.y, w0.z, w0.w); break;
+            default: fix_rot_form<3>(r, w0.y, w0.z, w0.w); break;
+          }
+          if (w0.y & kFixShift) {
+#pragma unroll
+            for (int j = 0; j < 2 * kFixAmps; ++j) r[j] >>= 1;
+          }
+        } else if (w0.x == FIX_TABLE) {
+          // groups of four entries: wait for this one, then start the one after the next
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            if (g < 3) fix_copy_wait<1>();
+            else fix_copy_wait<0>();
+            longlong2 t[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t[j] = stage[NT * (4 * (g & 1) + j)];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fix_phase(r[2 * (4 * g + j)], r[2 * (4 * g + j) + 1], t[j]);
+            if (g < 2) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) fix_copy16(stage + NT * (4 * g + j), ahead + NT * (4 * g + 8 + j));
+              fix_copy_commit();
+            }
+          }
+        } else if (w0.x == FIX_FETCH) {
+          ahead = fp.fix_tab + fix_slice(op, base) + tid;
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fix_copy16(stage + NT * (4 * g + j), ahead + NT * (4 * g + j));
+            fix_copy_commit();
+          }
+        } else if (w0.x == FIX_XOR) {
+          if ((base >> w0.y) & 1) cx ^= (uint32_t)w0.z;
+        } else {  // FIX_PHASE, FIX_END
+          const int4 w1 = *(reinterpret_cast<const int4*>(op) + 1);
+          if (loaded) {
+            int hmax = 0, hmin = 0;
+#pragma unroll
+            for (int j = 0; j < kFixAmps; ++j) {
+              ti[fix_reg(pbase, pr, j)] = make_longlong2(r[2 * j], r[2 * j + 1]);
+              hmax = max(hmax, max((int)(r[2 * j] >> 32), (int)(r[2 * j + 1] >> 32)));
+              hmin = min(hmin, min((int)(r[2 * j] >> 32), (int)(r[2 * j + 1] >> 32)));
+            }
+            if (hmax >= (1 << (kFixLimitBits - 32)) || hmin < -(1 << (kFixLimitBits - 32))) s_grown = 1;
+          }
+          __syncthreads();
+          const uint32_t img[6] = {(uint32_t)w0.y, (uint32_t)w0.z, (uint32_t)w0.w,
+                                   (uint32_t)w1.x, (uint32_t)w1.y, (uint32_t)w1.z};
+          pr[0] = img[0] & 0xFFFFu;
+          pr[1] = img[0] >> 16;
+          pr[2] = img[1] & 0xFFFFu;
+          pr[3] = img[1] >> 16;
+          cx ^= (uint32_t)op->a[8];
+          pbase = cx;
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            const uint32_t im = (b & 1) ? img[2 + b / 2] >> 16 : img[2 + b / 2] & 0xFFFFu;
+            if ((tid >> b) & 1) pbase ^= im;
+          }
+#pragma unroll
+          for (int j = 0; j < kFixAmps; ++j) {
+            const longlong2 v = ti[fix_reg(pbase, pr, j)];
+            r[2 * j] = v.x;
+            r[2 * j + 1] = v.y;
+          }
+          loaded = true;
+        }
+      }
+      if (s_grown) {  // written before the last barrier
+        plain = true;
+        store = false;
+        next = tix;
+      }
+      e_out = emax - 1078 + fp.shifts + 1075;
+    } else if (!zero) {
+      __syncthreads();
+      tile_apply_ops<FB>(reinterpret_cast<typename FB::T*>(tile), T, p.ops, p.num_ops, base, p.phase_tab);
+#pragma unroll
+      for (int u = 0; u < kFixAmps; ++u) {
+        const longlong2 v = ti[tid + NT * u];
+        r[2 * u] = v.x;
+        r[2 * u + 1] = v.y;
+      }
+    }
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) s_grown = 0;
+    if (mover && next < num_tiles) geom.load(&tmap, &s_bar, tile, next, boxes, tile_bytes, lane);
+    if (store) {
+      const int64_t at = base | t_off;
+#pragma unroll
+      for (int u = 0; u < kFixAmps; ++u) {
+        double2 v;
+        if (fixed) v = make_double2(fix_to_double(r[2 * u], e_out), fix_to_double(r[2 * u + 1], e_out));
+        else v = make_double2(__longlong_as_double(r[2 * u]), __longlong_as_double(r[2 * u + 1]));
+        amps[at | s_slot[u]] = v;
+      }
+    }
+    tix = next;
+  }
+}

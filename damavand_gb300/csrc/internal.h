@@ -63,9 +63,9 @@ enum OpClass : int32_t {
   OP_ANTI = 4,     // m00 = m11 = 0 (Y and scaled exchanges)
   OP_RXLIKE = 5,   // m00, m11 real and m01, m10 imaginary (RX and its adjoint): 8 multiply-adds
   // Only in window passes rewritten by rewrite_pass_rotations (diag_plan.cpp):
-  OP_ROT = 6,      // FP64: real rotation R = [[c, -s], [s, c]] applied as f * M, two multiply-adds per component:
-                   //   m[1] == 0: M = [[1, -w], [w, 1]] (w = s/c, f = c); m[1] == 1: M = [[w, -1], [1, w]] (w = c/s, f = s);
-                   //   m[0] = w. The state is left divided by f; the caller multiplies the product of the f's back.
+  OP_ROT = 6,      // FP64: real rotation R = [[c, -s], [s, c]] (0 <= s <= c) applied as f * M, M = [[1, -w], [w, 1]]
+                   //   (w = s/c, f = c), two multiply-adds per component; m[0] = w. The state is left divided by f; the
+                   //   caller multiplies the product of the f's back.
   OP_PHASE = 7     // every amplitude times a phase from a table (PhaseEntry); fields below
 };
 
@@ -111,6 +111,27 @@ struct alignas(32) PhaseEntry {
 };
 static_assert(sizeof(PhaseEntry) == 32, "PhaseEntry layout");
 constexpr int kMaxPhaseGlobals = 3;
+
+// A phase table before its entries are made: the angle of entry (gsel << k) |
+// l is c plus the turn of every term whose mask meets an odd number of set
+// bits of l | gsel << kPhaseGlobalBit, in units of 2^-64 of a full turn.
+constexpr int kPhaseGlobalBit = 20;
+struct PhaseTerm {
+  uint32_t mask;
+  uint32_t pad;
+  int64_t turn;
+};
+struct PhaseTable {
+  int64_t entry;  // first entry
+  int64_t c;
+  int32_t first_term, num_terms;
+  int32_t k, g;  // tile bits, global bits
+};
+struct PhaseTables {
+  std::vector<PhaseTerm> terms;
+  std::vector<PhaseTable> tables;
+  int64_t entries = 0;
+};
 
 // Register phases of a fused pass run by the TMA window kernel: each thread
 // keeps 2^rb amplitudes of the tile in registers, the ones that differ in rb
@@ -185,17 +206,16 @@ struct ScaleDD {
   }
 };
 int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot_ops, std::vector<Op>& dst,
-                               std::vector<PhaseEntry>& tab, ScaleDD* scale = nullptr);
+                               PhaseTables& tab, ScaleDD* scale = nullptr);
+// The entries of tables, on the host (the debug check; launch_plan has
+// k_phase_tables make them).
+void phase_entries(const PhaseTables& tabs, std::vector<PhaseEntry>& out);
 // e^{i phi} of a table entry in double.
 void phase_entry_value(const PhaseEntry& e, double& re, double& im);
-// The tables in the FP32-pair form (re_h, re_l, im_h, im_l) and as Q.54 limbs
-// (re_h, re_l, im_h, im_l: value = h * 2^31 + l, l in [0, 2^31)).
-void phase_tables_df(const std::vector<PhaseEntry>& in, std::vector<float4>& out);
 // The FP64 kernels' 16-byte form: (t, s) with the quadrant in bit 62 of each
 // (0 in both, as |t|, |s| < 2): bit 62 of t = swap_xy = q & 1, bit 62 of s =
 // q >> 1 (sign_y); sign_x = the xor of the two.
 void phase_tables_f64(const std::vector<PhaseEntry>& in, std::vector<double2>& out);
-void phase_tables_fx(const std::vector<PhaseEntry>& in, std::vector<int4>& out);
 
 // Arithmetic used for complex128 storage.
 enum Arith : int32_t {
@@ -267,12 +287,12 @@ int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
 // generator (PlanOptions::param_of / generator_of).
 int build_adjoint_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision, const PlanOptions& base,
                        Plan& plan);
-// rewrite_pass_rotations of several window passes, on host threads: pass
-// which[j] of `plan` into out[j] (its own ops, its own tables with OP_PHASE
-// offsets from 0, its factor product). Results do not depend on the threads.
+// rewrite_pass_rotations of several window passes: pass which[j] of `plan`
+// into out[j] (its own ops, its own tables with OP_PHASE offsets from 0, its
+// factor product).
 struct RewrittenPass {
   std::vector<Op> ops;
-  std::vector<PhaseEntry> tab;
+  PhaseTables tab;
   ScaleDD scale;
 };
 void rewrite_passes(const Plan& plan, const std::vector<int64_t>& which, bool rot_ops,
@@ -327,6 +347,48 @@ bool build_tc_pass(const Plan& plan, const Pass& ps, std::vector<TcStage>& stage
 void set_tc_convert_mode(int32_t mode);
 
 // ---------------------------------------------------------------------------
+// Fixed-point window passes (fix_window.cuh; complex128 storage): a rewritten
+// pass (rotations, phase tables, exchanges) as register phases over int64
+// amplitudes.
+//
+// The tile's logical amplitude l sits at shared-memory slot fix_slot(A l) xor
+// c: exchanges move no data, they change the linear map A (a CNOT inside the
+// tile) or the offset c (X, and per tile a CNOT controlled from outside it).
+// A phase keeps 16 amplitudes per thread in registers, those that differ in 4
+// register bits, and applies every op whose target is one of them.
+// ---------------------------------------------------------------------------
+enum FixKind : int32_t {
+  FIX_PHASE = 0,  // registers out, registers in: a[0..5] the images (fix_slot(A e_b)) of the 4 register bits, then of
+                  // the 8 thread bits, two 16-bit words each; a[8]: c ^= a[8] first. Host only: a[6] the tile bits of the
+                  // 8 thread bits, a[7] of the 4 register bits, 4 bits each
+  FIX_XOR = 1,    // slot offset c ^= a[1] on tiles where qubit a[0] is 1
+  FIX_ROT = 2,    // OP_ROT on register bit a[0] & 3: a[0] also holds kFixComplement and kFixShift; a[1], a[2]: the
+                  // multiplier as a[1] 2^-32 + a[2] 2^-64 (both signed words)
+  FIX_TABLE = 3,  // OP_PHASE: a[0] first table entry, a[1] number of global bits, a[2..4] those qubits. A table (and
+                  // each slice of it) lies in the order its phase reads it: register, then thread
+  FIX_FETCH = 4,  // a[0..4] as FIX_TABLE: start loading that table's first entries (the next FIX_TABLE's)
+  FIX_END = 5     // registers out; a[0..5], a[8] as FIX_PHASE for tile bits 8..11 and 0..7 under the final map
+};
+constexpr int32_t kFixComplement = 4;  // the multiplier is 1 - w
+constexpr int32_t kFixShift = 8;       // then every amplitude is halved
+struct alignas(16) FixOp {
+  int32_t kind;
+  int32_t a[11];
+};
+static_assert(sizeof(FixOp) == 48, "FixOp layout");
+// FixOps the kernel holds in shared memory; a longer pass reads them from HBM.
+constexpr int32_t kFixSmemOps = 256;
+// Shared-memory slot of 16-byte element l: its index within a row of 8 (the 32
+// banks) xored with the other three groups of 3 index bits, so that lanes that
+// differ in any three bits distinct modulo 3 meet different banks.
+inline int32_t fix_slot_host(int32_t l) { return l ^ (((l >> 3) ^ (l >> 6) ^ (l >> 9)) & 7); }
+// The ops of one rewritten pass over a 2^12-amplitude tile as FixOps, appended
+// to `out`; *shifts gets the number of halvings. False, appending nothing,
+// when the pass holds any op but OP_ROT, OP_PHASE and an uncontrolled or
+// CNOT-like OP_SWAP.
+bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32_t* shifts);
+
+// ---------------------------------------------------------------------------
 // Device state
 // ---------------------------------------------------------------------------
 struct DeviceBuffer {
@@ -355,13 +417,14 @@ struct dmv_state_s {
   std::vector<dmv::Pass> pass_staging;   // the launches of the last plan (long phase passes split)
   std::vector<dmv::PhaseOp> phase_ops;   // compact ops of the register-phase launches
   dmv::DeviceBuffer phase_ops_dev;
-  std::vector<dmv::PhaseEntry> phase_tab;  // phase tables of the rewritten passes
+  dmv::PhaseTables phase_tabs;             // phase tables of the rewritten passes
+  std::vector<unsigned char> phase_src;    // their terms and slices, as uploaded
+  dmv::DeviceBuffer phase_src_dev;
   std::vector<dmv::ScaleDD> pass_scale;  // launch_plan: OP_ROT factor product per staged pass
   dmv::DeviceBuffer phase_tab_dev;
-  std::vector<double2> phase_tab_f64;      // the tables in the FP64 kernels' 16-byte form
-  std::vector<float4> phase_tab_df;        // the same tables for the FP32-pair arithmetic
-  std::vector<int4> phase_tab_fx;          // and for the int64 arithmetic
   dmv::DeviceBuffer phase_tab2_dev;
+  std::vector<dmv::FixOp> fix_ops;         // fixed-point passes of the last plan
+  dmv::DeviceBuffer fix_ops_dev, phase_tab_fix_dev;
   std::vector<dmv::TcStage> tc_stages;  // tensor-core passes of the last plan
   std::vector<uint16_t> tc_u;
   dmv::DeviceBuffer tc_stages_dev, tc_u_dev;

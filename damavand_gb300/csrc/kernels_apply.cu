@@ -23,6 +23,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 #include <type_traits>
 
@@ -545,6 +546,74 @@ int encode_pass_map(CUtensorMap* map, void* amps, int32_t n, const Pass& ps, boo
 // The tensor-core window pass (ARITH_TC) and its launcher.
 #include "tc_window.cuh"
 
+// One slice (a pattern of global bits) of a phase table to be made.
+struct PhaseSlice {
+  int64_t entry;  // first entry
+  int64_t c;
+  int32_t first_term, num_terms;
+  uint32_t gsel;  // the slice's global bits, at kPhaseGlobalBit
+  int32_t k;      // tile bits
+  uint32_t tpos, rpos;  // the fixed-point table's order: the phase's thread and register bits (FixOp::a[6], a[7])
+};
+constexpr int kPhaseTabThreads = 256;
+constexpr int kPhaseTabEntries = 1024;  // per block
+
+// The entries of the phase tables from their terms, in the forms the pass
+// kernels read: FP64 (t, s) with the quadrant packed, FP32 pairs, Q.54 limbs,
+// and the fixed-point kernel's Q.62 (cos, sin), each where its pointer is set.
+// About 60 FP64 operations an entry: 30 us for the 24-qubit, 10-layer
+// forward's 230,000 entries, against 6 ms when the host made and uploaded them.
+__global__ void __launch_bounds__(kPhaseTabThreads)
+k_phase_tables(const PhaseSlice* __restrict__ slices, const PhaseTerm* __restrict__ terms, double2* f64, float4* df,
+               int4* fx, longlong2* fix) {
+  const PhaseSlice sl = slices[blockIdx.x];
+  const uint32_t first = blockIdx.y * kPhaseTabEntries;
+  const uint32_t end = min(first + (uint32_t)kPhaseTabEntries, 1u << sl.k);
+  for (uint32_t i = first + threadIdx.x; i < end; i += kPhaseTabThreads) {
+    uint32_t l = i;
+    if (sl.tpos) {
+      l = 0;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) l |= ((i >> b) & 1u) << ((sl.tpos >> (4 * b)) & 15u);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) l |= ((i >> (8 + b)) & 1u) << ((sl.rpos >> (4 * b)) & 15u);
+    }
+    const uint32_t bits = l | sl.gsel;
+    unsigned long long a = (unsigned long long)sl.c;
+    for (int j = 0; j < sl.num_terms; ++j) {
+      const PhaseTerm t = terms[sl.first_term + j];
+      if (__popc(t.mask & bits) & 1) a += (unsigned long long)t.turn;
+    }
+    // a = q quarter turns + r, |r| <= 1/8 turn
+    const unsigned q = (unsigned)((a + (1ull << 61)) >> 62) & 3u;
+    const double r = (double)(long long)(a - ((unsigned long long)q << 62));
+    double sh, ch;
+    sincospi(r * 0x1p-64, &sh, &ch);  // half the angle
+    const double t = -sh / ch, sn = 2.0 * sh * ch, cs = fma(-2.0 * sh, sh, 1.0);
+    const int64_t at = sl.entry + l;
+    if (f64)
+      f64[at] = make_double2(__hiloint2double(__double2hiint(t) | (int)((q & 1u) << 30), __double2loint(t)),
+                             __hiloint2double(__double2hiint(sn) | (int)((q >> 1) << 30), __double2loint(sn)));
+    const double x = (q & 1u) ? sn : cs, y = (q & 1u) ? cs : sn;
+    const double re = (q == 1u || q == 2u) ? -x : x, im = q >= 2u ? -y : y;
+    if (df) {
+      const float rh = (float)re, ih = (float)im;
+      df[at] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
+    }
+    if (fx) {
+      const long long fr = llrint(re * 0x1p54), fi = llrint(im * 0x1p54);
+      fx[at] = make_int4((int)(fr >> 31), (int)(fr & 0x7FFFFFFFll), (int)(fi >> 31), (int)(fi & 0x7FFFFFFFll));
+    }
+    if (fix) {  // the low words taken as signed
+      const long long fr = llrint(re * 0x1p62), fi = llrint(im * 0x1p62);
+      fix[sl.entry + i] = make_longlong2(fr + ((fr & 0x80000000ll) << 1), fi + ((fi & 0x80000000ll) << 1));
+    }
+  }
+}
+
+// The fixed-point window pass of complex128 states.
+#include "fix_window.cuh"
+
 // TMA kernels by policy: register phases for complex64 (FP32 arithmetic),
 // the shared-memory op loop for complex128 in FP64. The complex128 FP32-pair
 // and int64 arithmetics keep the shared-memory kernel (k_apply_window),
@@ -565,6 +634,56 @@ bool tma_eligible(const Pass& ps) {
   return tma_policy<P>() && k == kTileThreadBits + 3 && ps.num_high >= 3 && ps.low_bits >= row_bits<ES>();
 }
 
+// The parameters both TMA kernels and the fixed-point one read.
+TmaPassParams tma_params(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, const void* phase_tab) {
+  TmaPassParams p;
+  p.k = ps.low_bits + ps.num_high;
+  p.low = ps.low_bits;
+  p.nh = ps.num_high;
+  p.num_ops = (int32_t)ps.op_count;
+  for (int i = 0; i < 16; ++i) p.high[i] = i < ps.num_high ? ps.high[i] : 0;
+  p.boxes = 1 << (ps.num_high - 3);
+  p.wait_limit = g_tma_wait_limit;
+  p.num_tiles = int64_t(1) << (n - p.k);
+  p.ops = ops_dev + ps.op_begin;
+  p.phase_ops = nullptr;
+  p.phase_tab = phase_tab;
+  p.amps = amps;
+  p.status = tma_status_ptr();
+  return p;
+}
+
+// A rewritten pass (its FixOps in `fix_ops`, its FP64 ops in `ops_dev`) on the
+// fixed-point kernel.
+template <typename FB>
+int launch_window_fix(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, const void* phase_tab,
+                      const FixOp* fix_ops, int32_t num_fix_ops, int32_t shifts, const longlong2* fix_tab,
+                      cudaStream_t stream) {
+  if ((reinterpret_cast<uintptr_t>(amps) & 15u) != 0)
+    return set_error(DMV_ERR_INVALID, "statevector not 16-byte aligned");
+  CUtensorMap map;
+  DMV_TRY(encode_pass_map<16>(&map, amps, n, ps, false));
+  FixPassParams p;
+  p.t = tma_params(amps, n, ps, ops_dev, phase_tab);
+  if (!p.t.status) return set_error(DMV_ERR_CUDA, "cannot resolve the TMA status word");
+  p.fix_ops = fix_ops;
+  p.fix_tab = fix_tab;
+  p.num_fix_ops = num_fix_ops;
+  p.shifts = shifts;
+  const size_t smem = ((size_t)16 << 12) + 1024 + (size_t)8 * kFixThreads * 16 + kFixSmemOps * sizeof(FixOp);
+  static bool configured = false;
+  if (!configured) {
+    DMV_CUDA_TRY(cudaFuncSetAttribute(k_window_fix<FB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured = true;
+  }
+  int per_sm = 0;
+  DMV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_window_fix<FB>, kFixThreads, smem));
+  if (per_sm < 1) return set_error(DMV_ERR_CUDA, "fixed-point kernel cannot fit %zu bytes of shared memory", smem);
+  const int64_t grid = std::min<int64_t>(p.t.num_tiles, (int64_t)per_sm * num_sms());
+  k_window_fix<FB><<<(int)grid, kFixThreads, smem, stream>>>(map, p);
+  return DMV_OK;
+}
+
 template <typename P>
 int launch_window_tma(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, const PhaseOp* phase_ops_dev,
                       cudaStream_t stream, const void* phase_tab = nullptr, int fmt = 0) {
@@ -580,20 +699,8 @@ int launch_window_tma(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, 
       return set_error(DMV_ERR_INVALID, "statevector not 16-byte aligned");
     CUtensorMap map;
     DMV_TRY(encode_pass_map<ES>(&map, amps, n, ps, PHASES));
-    TmaPassParams p;
-    p.k = ps.low_bits + ps.num_high;
-    p.low = ps.low_bits;
-    p.nh = ps.num_high;
-    p.num_ops = (int32_t)ps.op_count;
-    for (int i = 0; i < 16; ++i) p.high[i] = i < ps.num_high ? ps.high[i] : 0;
-    p.boxes = 1 << (ps.num_high - 3);
-    p.wait_limit = g_tma_wait_limit;
-    p.num_tiles = int64_t(1) << (n - p.k);
-    p.ops = ops_dev + ps.op_begin;
+    TmaPassParams p = tma_params(amps, n, ps, ops_dev, phase_tab);
     p.phase_ops = phase_ops_dev ? phase_ops_dev + ps.op_begin : nullptr;
-    p.phase_tab = phase_tab;
-    p.amps = amps;
-    p.status = tma_status_ptr();
     if (!p.status) return set_error(DMV_ERR_CUDA, "cannot resolve the TMA status word");
     const size_t tile = (size_t)ES << p.k;
     if constexpr (PHASES) {
@@ -684,12 +791,11 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   const bool rewrite = c128 && ((s->arith == ARITH_FP64 && s->fp64_rewrite) || s->arith == ARITH_FP32X2 ||
                                 s->arith == ARITH_INT64);
   const bool rot_ops = s->arith == ARITH_FP64;
-  s->phase_tab.clear();
+  s->phase_tabs = PhaseTables();
   // Per staged pass, the product of its OP_ROT factors (1 elsewhere).
   std::vector<ScaleDD>& pass_scale = s->pass_scale;
   pass_scale.clear();
-  // The window passes' rewrites run on host threads (each pass independent);
-  // their tables are appended in pass order with the OP_PHASE offsets moved.
+  // The passes' tables are appended in pass order with the OP_PHASE offsets moved.
   std::vector<RewrittenPass> rewritten;
   std::vector<int64_t> rewritten_at(plan.passes.size(), -1);
   if (rewrite) {
@@ -710,12 +816,21 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       Pass rw = ps;
       rw.op_begin = (int64_t)ops.size();
       rw.op_count = (int64_t)r.ops.size();
-      const int32_t tab_base = (int32_t)s->phase_tab.size();
+      PhaseTables& all = s->phase_tabs;
+      const int64_t tab_base = all.entries;
+      if (tab_base + r.tab.entries > INT32_MAX)
+        return set_error(DMV_ERR_UNSUPPORTED, "gate list: too many phase tables for one call");
       for (Op op : r.ops) {
-        if (op.cls == OP_PHASE) op.fh[0] += tab_base;
+        if (op.cls == OP_PHASE) op.fh[0] += (int32_t)tab_base;
         ops.push_back(op);
       }
-      s->phase_tab.insert(s->phase_tab.end(), r.tab.begin(), r.tab.end());
+      for (PhaseTable t : r.tab.tables) {
+        t.entry += tab_base;
+        t.first_term += (int32_t)all.terms.size();
+        all.tables.push_back(t);
+      }
+      all.terms.insert(all.terms.end(), r.tab.terms.begin(), r.tab.terms.end());
+      all.entries += r.tab.entries;
       passes.push_back(rw);
       pass_scale.push_back(r.scale);
       continue;
@@ -754,32 +869,81 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
     phase_ops_dev = static_cast<const PhaseOp*>(s->phase_ops_dev.ptr);
   }
   const Op* ops_dev = static_cast<const Op*>(s->ops_dev.ptr);
-  // Phase tables: the FP64 form (also read by an int64 pass that falls back to
-  // FP64) and the FP32-pair or Q.54 form for those arithmetics.
+  // Fixed-point passes: every rewritten FP64 pass that the kernel takes.
+  std::vector<int64_t> fix_first(passes.size(), -1);
+  std::vector<int32_t> fix_count(passes.size(), 0), fix_shifts(passes.size(), 0);
+  s->fix_ops.clear();
+  if (rewrite && rot_ops)
+    for (size_t i = 0; i < passes.size(); ++i) {
+      const Pass& ps = passes[i];
+      if (ps.kind != 1 || !tma_eligible<PolF64>(ps)) continue;
+      const size_t mark = s->fix_ops.size();
+      if (!build_fix_pass(ops.data() + ps.op_begin, ps.op_count, s->fix_ops, &fix_shifts[i])) continue;
+      fix_first[i] = (int64_t)mark;
+      fix_count[i] = (int32_t)(s->fix_ops.size() - mark);
+    }
+  if (!s->fix_ops.empty()) {
+    DMV_TRY(s->fix_ops_dev.reserve(s->fix_ops.size() * sizeof(FixOp)));
+    DMV_CUDA_TRY(cudaMemcpyAsync(s->fix_ops_dev.ptr, s->fix_ops.data(), s->fix_ops.size() * sizeof(FixOp),
+                                 cudaMemcpyHostToDevice, s->stream));
+  }
+  // Phase tables, made on the device: the FP64 form (also read by an int64
+  // pass that falls back to FP64), the FP32-pair or Q.54 form for those
+  // arithmetics, and the fixed-point passes' form.
   const void* phase_tab_dev = nullptr;
   const void* phase_tab2_dev = nullptr;
-  int64_t tab2_bytes = 0;
-  if (!s->phase_tab.empty()) {
-    phase_tables_f64(s->phase_tab, s->phase_tab_f64);
-    DMV_TRY(s->phase_tab_dev.reserve(s->phase_tab_f64.size() * sizeof(double2)));
-    DMV_CUDA_TRY(cudaMemcpyAsync(s->phase_tab_dev.ptr, s->phase_tab_f64.data(),
-                                 s->phase_tab_f64.size() * sizeof(double2), cudaMemcpyHostToDevice, s->stream));
-    phase_tab_dev = s->phase_tab_dev.ptr;
-    const void* src2 = nullptr;
-    if (s->arith == ARITH_FP32X2) {
-      phase_tables_df(s->phase_tab, s->phase_tab_df);
-      src2 = s->phase_tab_df.data();
-      tab2_bytes = (int64_t)(s->phase_tab_df.size() * sizeof(float4));
-    } else if (s->arith == ARITH_INT64) {
-      phase_tables_fx(s->phase_tab, s->phase_tab_fx);
-      src2 = s->phase_tab_fx.data();
-      tab2_bytes = (int64_t)(s->phase_tab_fx.size() * sizeof(int4));
+  int64_t tab_bytes = 0;
+  const PhaseTables& tabs = s->phase_tabs;
+  if (tabs.entries > 0) {
+    std::vector<PhaseSlice> slices;
+    int32_t kmax = 0;
+    for (const PhaseTable& t : tabs.tables)
+      for (uint32_t g = 0; g < (1u << t.g); ++g) {
+        slices.push_back(PhaseSlice{t.entry + ((int64_t)g << t.k), t.c, t.first_term, t.num_terms,
+                                    g << kPhaseGlobalBit, t.k, 0u, 0u});
+        kmax = std::max(kmax, t.k);
+      }
+    // the orders of the fixed-point tables
+    uint32_t tpos = 0, rpos = 0;
+    for (const FixOp& f : s->fix_ops) {
+      if (f.kind == FIX_PHASE) {
+        tpos = (uint32_t)f.a[6];
+        rpos = (uint32_t)f.a[7];
+      } else if (f.kind == FIX_TABLE) {
+        auto it = std::lower_bound(slices.begin(), slices.end(), (int64_t)f.a[0],
+                                   [](const PhaseSlice& x, int64_t e) { return x.entry < e; });
+        for (int32_t g = 0; g < (1 << f.a[1]); ++g, ++it) {
+          it->tpos = tpos;
+          it->rpos = rpos;
+        }
+      }
     }
-    if (src2) {
-      DMV_TRY(s->phase_tab2_dev.reserve((size_t)tab2_bytes));
-      DMV_CUDA_TRY(cudaMemcpyAsync(s->phase_tab2_dev.ptr, src2, (size_t)tab2_bytes, cudaMemcpyHostToDevice, s->stream));
+    const size_t sb = slices.size() * sizeof(PhaseSlice), tb = tabs.terms.size() * sizeof(PhaseTerm);
+    s->phase_src.resize(sb + tb);
+    std::memcpy(s->phase_src.data(), slices.data(), sb);
+    if (tb) std::memcpy(s->phase_src.data() + sb, tabs.terms.data(), tb);
+    tab_bytes = (int64_t)(sb + tb);
+    DMV_TRY(s->phase_src_dev.reserve(sb + tb));
+    DMV_CUDA_TRY(cudaMemcpyAsync(s->phase_src_dev.ptr, s->phase_src.data(), sb + tb, cudaMemcpyHostToDevice, s->stream));
+    const size_t bytes = (size_t)tabs.entries * 16;  // every form has 16 bytes an entry
+    DMV_TRY(s->phase_tab_dev.reserve(bytes));
+    phase_tab_dev = s->phase_tab_dev.ptr;
+    const bool second = s->arith == ARITH_FP32X2 || s->arith == ARITH_INT64;
+    if (second) {
+      DMV_TRY(s->phase_tab2_dev.reserve(bytes));
       phase_tab2_dev = s->phase_tab2_dev.ptr;
     }
+    if (!s->fix_ops.empty()) DMV_TRY(s->phase_tab_fix_dev.reserve(bytes));
+    const dim3 grid((unsigned)slices.size(), (unsigned)(((1 << kmax) + kPhaseTabEntries - 1) / kPhaseTabEntries));
+    k_phase_tables<<<grid, kPhaseTabThreads, 0, s->stream>>>(
+        static_cast<const PhaseSlice*>(s->phase_src_dev.ptr),
+        reinterpret_cast<const PhaseTerm*>(static_cast<const char*>(s->phase_src_dev.ptr) + sb),
+        static_cast<double2*>(s->phase_tab_dev.ptr),
+        s->arith == ARITH_FP32X2 ? static_cast<float4*>(s->phase_tab2_dev.ptr) : nullptr,
+        s->arith == ARITH_INT64 ? static_cast<int4*>(s->phase_tab2_dev.ptr) : nullptr,
+        s->fix_ops.empty() ? nullptr : static_cast<longlong2*>(s->phase_tab_fix_dev.ptr));
+    count_launch();
+    DMV_CUDA_TRY(cudaGetLastError());
   }
   // Tensor-core arithmetic: the stages and block digit matrices of every
   // window pass it takes, uploaded once for the whole plan.
@@ -875,6 +1039,11 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       else if (arith == ARITH_FP32X2)
         DMV_TRY(launch_window_tma<PolDF>(a, s->n, ps, ops_dev, phase_ops_dev, st, phase_tab2_dev, df_fmt));
       else if (arith == ARITH_INT64) DMV_TRY(launch_window_tma<PolFX>(a, s->n, ps, ops_dev, phase_ops_dev, st, phase_tab2_dev));
+      else if (fix_first[pi] >= 0)
+        DMV_TRY(launch_window_fix<PolF64>(a, s->n, ps, ops_dev, phase_tab_dev,
+                                          static_cast<const FixOp*>(s->fix_ops_dev.ptr) + fix_first[pi],
+                                          fix_count[pi], fix_shifts[pi],
+                                          static_cast<const longlong2*>(s->phase_tab_fix_dev.ptr), st));
       else DMV_TRY(launch_window_tma<PolF64>(a, s->n, ps, ops_dev, phase_ops_dev, st, phase_tab_dev));
       prof_end(tok, s->stream);
       bytes += 2 * S;
@@ -895,8 +1064,8 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
     }
   s->last_passes = (int64_t)passes.size();
   s->last_ops = (int64_t)plan.ops.size();
-  s->last_phase_tab_bytes = (int64_t)(s->phase_tab_f64.size() * sizeof(double2));
-  s->last_upload_bytes = s->last_phase_tab_bytes + tab2_bytes + (any_window ? (int64_t)(ops.size() * sizeof(Op)) : 0) +
+  s->last_phase_tab_bytes = tab_bytes;
+  s->last_upload_bytes = s->last_phase_tab_bytes + (any_window ? (int64_t)(ops.size() * sizeof(Op)) : 0) +
                          (any_phases ? (int64_t)(s->phase_ops.size() * sizeof(PhaseOp)) : 0) +
                          (tc ? (int64_t)(s->tc_stages.size() * sizeof(TcStage) + s->tc_u.size() * 2) : 0);
   s->last_bytes = bytes;

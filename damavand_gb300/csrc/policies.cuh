@@ -317,25 +317,27 @@ __device__ __forceinline__ void tile_op(typename P::T* tile, int T, const Op& op
 }
 
 // OP_ROT (FP64 window passes): the real rotation [[c, -s], [s, c]] of every
-// pair along op.target, on the real parts and on the imaginary parts, as
-// f M: M = [[1, -w], [w, 1]] (op.m[1] == 0) or [[w, -1], [1, w]] (op.m[1] ==
-// 1), w = op.m[0]; one multiply-add per output (2 per amplitude). The factor
-// f is not applied here: the plan multiplies the product of its rotations'
-// factors back into the state once. Two pairs per iteration, as in tile_op.
-template <bool FORM_B>
-__device__ __forceinline__ void rot_pair(double w, double2& a0, double2& a1) {
-  const double x0 = a0.x, x1 = a1.x, y0 = a0.y, y1 = a1.y;
-  if constexpr (!FORM_B) {
-    a0 = make_double2(fma(-w, x1, x0), fma(-w, y1, y0));
-    a1 = make_double2(fma(w, x0, x1), fma(w, y0, y1));
-  } else {
-    a0 = make_double2(fma(w, x0, -x1), fma(w, y0, -y1));
-    a1 = make_double2(fma(w, x1, x0), fma(w, y1, y0));
-  }
+// pair along op.target, on the real parts and on the imaginary parts, as f M,
+// M = [[1, -w], [w, 1]], w = op.m[0]; one multiply-add per output (2 per
+// amplitude). The factor f is not applied here: the plan multiplies the
+// product of its rotations' factors back into the state once. Pairs of zeros
+// (a state that has not spread over every qubit yet) are left as they are. Two
+// pairs per iteration, as in tile_op.
+__device__ __forceinline__ bool any_bits(const double2& a, const double2& b) {
+  return ((__double2hiint(a.x) | __double2hiint(a.y) | __double2hiint(b.x) | __double2hiint(b.y)) & 0x7FFFFFFF) |
+         (__double2loint(a.x) | __double2loint(a.y) | __double2loint(b.x) | __double2loint(b.y));
 }
 
-template <bool FORM_B>
-__device__ __forceinline__ void tile_rot_form(double2* tile, int T, int t, double w) {
+__device__ __forceinline__ void rot_pair(double w, double2& a0, double2& a1) {
+  if (!any_bits(a0, a1)) return;
+  const double x0 = a0.x, x1 = a1.x, y0 = a0.y, y1 = a1.y;
+  a0 = make_double2(fma(-w, x1, x0), fma(-w, y1, y0));
+  a1 = make_double2(fma(w, x0, x1), fma(w, y0, y1));
+}
+
+__device__ __forceinline__ void tile_rot(double2* tile, int T, const Op& op) {
+  const int t = op.target;
+  const double w = op.m[0];
   const int half = T >> 1;
   const int bd = blockDim.x;
   for (int q = threadIdx.x; q < half; q += 2 * bd) {
@@ -345,21 +347,16 @@ __device__ __forceinline__ void tile_rot_form(double2* tile, int T, int t, doubl
     if (q2 < half) {
       const uint32_t m0 = insert_zero32((uint32_t)q2, t), m1 = m0 | (1u << t);
       double2 b0 = tile[m0], b1 = tile[m1];
-      rot_pair<FORM_B>(w, a0, a1);
-      rot_pair<FORM_B>(w, b0, b1);
+      rot_pair(w, a0, a1);
+      rot_pair(w, b0, b1);
       tile[m0] = b0;
       tile[m1] = b1;
     } else {
-      rot_pair<FORM_B>(w, a0, a1);
+      rot_pair(w, a0, a1);
     }
     tile[l0] = a0;
     tile[l1] = a1;
   }
-}
-
-__device__ __forceinline__ void tile_rot(double2* tile, int T, const Op& op) {
-  if (op.m[1] == 0.0) tile_rot_form<false>(tile, T, op.target, op.m[0]);
-  else tile_rot_form<true>(tile, T, op.target, op.m[0]);
 }
 
 // OP_PHASE (FP64 window passes): amplitude l times the phase of table entry
@@ -380,6 +377,7 @@ __device__ __forceinline__ void tile_phase(double2* tile, int T, const Op& op, c
     const double t = __hiloint2double(th & ~(1 << 30), __double2loint(ts.x));
     const double s = __hiloint2double(sh & ~(1 << 30), __double2loint(ts.y));
     const double2 v = tile[l];
+    if (!any_bits(v, v)) continue;
     const double x1 = fma(t, v.y, v.x);
     const double y1 = fma(s, x1, v.y);
     const double x2 = fma(t, y1, x1);
