@@ -383,6 +383,8 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
           if (acc.hi * f >= 0x1p-200) {
             r.cls = OP_ROT;
             r.m[0] = w;
+            r.mh[0] = (float)w;
+            r.ml[0] = (float)(w - (double)r.mh[0]);
             acc.mul(f);
           } else {
             const long double F = ((long double)acc.hi + (long double)acc.lo) * (long double)f;

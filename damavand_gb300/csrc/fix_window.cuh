@@ -14,14 +14,15 @@
 // Which tiles. Fixed point keeps less of a component the smaller it is, so a
 // tile runs in it only when every amplitude is within 2^kFixRange of its
 // largest one (entangled states: all but one tile in a few hundred). Any
-// other tile (product states, exact zeros, infinities, NaN) takes the FP64
-// ops in shared memory. A tile of zeros is left as it is.
+// other tile (product states, exact zeros, infinities, NaN) takes the pass's
+// ops in shared memory in the arithmetic FB (FP64, or FP32 pairs for states of
+// that arithmetic). A tile of zeros is left as it is.
 //
 // Headroom. A component of the tile can grow: every phase checks that each is
 // below 2^58 when it is written back. 16 amplitudes of that size have a norm
 // below 2^60.5, and inside a phase the stored norm grows at most 2 sqrt 2 times
 // (kFixShift halves it), so no sum leaves 63 bits. A tile that fails the check
-// is loaded again and runs in FP64.
+// is loaded again and runs in FB.
 
 constexpr int kFixThreads = 256;
 constexpr int kFixThreadBits = 8;
@@ -371,13 +372,21 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
       }
       e_out = emax - 1078 + fp.shifts + 1075;
     } else if (!zero) {
+      using V = typename FB::T;
+      static_assert(sizeof(V) == 16, "the tile is converted in place");
+      V* tv = reinterpret_cast<V*>(tile);
+      if constexpr (!std::is_same<V, double2>::value) {
+#pragma unroll
+        for (int u = 0; u < kFixAmps; ++u)
+          tv[tid + NT * u] = FB::in(make_double2(__longlong_as_double(r[2 * u]), __longlong_as_double(r[2 * u + 1])));
+      }
       __syncthreads();
-      tile_apply_ops<FB>(reinterpret_cast<typename FB::T*>(tile), T, p.ops, p.num_ops, base, p.phase_tab);
+      tile_apply_ops<FB>(tv, T, p.ops, p.num_ops, base, p.phase_tab);
 #pragma unroll
       for (int u = 0; u < kFixAmps; ++u) {
-        const longlong2 v = ti[tid + NT * u];
-        r[2 * u] = v.x;
-        r[2 * u + 1] = v.y;
+        const double2 v = FB::out(tv[tid + NT * u]);
+        r[2 * u] = __double_as_longlong(v.x);
+        r[2 * u + 1] = __double_as_longlong(v.y);
       }
     }
     fence_proxy_async_smem();

@@ -64,7 +64,7 @@ enum OpClass : int32_t {
   OP_RXLIKE = 5,   // m00, m11 real and m01, m10 imaginary (RX and its adjoint): 8 multiply-adds
   // Only in window passes rewritten by rewrite_pass_rotations (diag_plan.cpp):
   OP_ROT = 6,      // FP64: real rotation R = [[c, -s], [s, c]] (0 <= s <= c) applied as f * M, M = [[1, -w], [w, 1]]
-                   //   (w = s/c, f = c), two multiply-adds per component; m[0] = w. The state is left divided by f; the
+                   //   (w = s/c, f = c), two multiply-adds per component; m[0] = w (mh[0], ml[0] its FP32 pair). The state is left divided by f; the
                    //   caller multiplies the product of the f's back.
   OP_PHASE = 7     // every amplitude times a phase from a table (PhaseEntry); fields below
 };

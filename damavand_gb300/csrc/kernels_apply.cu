@@ -759,7 +759,7 @@ double op_multiply_adds(const Op& op, int64_t N, int arith) {
     case OP_GENERAL: per_pair = pair_arith ? 172. : fixed ? 64. : 16.; break;
     case OP_RXLIKE: per_pair = pair_arith ? 76. : fixed ? 64. : 8.; break;  // int64: the general code
     case OP_SWAP: per_pair = 0.; break;
-    case OP_ROT: per_pair = 4.; break;  // FP64 only: one multiply-add per output, re and im
+    case OP_ROT: per_pair = pair_arith ? 60. : 4.; break;  // one multiply-add per output, re and im
     case OP_PHASE: per_pair = pair_arith ? 76. : fixed ? 32. : 6.; break;  // one complex product per amplitude
     default: per_pair = pair_arith ? 76. : fixed ? 32. : 8.; break;
   }
@@ -773,6 +773,10 @@ int window_reg_bits(const dmv_state_s* s, const Pass& ps) {
   if (s->precision == DMV_C64 && tma_eligible<PolF32>(ps)) return kPhaseRegBits;
   return 0;
 }
+
+// FP32-pair states: the least product of rotation factors a state or a pass
+// leaves out.
+constexpr double kPairScale = 0x1p-40;
 
 int launch_plan(dmv_state_s* s, const Plan& plan) {
   // The launches: every pass, except that a register-phase pass with more
@@ -791,6 +795,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   const bool rewrite = c128 && ((s->arith == ARITH_FP64 && s->fp64_rewrite) || s->arith == ARITH_FP32X2 ||
                                 s->arith == ARITH_INT64);
   const bool rot_ops = s->arith == ARITH_FP64;
+  const bool fix = rewrite && s->arith != ARITH_INT64 && s->n >= 12;  // fixed-point passes where the kernel takes them
   s->phase_tabs = PhaseTables();
   // Per staged pass, the product of its OP_ROT factors (1 elsewhere).
   std::vector<ScaleDD>& pass_scale = s->pass_scale;
@@ -805,14 +810,29 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
         rewritten_at[i] = (int64_t)which.size();
         which.push_back((int64_t)i);
       }
-    rewrite_passes(plan, which, rot_ops, rewritten);
+    rewrite_passes(plan, which, rot_ops || fix, rewritten);
   }
+  // Fixed-point passes: the FixOps of every rewritten pass that the kernel takes.
+  std::vector<int64_t> fix_first;
+  std::vector<int32_t> fix_count, fix_shifts;
+  s->fix_ops.clear();
   for (size_t pi = 0; pi < plan.passes.size(); ++pi) {
     const Pass& ps = plan.passes[pi];
     const int rb = ps.kind == 1 ? window_reg_bits(s, ps) : 0;
     any_window |= ps.kind == 1;
     if (rewritten_at[pi] >= 0) {
-      const RewrittenPass& r = rewritten[(size_t)rewritten_at[pi]];
+      RewrittenPass& r = rewritten[(size_t)rewritten_at[pi]];
+      const size_t mark = s->fix_ops.size();
+      int32_t shifts = 0;
+      // FP32 pairs hold the unscaled values of a pass only to 2^40
+      bool fixed = fix && tma_eligible<PolF64>(ps) && (rot_ops || r.scale.hi >= kPairScale) &&
+                   build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), s->fix_ops, &shifts);
+      if (fix && !rot_ops && !fixed) {  // FP32 pairs outside the fixed-point kernel: rotations as real 2x2 ops
+        s->fix_ops.resize(mark);
+        r = RewrittenPass();
+        rewrite_pass_rotations(plan.ops.data() + ps.op_begin, ps.op_count, ps.low_bits + ps.num_high, false, r.ops,
+                               r.tab, &r.scale);
+      }
       Pass rw = ps;
       rw.op_begin = (int64_t)ops.size();
       rw.op_count = (int64_t)r.ops.size();
@@ -824,6 +844,8 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
         if (op.cls == OP_PHASE) op.fh[0] += (int32_t)tab_base;
         ops.push_back(op);
       }
+      for (size_t i = mark; i < s->fix_ops.size(); ++i)
+        if (s->fix_ops[i].kind == FIX_TABLE || s->fix_ops[i].kind == FIX_FETCH) s->fix_ops[i].a[0] += (int32_t)tab_base;
       for (PhaseTable t : r.tab.tables) {
         t.entry += tab_base;
         t.first_term += (int32_t)all.terms.size();
@@ -831,6 +853,12 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       }
       all.terms.insert(all.terms.end(), r.tab.terms.begin(), r.tab.terms.end());
       all.entries += r.tab.entries;
+      fix_first.resize(passes.size(), -1);
+      fix_count.resize(passes.size(), 0);
+      fix_shifts.resize(passes.size(), 0);
+      fix_first.push_back(fixed ? (int64_t)mark : -1);
+      fix_count.push_back((int32_t)(s->fix_ops.size() - mark));
+      fix_shifts.push_back(shifts);
       passes.push_back(rw);
       pass_scale.push_back(r.scale);
       continue;
@@ -869,19 +897,9 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
     phase_ops_dev = static_cast<const PhaseOp*>(s->phase_ops_dev.ptr);
   }
   const Op* ops_dev = static_cast<const Op*>(s->ops_dev.ptr);
-  // Fixed-point passes: every rewritten FP64 pass that the kernel takes.
-  std::vector<int64_t> fix_first(passes.size(), -1);
-  std::vector<int32_t> fix_count(passes.size(), 0), fix_shifts(passes.size(), 0);
-  s->fix_ops.clear();
-  if (rewrite && rot_ops)
-    for (size_t i = 0; i < passes.size(); ++i) {
-      const Pass& ps = passes[i];
-      if (ps.kind != 1 || !tma_eligible<PolF64>(ps)) continue;
-      const size_t mark = s->fix_ops.size();
-      if (!build_fix_pass(ops.data() + ps.op_begin, ps.op_count, s->fix_ops, &fix_shifts[i])) continue;
-      fix_first[i] = (int64_t)mark;
-      fix_count[i] = (int32_t)(s->fix_ops.size() - mark);
-    }
+  fix_first.resize(passes.size(), -1);
+  fix_count.resize(passes.size(), 0);
+  fix_shifts.resize(passes.size(), 0);
   if (!s->fix_ops.empty()) {
     DMV_TRY(s->fix_ops_dev.reserve(s->fix_ops.size() * sizeof(FixOp)));
     DMV_CUDA_TRY(cudaMemcpyAsync(s->fix_ops_dev.ptr, s->fix_ops.data(), s->fix_ops.size() * sizeof(FixOp),
@@ -926,8 +944,10 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
     DMV_TRY(s->phase_src_dev.reserve(sb + tb));
     DMV_CUDA_TRY(cudaMemcpyAsync(s->phase_src_dev.ptr, s->phase_src.data(), sb + tb, cudaMemcpyHostToDevice, s->stream));
     const size_t bytes = (size_t)tabs.entries * 16;  // every form has 16 bytes an entry
-    DMV_TRY(s->phase_tab_dev.reserve(bytes));
-    phase_tab_dev = s->phase_tab_dev.ptr;
+    if (s->arith != ARITH_FP32X2) {
+      DMV_TRY(s->phase_tab_dev.reserve(bytes));
+      phase_tab_dev = s->phase_tab_dev.ptr;
+    }
     const bool second = s->arith == ARITH_FP32X2 || s->arith == ARITH_INT64;
     if (second) {
       DMV_TRY(s->phase_tab2_dev.reserve(bytes));
@@ -938,7 +958,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
     k_phase_tables<<<grid, kPhaseTabThreads, 0, s->stream>>>(
         static_cast<const PhaseSlice*>(s->phase_src_dev.ptr),
         reinterpret_cast<const PhaseTerm*>(static_cast<const char*>(s->phase_src_dev.ptr) + sb),
-        static_cast<double2*>(s->phase_tab_dev.ptr),
+        s->arith == ARITH_FP32X2 ? nullptr : static_cast<double2*>(s->phase_tab_dev.ptr),
         s->arith == ARITH_FP32X2 ? static_cast<float4*>(s->phase_tab2_dev.ptr) : nullptr,
         s->arith == ARITH_INT64 ? static_cast<int4*>(s->phase_tab2_dev.ptr) : nullptr,
         s->fix_ops.empty() ? nullptr : static_cast<longlong2*>(s->phase_tab_fix_dev.ptr));
@@ -982,16 +1002,18 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   // FP32-pair arithmetic: when every launch is a window pass, the state stays in
   // the FP32-pair form between them (k_apply_window's FMT bits).
   bool df_chain = c128 && s->arith == ARITH_FP32X2 && passes.size() >= 2;
-  for (const Pass& ps : passes) df_chain = df_chain && ps.kind == 1;
+  for (size_t pi = 0; pi < passes.size(); ++pi) df_chain = df_chain && passes[pi].kind == 1 && fix_first[pi] < 0;
   // The OP_ROT factors left out of the state so far (each in [1/sqrt 2, 1];
   // a pass leaves at most 2^200 out, rewrite_pass_rotations folds the rest
   // back itself): multiplied back at the end, or after a pass when the stored
-  // values could have grown past 2^200.
+  // values could have grown past 2^200 (FP32 pairs: 2^40, twice that stays in
+  // FP32's range with the pairs' 48 bits).
   ScaleDD owed;
+  const double owed_min = rot_ops ? 0x1p-200 : kPairScale;
   for (size_t pi = 0; pi < passes.size(); ++pi) {
     if (pi > 0) {
       owed.mul(pass_scale[pi - 1]);
-      if (std::fabs(owed.hi) < 0x1p-200) {
+      if (std::fabs(owed.hi) < owed_min) {
         DMV_TRY(launch_scale_state(s, owed.hi));
         owed = ScaleDD();
       }
@@ -1036,14 +1058,16 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       void* a = s->amps;
       cudaStream_t st = s->stream;
       if (s->precision == DMV_C64) DMV_TRY(launch_window_tma<PolF32>(a, s->n, ps, ops_dev, phase_ops_dev, st));
-      else if (arith == ARITH_FP32X2)
+      else if (fix_first[pi] >= 0) {
+        const FixOp* f = static_cast<const FixOp*>(s->fix_ops_dev.ptr) + fix_first[pi];
+        const longlong2* ft = static_cast<const longlong2*>(s->phase_tab_fix_dev.ptr);
+        if (arith == ARITH_FP32X2)
+          DMV_TRY(launch_window_fix<PolDF>(a, s->n, ps, ops_dev, phase_tab2_dev, f, fix_count[pi], fix_shifts[pi], ft, st));
+        else
+          DMV_TRY(launch_window_fix<PolF64>(a, s->n, ps, ops_dev, phase_tab_dev, f, fix_count[pi], fix_shifts[pi], ft, st));
+      } else if (arith == ARITH_FP32X2)
         DMV_TRY(launch_window_tma<PolDF>(a, s->n, ps, ops_dev, phase_ops_dev, st, phase_tab2_dev, df_fmt));
       else if (arith == ARITH_INT64) DMV_TRY(launch_window_tma<PolFX>(a, s->n, ps, ops_dev, phase_ops_dev, st, phase_tab2_dev));
-      else if (fix_first[pi] >= 0)
-        DMV_TRY(launch_window_fix<PolF64>(a, s->n, ps, ops_dev, phase_tab_dev,
-                                          static_cast<const FixOp*>(s->fix_ops_dev.ptr) + fix_first[pi],
-                                          fix_count[pi], fix_shifts[pi],
-                                          static_cast<const longlong2*>(s->phase_tab_fix_dev.ptr), st));
       else DMV_TRY(launch_window_tma<PolF64>(a, s->n, ps, ops_dev, phase_ops_dev, st, phase_tab_dev));
       prof_end(tok, s->stream);
       bytes += 2 * S;

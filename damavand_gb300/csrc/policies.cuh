@@ -359,6 +359,30 @@ __device__ __forceinline__ void tile_rot(double2* tile, int T, const Op& op) {
   }
 }
 
+// The same in FP32 pairs: each output a one-product compensated sum.
+__device__ __forceinline__ void df_rot_out(float wh, float wl, float xh, float xl, float yh, float yl, float& oh,
+                                           float& ol) {  // y + w x
+  DFAcc a{yh, yl};
+  df_add(a, wh, wl, xh, xl);
+  df_finish(a, oh, ol);
+}
+
+__device__ __forceinline__ void tile_rot(float4* tile, int T, const Op& op) {
+  const int t = op.target;
+  const float wh = op.mh[0], wl = op.ml[0];
+  for (int q = threadIdx.x; q < (T >> 1); q += blockDim.x) {
+    const uint32_t l0 = insert_zero32((uint32_t)q, t), l1 = l0 | (1u << t);
+    const float4 a0 = tile[l0], a1 = tile[l1];
+    float4 b0, b1;
+    df_rot_out(-wh, -wl, a1.x, a1.y, a0.x, a0.y, b0.x, b0.y);
+    df_rot_out(-wh, -wl, a1.z, a1.w, a0.z, a0.w, b0.z, b0.w);
+    df_rot_out(wh, wl, a0.x, a0.y, a1.x, a1.y, b1.x, b1.y);
+    df_rot_out(wh, wl, a0.z, a0.w, a1.z, a1.w, b1.z, b1.w);
+    tile[l0] = b0;
+    tile[l1] = b1;
+  }
+}
+
 // OP_PHASE (FP64 window passes): amplitude l times the phase of table entry
 // op.fh[0] + (gsel << k) + l, in the 16-byte form of phase_tables_f64: three
 // shears by (t, s), then for the factor i^q a swap and sign flips on the
@@ -460,6 +484,11 @@ __device__ __forceinline__ void tile_apply_ops(typename P::T* tile, int T, const
         continue;
       }
     } else if constexpr (std::is_same<P, PolDF>::value) {
+      if (op.cls == OP_ROT) {
+        tile_rot(tile, T, op);
+        __syncthreads();
+        continue;
+      }
       if (op.cls == OP_PHASE) {
         tile_phase_df(tile, T, op, static_cast<const float4*>(tab), base);
         __syncthreads();

@@ -16,9 +16,11 @@ from helpers import apply_gates, free_state, load_state, new_state, oracle_forwa
 pytestmark = pytest.mark.gpu
 
 
-def _run(n, gates, psi):
+def _run(n, gates, psi, arith=0):
+    from damavand_gb300._lib import check, lib
     st = new_state(n)
     try:
+        check(lib.dmv_state_set_arithmetic(st.handle, arith))
         load_state(st, psi)
         apply_gates(st, gates, 1)
         return st.numpy()
@@ -93,3 +95,19 @@ def test_non_finite_tile_stays_apart(built_lib, oracle_mod):
     part = 1 << 12  # the gates act on qubits 0-11
     assert not np.all(np.isfinite(got[:part]))
     assert np.max(np.abs(got[part:] - want[part:])) <= _tol(gates) * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("start", ["uniform", "zero", "dense"])
+def test_pair_states_off_the_integers(built_lib, oracle_mod, start):
+    """FP32-pair states: tiles that leave the fixed point run in pairs (48 bits), next to ones that
+    do not, over enough passes that the factors left out are multiplied back in between."""
+    from damavand_gb300._lib import ARITH_FP32X2
+    from damavand_gb300.workloads import ladder_circuit
+    n = 15
+    rng = np.random.default_rng(6)
+    psi = {"uniform": np.full(1 << n, 2.0 ** (-n / 2), dtype=np.complex128),
+           "zero": np.eye(1, 1 << n, dtype=np.complex128)[0], "dense": random_state(n, rng)}[start]
+    gates = ladder_circuit(n, 25, 3, False)
+    want = oracle_forward_any_control(oracle_mod, n, gates, psi)
+    got = _run(n, gates, psi, ARITH_FP32X2)
+    assert np.max(np.abs(got - want)) <= 2 * len(gates) * 2.0 ** -47 * np.max(np.abs(want))
