@@ -419,6 +419,7 @@ extern "C" int dmv_state_create(int32_t num_qubits, int32_t precision, void* str
 extern "C" int dmv_state_destroy(dmv_state_t s) {
   if (!s) return DMV_OK;
   if (s->stream) cudaStreamSynchronize(s->stream);
+  release_adjoint(s);
   if (s->amps) cudaFree(s->amps);
   s->amps = nullptr;
   s->ops_dev.release();

@@ -337,9 +337,34 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
     emit(x);
   };
 
+  // The measurement of an adjoint sweep's op, where the pending factors leave
+  // its target alone; `frame`: the phase already applied to the set bit.
+  auto emit_grad = [&](const Op& op, int64_t frame) {
+    Op g = blank_op();
+    g.cls = OP_GRAD;
+    g.target = op.target;
+    g.ctrl = -1;
+    g.ctrl_kind = CTRL_NONE;
+    g.param = op.param;
+    g.m[0] = acc.hi * acc.hi;
+    std::memcpy(g.fh, &frame, sizeof(frame));
+    emit(g);
+  };
+
   for (int64_t i = 0; i < count; ++i) {
     const Op& op = src[i];
     const uint32_t tb = 1u << op.target;
+    bool measure = op.generator != 0 && rot_ops;
+    double Tq, Sq, Cq;
+    int64_t a1, a2, g2;
+    const bool rotation = op.unitary && op.ctrl_kind == CTRL_NONE &&
+                          (op.cls == OP_GENERAL || op.cls == OP_REAL || op.cls == OP_RXLIKE) &&
+                          zyz(op.m, Tq, Sq, Cq, a1, a2, g2);
+    if (measure && !rotation) {
+      if (pend.supp & tb) flush();
+      emit_grad(op, 0);
+      measure = false;
+    }
     if (op.cls == OP_SWAP) {
       if (!permute(pend, op)) {
         flush();
@@ -348,68 +373,64 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
       emit(op);
       continue;
     }
-    if (op.unitary && op.ctrl_kind == CTRL_NONE &&
-        (op.cls == OP_GENERAL || op.cls == OP_REAL || op.cls == OP_RXLIKE)) {
-      double Tq, Sq, Cq;
-      int64_t a1, a2, g2;
-      if (zyz(op.m, Tq, Sq, Cq, a1, a2, g2)) {
-        const int t = op.target;
-        // FP64: t > pi/4 as R(t) = X R(pi/2 - t) Z, so every rotation has
-        // tan t <= 1; Z joins D2 and X is an exchange.
-        const bool flip = rot_ops && Cq < Sq;
-        if (flip) {
-          std::swap(Cq, Sq);
-          g2 = add_turns(g2, kHalfTurn);
-        }
-        if (g2 != 0) add_bit_term(*home(tb), t, 0, g2);  // D2
-        if (pend.supp & tb) flush();
-        Op r = blank_op();
-        r.target = t;
-        r.ctrl = -1;
-        r.ctrl_kind = CTRL_NONE;
-        if (rot_ops) {
-          // R = f M with M's diagonal exactly 1: two multiply-adds per
-          // component instead of three shears; f (>= 1/sqrt 2) goes to *scale.
-          // f = 1 / sqrt(1 + w^2), rounded once from a wider result, so that
-          // f M is orthogonal to within that rounding (no norm drift).
-          // The factors left out since the last fold live in `acc`; before
-          // the stored values could grow past 2^200 this rotation is applied
-          // as the real 2x2 acc f M instead (8 multiply-adds per pair), which
-          // gives the state its true scale back.
-          (void)Tq;
-          const double w = Sq / Cq;
-          const long double wl = w;
-          const double f = (double)(1.0L / std::sqrt(1.0L + wl * wl));
-          if (acc.hi * f >= 0x1p-200) {
-            r.cls = OP_ROT;
-            r.m[0] = w;
-            r.mh[0] = (float)w;
-            r.ml[0] = (float)(w - (double)r.mh[0]);
-            acc.mul(f);
-          } else {
-            const long double F = ((long double)acc.hi + (long double)acc.lo) * (long double)f;
-            const double one = (double)F, ww = (double)(F * wl);
-            r.cls = OP_REAL;
-            r.m[0] = one;
-            r.m[2] = -ww;
-            r.m[4] = ww;
-            r.m[6] = one;
-            acc = ScaleDD();
-          }
-        } else {  // the rotation as a real 2x2 in the arithmetic's own form
-          r.cls = OP_REAL;
-          r.m[0] = Cq;
-          r.m[2] = -Sq;
-          r.m[4] = Sq;
-          r.m[6] = Cq;
-          split_matrix(r);
-        }
-        emit(r);
-        if (flip) emit_x(t);
-        // D1: after the rotation on its own bit, so it cannot join an earlier table
-        add_bit_term(pend, t, a1, a2);
-        continue;
+    if (rotation) {
+      const int t = op.target;
+      // FP64: t > pi/4 as R(t) = X R(pi/2 - t) Z, so every rotation has
+      // tan t <= 1; Z joins D2 and X is an exchange.
+      const bool flip = rot_ops && Cq < Sq;
+      if (flip) {
+        std::swap(Cq, Sq);
+        g2 = add_turns(g2, kHalfTurn);
       }
+      if (g2 != 0) add_bit_term(*home(tb), t, 0, g2);  // D2
+      if (pend.supp & tb) flush();
+      if (measure) emit_grad(op, g2);
+      Op r = blank_op();
+      r.target = t;
+      r.ctrl = -1;
+      r.ctrl_kind = CTRL_NONE;
+      if (rot_ops) {
+        // R = f M with M's diagonal exactly 1: two multiply-adds per
+        // component instead of three shears; f (>= 1/sqrt 2) goes to *scale.
+        // f = 1 / sqrt(1 + w^2), rounded once from a wider result, so that
+        // f M is orthogonal to within that rounding (no norm drift).
+        // The factors left out since the last fold live in `acc`; before
+        // the stored values could grow past 2^200 this rotation is applied
+        // as the real 2x2 acc f M instead (8 multiply-adds per pair), which
+        // gives the state its true scale back.
+        (void)Tq;
+        const double w = Sq / Cq;
+        const long double wl = w;
+        const double f = (double)(1.0L / std::sqrt(1.0L + wl * wl));
+        if (acc.hi * f >= 0x1p-200) {
+          r.cls = OP_ROT;
+          r.m[0] = w;
+          r.mh[0] = (float)w;
+          r.ml[0] = (float)(w - (double)r.mh[0]);
+          acc.mul(f);
+        } else {
+          const long double F = ((long double)acc.hi + (long double)acc.lo) * (long double)f;
+          const double one = (double)F, ww = (double)(F * wl);
+          r.cls = OP_REAL;
+          r.m[0] = one;
+          r.m[2] = -ww;
+          r.m[4] = ww;
+          r.m[6] = one;
+          acc = ScaleDD();
+        }
+      } else {  // the rotation as a real 2x2 in the arithmetic's own form
+        r.cls = OP_REAL;
+        r.m[0] = Cq;
+        r.m[2] = -Sq;
+        r.m[4] = Sq;
+        r.m[6] = Cq;
+        split_matrix(r);
+      }
+      emit(r);
+      if (flip) emit_x(t);
+      // D1: after the rotation on its own bit, so it cannot join an earlier table
+      add_bit_term(pend, t, a1, a2);
+      continue;
     }
     if (op.unitary && op.cls == OP_DIAG && unit(op.m[0], op.m[1]) && unit(op.m[6], op.m[7]) &&
         op.ctrl_kind != CTRL_GLOBAL) {

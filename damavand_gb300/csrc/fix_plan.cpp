@@ -9,12 +9,13 @@
 namespace dmv {
 namespace {
 
-constexpr int kFixTileBits = 12;
-constexpr int kFixRegBits = 4;
+constexpr int kMaxTileBits = 12;
+constexpr int kThreadBits = 8;
+constexpr int kMaxFixRegBits = kMaxTileBits - kThreadBits;
 
 // The linear map l -> fix_slot(A l): images of the tile bits.
 struct SlotMap {
-  int32_t img[kFixTileBits];
+  int32_t img[kMaxTileBits];
 };
 
 int rank3(const int32_t* v, int n) {
@@ -43,18 +44,18 @@ void pack_images(FixOp& op, const int32_t* slot12) {
 // so that eight consecutive lanes' 16-byte accesses meet all 32 banks (their
 // slots differ in three independent ways modulo 8), low bits first: those also
 // read consecutive table entries.
-void thread_bits(const SlotMap& m, uint32_t regs, int32_t* bits) {
+void thread_bits(const SlotMap& m, int tile_bits, uint32_t regs, int32_t* bits) {
   int n = 0;
   uint32_t used = regs;
   int32_t pick[3];
-  for (int b = 0; b < kFixTileBits && n < 3; ++b) {
+  for (int b = 0; b < tile_bits && n < 3; ++b) {
     if ((used >> b) & 1u) continue;
     pick[n] = m.img[b];
     if (rank3(pick, n + 1) != n + 1) continue;
     bits[n++] = b;
     used |= 1u << b;
   }
-  for (int b = 0; b < kFixTileBits; ++b)
+  for (int b = 0; b < tile_bits; ++b)
     if (!((used >> b) & 1u)) bits[n++] = b;
 }
 
@@ -72,11 +73,13 @@ bool split_multiplier(double w, int32_t& hi, int32_t& lo) {
 
 }  // namespace
 
-bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32_t* shifts) {
+bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector<FixOp>& out, int32_t* shifts) {
+  const int32_t reg_bits = tile_bits - kThreadBits;
+  const uint32_t all_bits = (1u << tile_bits) - 1u;
   const size_t mark = out.size();
   *shifts = 0;
   SlotMap m;
-  for (int b = 0; b < kFixTileBits; ++b) m.img[b] = fix_slot_host(1 << b);
+  for (int b = 0; b < tile_bits; ++b) m.img[b] = fix_slot_host(1 << b);
   auto blank = [](int32_t kind) {
     FixOp f;
     std::memset(&f, 0, sizeof(f));
@@ -101,16 +104,17 @@ bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32
   };
   // The stored state is the true one times `grown`, kept in (1/sqrt 2, sqrt 2].
   double grown = 1.0;
+  double factor = 1.0;  // of the rotations so far (FIX_GRAD)
   std::vector<char> done((size_t)count, 0);
   std::vector<FixOp> taken;
   int64_t left = count, first = 0;
   while (left > 0) {
     while (done[(size_t)first]) ++first;
-    int32_t reg[kFixRegBits];
+    int32_t reg[kMaxFixRegBits];
     int nr = 0;
     uint32_t regs = 0, blocked = 0, used = 0;
     taken.clear();
-    for (int64_t i = first; i < count && blocked != 0xfffu; ++i) {
+    for (int64_t i = first; i < count && blocked != all_bits; ++i) {
       if (done[(size_t)i]) continue;
       const Op& op = ops[i];
       const uint32_t tb = 1u << op.target;
@@ -133,10 +137,10 @@ bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32
         for (int j = 0; j < op.fh[1]; ++j) f.a[2 + j] = op.fh[2 + j];
         used |= qs;
         taken.push_back(f);
-      } else if (op.cls == OP_ROT && op.ctrl_kind == CTRL_NONE) {
+      } else if ((op.cls == OP_ROT || op.cls == OP_GRAD) && op.ctrl_kind == CTRL_NONE) {
         if (tb & blocked) continue;
         if (!(regs & tb)) {
-          if (nr == kFixRegBits) {
+          if (nr == reg_bits) {
             blocked |= tb;
             continue;
           }
@@ -144,6 +148,18 @@ bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32
           regs |= tb;
         }
         used |= tb;
+        done[(size_t)i] = 1;
+        --left;
+        if (op.cls == OP_GRAD) {
+          FixOp f = blank(FIX_GRAD);
+          f.a[0] = op.target;
+          f.a[1] = op.param;
+          f.a[2] = *shifts;
+          const double sq = factor * factor;
+          std::memcpy(&f.a[3], &sq, sizeof(sq));
+          taken.push_back(f);
+          continue;
+        }
         FixOp f = blank(FIX_ROT);
         f.a[0] = op.target;  // the register bit once the phase is complete
         const double w = op.m[0];
@@ -155,12 +171,14 @@ bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32
           }
         }
         grown *= std::sqrt(1.0 + w * w);
+        factor /= std::sqrt(1.0 + w * w);
         if (grown > 1.4142135623730951) {
           f.a[0] |= kFixShift << 8;
           grown *= 0.5;
           ++*shifts;
         }
         taken.push_back(f);
+        continue;
       } else {
         out.resize(mark);
         return false;
@@ -170,27 +188,27 @@ bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32
     }
     if (taken.empty()) continue;
     // unused register bits from the top: the low ones serve the lanes
-    for (int b = kFixTileBits - 1; nr < kFixRegBits; --b)
+    for (int b = tile_bits - 1; nr < reg_bits; --b)
       if (!((regs >> b) & 1u)) {
         reg[nr++] = b;
         regs |= 1u << b;
       }
-    int32_t tbits[8], slots[12];
-    thread_bits(m, regs, tbits);
+    int32_t tbits[kThreadBits], slots[kMaxTileBits] = {};
+    thread_bits(m, tile_bits, regs, tbits);
     FixOp ph = blank(FIX_PHASE);
-    for (int i = 0; i < kFixRegBits; ++i) slots[i] = m.img[reg[i]];
-    for (int i = 0; i < 8; ++i) slots[kFixRegBits + i] = m.img[tbits[i]];
+    for (int i = 0; i < reg_bits; ++i) slots[i] = m.img[reg[i]];
+    for (int i = 0; i < kThreadBits; ++i) slots[kMaxFixRegBits + i] = m.img[tbits[i]];
     pack_images(ph, slots);
     uint32_t tpos = 0, rpos = 0;
-    for (int i = 0; i < 8; ++i) tpos |= (uint32_t)tbits[i] << (4 * i);
-    for (int i = 0; i < kFixRegBits; ++i) rpos |= (uint32_t)reg[i] << (4 * i);
+    for (int i = 0; i < kThreadBits; ++i) tpos |= (uint32_t)tbits[i] << (4 * i);
+    for (int i = 0; i < reg_bits; ++i) rpos |= (uint32_t)reg[i] << (4 * i);
     ph.a[6] = (int32_t)tpos;
     ph.a[7] = (int32_t)rpos;
     ph.a[8] = flip;
     flip = 0;
     out.push_back(ph);
     for (FixOp& f : taken) {
-      if (f.kind == FIX_ROT) {
+      if (f.kind == FIX_ROT || f.kind == FIX_GRAD) {
         const int32_t t = f.a[0] & 15, flags = f.a[0] >> 8;
         int32_t b = 0;
         while (reg[b] != t) ++b;
@@ -200,9 +218,9 @@ bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32
     }
   }
   FixOp end = blank(FIX_END);
-  int32_t slots[12];
-  for (int i = 0; i < 4; ++i) slots[i] = m.img[8 + i];
-  for (int i = 0; i < 8; ++i) slots[4 + i] = m.img[i];
+  int32_t slots[kMaxTileBits] = {};
+  for (int i = 0; i < reg_bits; ++i) slots[i] = m.img[kThreadBits + i];
+  for (int i = 0; i < kThreadBits; ++i) slots[kMaxFixRegBits + i] = m.img[i];
   pack_images(end, slots);
   end.a[8] = flip;
   out.push_back(end);

@@ -300,6 +300,7 @@ int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
   fg.reserve(gates.size());
   std::vector<int64_t> last_on((size_t)n, -1);
   const bool tagged = opt.param_of != nullptr;
+  if (opt.run_of) opt.run_of->assign(gates.size(), -1);
   for (size_t gi = 0; gi < gates.size(); ++gi) {
     const Gate& g = gates[gi];
     if (g.observable) continue;
@@ -308,6 +309,10 @@ int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
       const int64_t j = last_on[(size_t)g.target];
       if (j >= 0 && fg[(size_t)j].control < 0 && fg[(size_t)j].target == g.target) {
         matmul2(g.m, fg[(size_t)j].m, fg[(size_t)j].m);
+        if (opt.run_of) {
+          (*opt.run_of)[gi] = (int32_t)j;
+          if (opt.generator_of && opt.generator_of[gi]) fg[(size_t)j].generator = 1;
+        }
         continue;
       }
     }
@@ -317,6 +322,11 @@ int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
     std::memcpy(p.m, g.m, sizeof(p.m));
     p.param = tagged ? opt.param_of[gi] : -1;
     p.generator = tagged && opt.generator_of ? opt.generator_of[gi] : 0;
+    if (opt.run_of) {
+      p.param = (int32_t)fg.size();
+      p.generator = opt.generator_of && opt.generator_of[gi] ? 1 : 0;
+      (*opt.run_of)[gi] = p.param;
+    }
     fg.push_back(p);
     last_on[(size_t)g.target] = (int64_t)fg.size() - 1;
     if (g.control >= 0) last_on[(size_t)g.control] = (int64_t)fg.size() - 1;

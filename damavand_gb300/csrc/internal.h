@@ -66,7 +66,9 @@ enum OpClass : int32_t {
   OP_ROT = 6,      // FP64: real rotation R = [[c, -s], [s, c]] (0 <= s <= c) applied as f * M, M = [[1, -w], [w, 1]]
                    //   (w = s/c, f = c), two multiply-adds per component; m[0] = w (mh[0], ml[0] its FP32 pair). The state is left divided by f; the
                    //   caller multiplies the product of the f's back.
-  OP_PHASE = 7     // every amplitude times a phase from a table (PhaseEntry); fields below
+  OP_PHASE = 7,    // every amplitude times a phase from a table (PhaseEntry); fields below
+  OP_GRAD = 8      // adjoint sweeps: Im <lambda| P |psi> for P = X, Y, Z on `target` goes to slot `param`; in FP64 list
+                   //   order the squared product of the rotation factors before it is m[0]
 };
 
 // Control kinds inside a fused pass.
@@ -277,6 +279,11 @@ struct PlanOptions {
   // gates[i] carries param_of[i] / generator_of[i] (Op::param, Op::generator).
   const int32_t* param_of = nullptr;
   const int32_t* generator_of = nullptr;
+  // Adjoint sweeps in runs: when set (param_of null), gates are merged and
+  // (*run_of)[i] gets the index of the merged gate that gates[i] joined, which
+  // is also the Op::param of its op; Op::generator is set when any of its
+  // gates has a generator.
+  std::vector<int32_t>* run_of = nullptr;
 };
 
 int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
@@ -367,7 +374,9 @@ enum FixKind : int32_t {
   FIX_TABLE = 3,  // OP_PHASE: a[0] first table entry, a[1] number of global bits, a[2..4] those qubits. A table (and
                   // each slice of it) lies in the order its phase reads it: register, then thread
   FIX_FETCH = 4,  // a[0..4] as FIX_TABLE: start loading that table's first entries (the next FIX_TABLE's)
-  FIX_END = 5     // registers out; a[0..5], a[8] as FIX_PHASE for tile bits 8..11 and 0..7 under the final map
+  FIX_GRAD = 5,   // OP_GRAD on register bit a[0]: slot a[1], after a[2] halvings, a[3..4]: the squared product of the
+                  // rotation factors before it (double)
+  FIX_END = 6     // registers out; a[0..5], a[8] as FIX_PHASE for tile bits 8..11 and 0..7 under the final map
 };
 constexpr int32_t kFixComplement = 4;  // the multiplier is 1 - w
 constexpr int32_t kFixShift = 8;       // then every amplitude is halved
@@ -382,11 +391,23 @@ constexpr int32_t kFixSmemOps = 256;
 // banks) xored with the other three groups of 3 index bits, so that lanes that
 // differ in any three bits distinct modulo 3 meet different banks.
 inline int32_t fix_slot_host(int32_t l) { return l ^ (((l >> 3) ^ (l >> 6) ^ (l >> 9)) & 7); }
-// The ops of one rewritten pass over a 2^12-amplitude tile as FixOps, appended
-// to `out`; *shifts gets the number of halvings. False, appending nothing,
-// when the pass holds any op but OP_ROT, OP_PHASE and an uncontrolled or
-// CNOT-like OP_SWAP.
-bool build_fix_pass(const Op* ops, int64_t count, std::vector<FixOp>& out, int32_t* shifts);
+// The ops of one rewritten pass over a tile of 2^tile_bits amplitudes (12: 16
+// per thread, 11: 8) as FixOps, appended to `out`; *shifts gets the number of
+// halvings. False, appending nothing, when the pass holds any op but OP_ROT,
+// OP_PHASE, OP_GRAD and an uncontrolled or CNOT-like OP_SWAP.
+bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector<FixOp>& out, int32_t* shifts);
+// Where make_phase_tables puts each form of the tables' entries (null: nowhere).
+struct PhaseTableForms {
+  double2* f64 = nullptr;
+  float4* df = nullptr;
+  int4* fx = nullptr;
+  longlong2* fix = nullptr;  // in the order of fix_ops
+};
+struct DeviceBuffer;
+// Makes the entries of `tabs` on the device (k_phase_tables). `src`, `src_dev`
+// hold the upload.
+int make_phase_tables(const PhaseTables& tabs, const std::vector<FixOp>& fix_ops, const PhaseTableForms& forms,
+                      std::vector<unsigned char>& src, DeviceBuffer& src_dev, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------
 // Device state
@@ -435,11 +456,18 @@ struct dmv_state_s {
   int64_t last_phase_tab_bytes = 0;  // phase tables uploaded by the last plan
   int64_t last_upload_bytes = 0;     // every host-to-device byte of the last plan (ops, tables, digit matrices)
   bool fp64_rewrite = true;          // FP64 window passes as rotations and phase tables
+  // Adjoint gradients: psi and lambda, the partial sums, the plan, its tables.
+  // Kept between calls for states of at most kKeepAdjointBytes (allocating and
+  // freeing them took 0.3 ms of a 10-qubit gradient's 0.9 ms).
+  dmv_state_s* adj_state[2] = {nullptr, nullptr};
+  dmv::DeviceBuffer adj_partial, adj_src, adj_work, adj_tab, adj_fix_tab;
   cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
   size_t amp_bytes() const { return (size_t)N * (precision == DMV_C128 ? 16 : 8); }
 };
 
 namespace dmv {
+constexpr size_t kKeepAdjointBytes = size_t(64) << 20;
+void release_adjoint(dmv_state_s* s);
 int ensure_pinned(dmv_state_s* s, size_t bytes);
 
 // Planner settings for a state: tiles of 2^12 amplitudes (the TMA window
@@ -472,6 +500,9 @@ int sample_from_device_probs(const double* probs_device, int64_t num_probs, int3
                              uint64_t* samples_host);
 int launch_inner_product(dmv_state_s* a, dmv_state_s* b, double* re, double* im);
 int launch_scale_by_z_observable(dmv_state_s* dst, dmv_state_s* src, const double* weights_host);
+int adjoint_sweep_fix(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, const std::vector<Gate>& gates, double* grads,
+                      bool* done);
+int launch_reduce_rows(const double* in, int64_t rows, int cols, double* out, cudaStream_t stream);
 int launch_adjoint_step(dmv_state_s* psi, dmv_state_s* lam, const Op& op, double* grad_slot_device);
 int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const double* weights,
                      double* loss, double* grads);

@@ -27,6 +27,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "fix_ops.cuh"
 #include "internal.h"
 #include "phases.cuh"
 #include "policies.cuh"
@@ -774,6 +775,47 @@ int window_reg_bits(const dmv_state_s* s, const Pass& ps) {
   return 0;
 }
 
+int make_phase_tables(const PhaseTables& tabs, const std::vector<FixOp>& fix_ops, const PhaseTableForms& forms,
+                      std::vector<unsigned char>& src, DeviceBuffer& src_dev, cudaStream_t stream) {
+  std::vector<PhaseSlice> slices;
+  int32_t kmax = 0;
+  for (const PhaseTable& t : tabs.tables)
+    for (uint32_t g = 0; g < (1u << t.g); ++g) {
+      slices.push_back(PhaseSlice{t.entry + ((int64_t)g << t.k), t.c, t.first_term, t.num_terms, g << kPhaseGlobalBit,
+                                  t.k, 0u, 0u});
+      kmax = std::max(kmax, t.k);
+    }
+  // the orders of the fixed-point tables
+  uint32_t tpos = 0, rpos = 0;
+  for (const FixOp& f : fix_ops) {
+    if (f.kind == FIX_PHASE) {
+      tpos = (uint32_t)f.a[6];
+      rpos = (uint32_t)f.a[7];
+    } else if (f.kind == FIX_TABLE) {
+      auto it = std::lower_bound(slices.begin(), slices.end(), (int64_t)f.a[0],
+                                 [](const PhaseSlice& x, int64_t e) { return x.entry < e; });
+      for (int32_t g = 0; g < (1 << f.a[1]); ++g, ++it) {
+        it->tpos = tpos;
+        it->rpos = rpos;
+      }
+    }
+  }
+  const size_t sb = slices.size() * sizeof(PhaseSlice), tb = tabs.terms.size() * sizeof(PhaseTerm);
+  src.resize(sb + tb);
+  std::memcpy(src.data(), slices.data(), sb);
+  if (tb) std::memcpy(src.data() + sb, tabs.terms.data(), tb);
+  DMV_TRY(src_dev.reserve(sb + tb));
+  DMV_CUDA_TRY(cudaMemcpyAsync(src_dev.ptr, src.data(), sb + tb, cudaMemcpyHostToDevice, stream));
+  const dim3 grid((unsigned)slices.size(), (unsigned)(((1 << kmax) + kPhaseTabEntries - 1) / kPhaseTabEntries));
+  k_phase_tables<<<grid, kPhaseTabThreads, 0, stream>>>(
+      static_cast<const PhaseSlice*>(src_dev.ptr),
+      reinterpret_cast<const PhaseTerm*>(static_cast<const char*>(src_dev.ptr) + sb), forms.f64, forms.df, forms.fx,
+      forms.fix);
+  count_launch();
+  DMV_CUDA_TRY(cudaGetLastError());
+  return DMV_OK;
+}
+
 // FP32-pair states: the least product of rotation factors a state or a pass
 // leaves out.
 constexpr double kPairScale = 0x1p-40;
@@ -826,7 +868,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       int32_t shifts = 0;
       // FP32 pairs hold the unscaled values of a pass only to 2^40
       bool fixed = fix && tma_eligible<PolF64>(ps) && (rot_ops || r.scale.hi >= kPairScale) &&
-                   build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), s->fix_ops, &shifts);
+                   build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), 12, s->fix_ops, &shifts);
       if (fix && !rot_ops && !fixed) {  // FP32 pairs outside the fixed-point kernel: rotations as real 2x2 ops
         s->fix_ops.resize(mark);
         r = RewrittenPass();
@@ -913,57 +955,23 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   int64_t tab_bytes = 0;
   const PhaseTables& tabs = s->phase_tabs;
   if (tabs.entries > 0) {
-    std::vector<PhaseSlice> slices;
-    int32_t kmax = 0;
-    for (const PhaseTable& t : tabs.tables)
-      for (uint32_t g = 0; g < (1u << t.g); ++g) {
-        slices.push_back(PhaseSlice{t.entry + ((int64_t)g << t.k), t.c, t.first_term, t.num_terms,
-                                    g << kPhaseGlobalBit, t.k, 0u, 0u});
-        kmax = std::max(kmax, t.k);
-      }
-    // the orders of the fixed-point tables
-    uint32_t tpos = 0, rpos = 0;
-    for (const FixOp& f : s->fix_ops) {
-      if (f.kind == FIX_PHASE) {
-        tpos = (uint32_t)f.a[6];
-        rpos = (uint32_t)f.a[7];
-      } else if (f.kind == FIX_TABLE) {
-        auto it = std::lower_bound(slices.begin(), slices.end(), (int64_t)f.a[0],
-                                   [](const PhaseSlice& x, int64_t e) { return x.entry < e; });
-        for (int32_t g = 0; g < (1 << f.a[1]); ++g, ++it) {
-          it->tpos = tpos;
-          it->rpos = rpos;
-        }
-      }
-    }
-    const size_t sb = slices.size() * sizeof(PhaseSlice), tb = tabs.terms.size() * sizeof(PhaseTerm);
-    s->phase_src.resize(sb + tb);
-    std::memcpy(s->phase_src.data(), slices.data(), sb);
-    if (tb) std::memcpy(s->phase_src.data() + sb, tabs.terms.data(), tb);
-    tab_bytes = (int64_t)(sb + tb);
-    DMV_TRY(s->phase_src_dev.reserve(sb + tb));
-    DMV_CUDA_TRY(cudaMemcpyAsync(s->phase_src_dev.ptr, s->phase_src.data(), sb + tb, cudaMemcpyHostToDevice, s->stream));
     const size_t bytes = (size_t)tabs.entries * 16;  // every form has 16 bytes an entry
     if (s->arith != ARITH_FP32X2) {
       DMV_TRY(s->phase_tab_dev.reserve(bytes));
       phase_tab_dev = s->phase_tab_dev.ptr;
     }
-    const bool second = s->arith == ARITH_FP32X2 || s->arith == ARITH_INT64;
-    if (second) {
+    if (s->arith == ARITH_FP32X2 || s->arith == ARITH_INT64) {
       DMV_TRY(s->phase_tab2_dev.reserve(bytes));
       phase_tab2_dev = s->phase_tab2_dev.ptr;
     }
     if (!s->fix_ops.empty()) DMV_TRY(s->phase_tab_fix_dev.reserve(bytes));
-    const dim3 grid((unsigned)slices.size(), (unsigned)(((1 << kmax) + kPhaseTabEntries - 1) / kPhaseTabEntries));
-    k_phase_tables<<<grid, kPhaseTabThreads, 0, s->stream>>>(
-        static_cast<const PhaseSlice*>(s->phase_src_dev.ptr),
-        reinterpret_cast<const PhaseTerm*>(static_cast<const char*>(s->phase_src_dev.ptr) + sb),
-        s->arith == ARITH_FP32X2 ? nullptr : static_cast<double2*>(s->phase_tab_dev.ptr),
-        s->arith == ARITH_FP32X2 ? static_cast<float4*>(s->phase_tab2_dev.ptr) : nullptr,
-        s->arith == ARITH_INT64 ? static_cast<int4*>(s->phase_tab2_dev.ptr) : nullptr,
-        s->fix_ops.empty() ? nullptr : static_cast<longlong2*>(s->phase_tab_fix_dev.ptr));
-    count_launch();
-    DMV_CUDA_TRY(cudaGetLastError());
+    PhaseTableForms forms;
+    forms.f64 = static_cast<double2*>(s->arith == ARITH_FP32X2 ? nullptr : s->phase_tab_dev.ptr);
+    forms.df = static_cast<float4*>(s->arith == ARITH_FP32X2 ? s->phase_tab2_dev.ptr : nullptr);
+    forms.fx = static_cast<int4*>(s->arith == ARITH_INT64 ? s->phase_tab2_dev.ptr : nullptr);
+    forms.fix = static_cast<longlong2*>(s->fix_ops.empty() ? nullptr : s->phase_tab_fix_dev.ptr);
+    DMV_TRY(make_phase_tables(tabs, s->fix_ops, forms, s->phase_src, s->phase_src_dev, s->stream));
+    tab_bytes = (int64_t)s->phase_src.size();
   }
   // Tensor-core arithmetic: the stages and block digit matrices of every
   // window pass it takes, uploaded once for the whole plan.

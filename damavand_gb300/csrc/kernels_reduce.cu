@@ -1496,6 +1496,25 @@ int adjoint_sweep_windows(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, co
   return DMV_OK;
 }
 
+int launch_reduce_rows(const double* in, int64_t rows, int cols, double* out, cudaStream_t stream) {
+  k_reduce_rows<<<(int)((rows + 127) / 128), 128, 0, stream>>>(in, rows, cols, out);
+  count_launch();
+  DMV_CUDA_TRY(cudaGetLastError());
+  return DMV_OK;
+}
+
+void release_adjoint(dmv_state_s* s) {
+  for (dmv_state_t& a : s->adj_state) {
+    if (a) dmv_state_destroy(a);
+    a = nullptr;
+  }
+  s->adj_partial.release();
+  s->adj_src.release();
+  s->adj_work.release();
+  s->adj_tab.release();
+  s->adj_fix_tab.release();
+}
+
 int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const double* weights,
                      double* loss, double* grads) {
   // Forward from |0...0> with the fused plan.
@@ -1517,14 +1536,17 @@ int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const doubl
     if (!gates[i].observable && is_parametrised(gates[i].kind)) slot_of[i] = num_params++;
   if (num_params == 0) return DMV_OK;
 
-  dmv_state_t psi = nullptr, lam = nullptr;
-  int rc = dmv_state_create(s->n, s->precision, s->stream, &psi);
-  if (rc != DMV_OK) return rc;
-  rc = dmv_state_create(s->n, s->precision, s->stream, &lam);
-  if (rc != DMV_OK) { dmv_state_destroy(psi); return rc; }
+  int rc = DMV_OK;
+  for (dmv_state_t& a : s->adj_state)
+    if (!a && (rc = dmv_state_create(s->n, s->precision, s->stream, &a)) != DMV_OK) {
+      release_adjoint(s);
+      return rc;
+    }
+  const dmv_state_t psi = s->adj_state[0], lam = s->adj_state[1];
   psi->arith = lam->arith = s->arith;  // the sweep runs in the state's arithmetic
 
-  DeviceBuffer partial, adj_ops;
+  DeviceBuffer& partial = s->adj_partial;
+  DeviceBuffer adj_ops;
   const int64_t pairs_u = s->N >> 1;
   // Columns of the per-parameter partials: the widest grid of the sweep's kernels.
   const int grid = std::max(adjoint_grid(pairs_u), adjoint_window_grid(int64_t(1) << std::max(0, s->n - 12)));
@@ -1543,6 +1565,11 @@ int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const doubl
     }
     rc = launch_scale_by_z_observable(lam, s, weights);
     if (rc != DMV_OK) break;
+    if (s->precision == DMV_C128 && ((s->arith == ARITH_FP64 && s->fp64_rewrite) || s->arith == ARITH_FP32X2)) {
+      bool swept = false;
+      rc = adjoint_sweep_fix(s, psi, lam, gates, grads, &swept);
+      if (rc != DMV_OK || swept) break;
+    }
     // FP32-pair arithmetic: psi and lam are scratch, so they take the pair form
     // once and keep it for the whole sweep.
     const bool df_raw = s->precision == DMV_C128 && s->arith == ARITH_FP32X2;
@@ -1585,10 +1612,8 @@ int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const doubl
     }
   } while (false);
   cudaStreamSynchronize(s->stream);
-  partial.release();
   adj_ops.release();
-  dmv_state_destroy(psi);
-  dmv_state_destroy(lam);
+  if (rc != DMV_OK || s->amp_bytes() > kKeepAdjointBytes) release_adjoint(s);
   return rc;
 }
 
