@@ -11,8 +11,40 @@
 
 namespace dmv {
 
-constexpr int kFixRange = 12;      // binary orders between a tile's largest and smallest amplitude
-constexpr int kFixLimitBits = 58;  // components checked below 2^58 between phases
+// A tile's largest component starts at 57 bits. Between phases the tile is
+// brought back below 2^57 when one has grown past 2^58, and up to there when
+// all have shrunk below 2^55.
+constexpr int kFixTopBits = 26;  // of the high word
+constexpr int kFixLowBits = 24;
+
+// The shift (right, or left when negative) that a largest high word `m` asks for.
+__device__ __forceinline__ int fix_renorm(int m) {
+  const int bits = 32 - __clz(m);
+  return bits > kFixTopBits || bits < kFixLowBits ? bits - (kFixTopBits - 1) : 0;
+}
+
+template <int N>
+__device__ __forceinline__ void fix_shift(long long (&r)[N], int s) {
+  if (s > 0) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) r[j] >>= s;
+  } else if (s < 0) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) r[j] <<= -s;
+  }
+}
+
+// The largest |high word| (x >= 0: x, else ~x) of the registers.
+template <int N>
+__device__ __forceinline__ int fix_top(const long long (&r)[N]) {
+  int hi = 0, lo = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    hi = max(hi, (int)(r[j] >> 32));
+    lo = min(lo, (int)(r[j] >> 32));
+  }
+  return max(hi, ~lo);
+}
 
 __device__ __forceinline__ uint32_t fix_slot(uint32_t l) { return l ^ (((l >> 3) ^ (l >> 6) ^ (l >> 9)) & 7u); }
 
@@ -50,13 +82,13 @@ __device__ __forceinline__ long long fix_sub(long long x, int q) {
   return (long long)((unsigned long long)h << 32 | l);
 }
 
-// x in double -> round(x 2^(1078 - emax)) for |x| < 2^(emax - 1022): below 2^56.
+// x in double -> round(x 2^(1079 - emax)) for |x| < 2^(emax - 1022): below 2^57.
 __device__ __forceinline__ long long fix_from_double(double x, int emax) {
   const int hi = __double2hiint(x);
   const int E = (hi >> 20) & 0x7FF;
   const unsigned long long M =
       ((unsigned long long)(unsigned)((hi & 0xFFFFF) | 0x100000) << 32 | (unsigned)__double2loint(x)) << 11;
-  const int s = 7 + emax - E;  // the leading one goes from bit 63 to bit 56 - (emax - E), one bit kept to round
+  const int s = 6 + emax - E;  // the leading one goes from bit 63 to bit 57 - (emax - E), one bit kept to round
   unsigned long long X = E > 0 && s < 64 ? M >> s : 0ull;
   X = (X + 1) >> 1;
   const long long sg = (long long)(hi >> 31);

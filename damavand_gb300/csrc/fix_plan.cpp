@@ -73,7 +73,8 @@ bool split_multiplier(double w, int32_t& hi, int32_t& lo) {
 
 }  // namespace
 
-bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector<FixOp>& out, int32_t* shifts) {
+bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector<FixOp>& out, int32_t* shifts,
+                    uint32_t* sparse) {
   const int32_t reg_bits = tile_bits - kThreadBits;
   const uint32_t all_bits = (1u << tile_bits) - 1u;
   const size_t mark = out.size();
@@ -104,6 +105,8 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
   };
   // The stored state is the true one times `grown`, kept in (1/sqrt 2, sqrt 2].
   double grown = 1.0;
+  double least[16];  // per tile bit, its least rotation multiplier
+  for (double& w : least) w = 1.0;
   double factor = 1.0;  // of the rotations so far (FIX_GRAD)
   std::vector<char> done((size_t)count, 0);
   std::vector<FixOp> taken;
@@ -154,7 +157,6 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
           FixOp f = blank(FIX_GRAD);
           f.a[0] = op.target;
           f.a[1] = op.param;
-          f.a[2] = *shifts;
           const double sq = factor * factor;
           std::memcpy(&f.a[3], &sq, sizeof(sq));
           taken.push_back(f);
@@ -163,6 +165,7 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
         FixOp f = blank(FIX_ROT);
         f.a[0] = op.target;  // the register bit once the phase is complete
         const double w = op.m[0];
+        if (w != 0.0) least[op.target] = std::min(least[op.target], std::fabs(w));
         if (!split_multiplier(w, f.a[1], f.a[2])) {
           f.a[0] |= kFixComplement << 8;
           if (!split_multiplier(1.0 - w, f.a[1], f.a[2])) {
@@ -215,6 +218,15 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
         f.a[0] = b | flags;
       }
       out.push_back(f);
+    }
+  }
+  if (sparse) {
+    std::sort(least, least + tile_bits);
+    double p = 1.0;
+    *sparse = 1u;
+    for (int z = 1; z <= tile_bits; ++z) {
+      p *= least[z - 1];
+      if (z <= kFixUnreached && p >= std::ldexp(1.0, -kFixRange)) *sparse |= 1u << z;
     }
   }
   FixOp end = blank(FIX_END);

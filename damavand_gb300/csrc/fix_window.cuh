@@ -4,9 +4,9 @@
 // GB300 issues an FP64 multiply-add from one warp every ~77 cycles per SM
 // quarter, a 32 x 32 -> 64-bit integer one every few. So a tile of 2^12
 // amplitudes is turned into integers under one exponent: the largest
-// component gets 56 bits, and a rotation output x0 - w x1 (the same f M form
+// component gets 57 bits, and a rotation output x0 - w x1 (the same f M form
 // as OP_ROT) is three integer multiply-adds and one rounding to the last bit,
-// 2^-56 of the tile's largest component: less than FP64 rounds a component of
+// 2^-57 of the tile's largest component: less than FP64 rounds a component of
 // the tile's average size by. The ops run in register phases (build_fix_pass):
 // 256 threads hold 16 amplitudes each, the tile crosses shared memory once per
 // phase, exchanges cost nothing (they re-index the tile).
@@ -18,11 +18,15 @@
 // ops in shared memory in the arithmetic FB (FP64, or FP32 pairs for states of
 // that arithmetic). A tile of zeros is left as it is.
 //
-// Headroom. A component of the tile can grow: every phase checks that each is
-// below 2^58 when it is written back. 16 amplitudes of that size have a norm
-// below 2^60.5, and inside a phase the stored norm grows at most 2 sqrt 2 times
-// (kFixShift halves it), so no sum leaves 63 bits. A tile that fails the check
-// is loaded again and runs in FB.
+// An exact zero is in range where the pass's rotations spread no further than
+// that (build_fix_pass's `sparse`): the tiles of a state that has not reached
+// its last qubits yet.
+//
+// Headroom. A component of the tile can grow: every phase takes the largest
+// when it is written back, and the next shifts all of them below 2^58. 16
+// amplitudes of that size have a norm below 2^60.5, and inside a phase the
+// stored norm grows at most 2 sqrt 2 times (kFixShift halves it), so no sum
+// leaves 63 bits.
 
 constexpr int kFixThreads = 256;
 constexpr int kFixThreadBits = 8;
@@ -34,6 +38,7 @@ struct FixPassParams {
   const longlong2* fix_tab;
   int32_t num_fix_ops;
   int32_t shifts;  // halvings over the whole pass
+  uint32_t sparse; // numbers of unreached qubits a fixed-point tile may have (build_fix_pass)
 };
 
 template <typename FB>
@@ -42,10 +47,10 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
   constexpr int NT = kFixThreads;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_mx[NT / 32], s_mn[NT / 32], s_any[NT / 32];
+  __shared__ uint32_t s_mx[NT / 32], s_mn[NT / 32], s_any[NT / 32], s_cnt[NT / 32];
   __shared__ int s_high[16];
   __shared__ int64_t s_slot[kFixAmps];
-  __shared__ int s_grown;
+  __shared__ int s_top[3];  // largest component, by phase
   const TmaPassParams& p = fp.t;
   unsigned char* tile =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -56,7 +61,7 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
   const int tid = (int)threadIdx.x;
   if (tid < 16) s_high[tid] = p.high[tid];
   if (tid == 0) {
-    s_grown = 0;
+    s_top[0] = s_top[1] = s_top[2] = 0;
     mbar_init(&s_bar, 1);
     fence_mbar_init();
     tma_prefetch_map(&tmap);
@@ -87,7 +92,6 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
   }
 
   int64_t tix = blockIdx.x;
-  bool plain = false;  // this tile's fixed-point run failed its headroom check
   uint32_t parity = 0;
   if (mover && tix < num_tiles) geom.load(&tmap, &s_bar, tile, tix, boxes, tile_bytes, lane);
   while (tix < num_tiles) {
@@ -101,20 +105,25 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
     }
     parity ^= 1u;
     const int64_t base = geom.base(tix);
-    int64_t next = tix + gridDim.x;
+    const int64_t next = tix + gridDim.x;
     long long r[2 * kFixAmps];
     // largest and smallest amplitude (top words of their larger component)
-    uint32_t mx = 0, mn = ~0u, any = 0;
+    uint32_t mx = 0, mn = ~0u, any = 0, cnt = 0;
 #pragma unroll
     for (int u = 0; u < kFixAmps; ++u) {
       const longlong2 v = ti[tid + NT * u];
       r[2 * u] = v.x;
       r[2 * u + 1] = v.y;
       const uint32_t h = max((uint32_t)(v.x >> 32) & 0x7FFFFFFFu, (uint32_t)(v.y >> 32) & 0x7FFFFFFFu);
+      const uint32_t lo = (uint32_t)v.x | (uint32_t)v.y;
       mx = max(mx, h);
-      mn = min(mn, h);
-      any |= (uint32_t)v.x | (uint32_t)v.y;
+      any |= lo;
+      if (h | lo) {
+        mn = min(mn, h);
+        ++cnt;
+      }
     }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
     mx = __reduce_max_sync(0xffffffffu, mx);
     mn = __reduce_min_sync(0xffffffffu, mn);
     any = __reduce_or_sync(0xffffffffu, any);
@@ -122,20 +131,25 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
       s_mx[tid >> 5] = mx;
       s_mn[tid >> 5] = mn;
       s_any[tid >> 5] = any;
+      s_cnt[tid >> 5] = cnt;
     }
     __syncthreads();
+    cnt = 0;
 #pragma unroll
     for (int w = 0; w < NT / 32; ++w) {
       mx = max(mx, s_mx[w]);
       mn = min(mn, s_mn[w]);
       any |= s_any[w];
+      cnt += s_cnt[w];
     }
     const int emax = (int)(mx >> 20);
     const bool zero = mx == 0 && any == 0;
-    const bool fixed = !plain && emax - (int)(mn >> 20) <= kFixRange && emax > 200 && emax < 1800;
+    // qubits of the tile that the state has not reached: log2 (4096 / nonzero amplitudes)
+    const int unreached = k - (31 - __clz((int)cnt | 1));
+    const bool fixed = emax - (int)(mn >> 20) <= kFixRange && emax > 200 && emax < 1800 &&
+                       ((fp.sparse >> unreached) & 1u);
     int e_out = 0;
-    bool store = !zero;
-    plain = false;
+    const bool store = !zero;
     if (fixed) {
 #pragma unroll
       for (int u = 0; u < kFixAmps; ++u)
@@ -144,7 +158,8 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
                            fix_from_double(__longlong_as_double(r[2 * u + 1]), emax));
       uint32_t pr[4] = {0, 0, 0, 0};
       uint32_t pbase = 0, cx = 0;
-      bool loaded = false;
+      int phase = -1;  // of the registers
+      int renorm = 0;  // further halvings so far
       const longlong2* ahead = nullptr;  // the entries of the table being fetched
       int4 nxt = *reinterpret_cast<const int4*>(ops);
       for (int o = 0; o < fp.num_fix_ops; ++o) {
@@ -191,15 +206,13 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
           if ((base >> w0.y) & 1) cx ^= (uint32_t)w0.z;
         } else {  // FIX_PHASE, FIX_END
           const int4 w1 = *(reinterpret_cast<const int4*>(op) + 1);
-          if (loaded) {
-            int hmax = 0, hmin = 0;
+          if (phase >= 0) {
 #pragma unroll
-            for (int j = 0; j < kFixAmps; ++j) {
-              ti[fix_reg(pbase, pr, j)] = make_longlong2(r[2 * j], r[2 * j + 1]);
-              hmax = max(hmax, max((int)(r[2 * j] >> 32), (int)(r[2 * j + 1] >> 32)));
-              hmin = min(hmin, min((int)(r[2 * j] >> 32), (int)(r[2 * j + 1] >> 32)));
-            }
-            if (hmax >= (1 << (kFixLimitBits - 32)) || hmin < -(1 << (kFixLimitBits - 32))) s_grown = 1;
+            for (int j = 0; j < kFixAmps; ++j) ti[fix_reg(pbase, pr, j)] = make_longlong2(r[2 * j], r[2 * j + 1]);
+            const int top = __reduce_max_sync(0xffffffffu, fix_top(r));
+            if (lane == 0) atomicMax(&s_top[phase % 3], top);
+            // the next phase's word: last read before the barrier before this one
+            if (tid == 0) s_top[(phase + 1) % 3] = 0;
           }
           __syncthreads();
           const uint32_t img[6] = {(uint32_t)w0.y, (uint32_t)w0.z, (uint32_t)w0.w,
@@ -221,15 +234,15 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
             r[2 * j] = v.x;
             r[2 * j + 1] = v.y;
           }
-          loaded = true;
+          if (phase >= 0) {
+            const int sh = fix_renorm(s_top[phase % 3]);
+            fix_shift(r, sh);
+            renorm += sh;
+          }
+          ++phase;
         }
       }
-      if (s_grown) {  // written before the last barrier
-        plain = true;
-        store = false;
-        next = tix;
-      }
-      e_out = emax - 1078 + fp.shifts + 1075;
+      e_out = emax - 1079 + fp.shifts + renorm + 1075;
     } else if (!zero) {
       using V = typename FB::T;
       static_assert(sizeof(V) == 16, "the tile is converted in place");
@@ -250,7 +263,7 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
     }
     fence_proxy_async_smem();
     __syncthreads();
-    if (tid == 0) s_grown = 0;
+    if (tid == 0) s_top[0] = s_top[1] = s_top[2] = 0;
     if (mover && next < num_tiles) geom.load(&tmap, &s_bar, tile, next, boxes, tile_bytes, lane);
     if (store) {
       const int64_t at = base | t_off;

@@ -374,8 +374,8 @@ enum FixKind : int32_t {
   FIX_TABLE = 3,  // OP_PHASE: a[0] first table entry, a[1] number of global bits, a[2..4] those qubits. A table (and
                   // each slice of it) lies in the order its phase reads it: register, then thread
   FIX_FETCH = 4,  // a[0..4] as FIX_TABLE: start loading that table's first entries (the next FIX_TABLE's)
-  FIX_GRAD = 5,   // OP_GRAD on register bit a[0]: slot a[1], after a[2] halvings, a[3..4]: the squared product of the
-                  // rotation factors before it (double)
+  FIX_GRAD = 5,   // OP_GRAD on register bit a[0]: slot a[1], a[3..4]: the squared product of the rotation factors
+                  // before it (double)
   FIX_END = 6     // registers out; a[0..5], a[8] as FIX_PHASE for tile bits 8..11 and 0..7 under the final map
 };
 constexpr int32_t kFixComplement = 4;  // the multiplier is 1 - w
@@ -395,7 +395,15 @@ inline int32_t fix_slot_host(int32_t l) { return l ^ (((l >> 3) ^ (l >> 6) ^ (l 
 // per thread, 11: 8) as FixOps, appended to `out`; *shifts gets the number of
 // halvings. False, appending nothing, when the pass holds any op but OP_ROT,
 // OP_PHASE, OP_GRAD and an uncontrolled or CNOT-like OP_SWAP.
-bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector<FixOp>& out, int32_t* shifts);
+// Bit z of *sparse: the z smallest rotation multipliers (one per tile bit, the
+// least of its rotations) have a product of at least 2^-kFixRange, so that an
+// amplitude that spreads from a nonzero one over z bits stays within that
+// range of it, and z is at most kFixUnreached (a tile of 2^(12-z) nonzero
+// amplitudes rounds every one of 2^12).
+bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector<FixOp>& out, int32_t* shifts,
+                    uint32_t* sparse = nullptr);
+constexpr int kFixUnreached = 4;
+constexpr int kFixRange = 12;  // binary orders between a fixed-point tile's largest and smallest amplitude
 // Where make_phase_tables puts each form of the tables' entries (null: nowhere).
 struct PhaseTableForms {
   double2* f64 = nullptr;

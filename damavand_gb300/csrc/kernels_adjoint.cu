@@ -8,7 +8,10 @@
 // window pass (the forward planner's windows over the reversed gate list)
 // holds a tile of both states while it applies many runs. The updates are the
 // forward pass's rotations, phase tables and exchanges, in the fixed-point
-// arithmetic of fix_ops.cuh on tiles that qualify and in FP64 on the others.
+// arithmetic of fix_ops.cuh (2^-57 of a tile's largest component: psi and
+// lambda are scratch, and the sums they end in are no finer than that where
+// the tile's norm is spread). Concentrated tiles (the last ones before |0...0>),
+// and any out of the exponent range, non-finite ones among them, run in FP64.
 // A gate at a time in FP64 (k_adjoint_step) spends about 26 FP64 multiply-adds
 // per amplitude pair and rotation, one per 75 cycles and warp, and streams both
 // states from HBM for each gate.
@@ -31,6 +34,7 @@ constexpr int kAdjThreads = 256;
 constexpr int kAdjThreadBits = 8;
 constexpr int kAdjAmps = 8;
 constexpr int kAdjWarps = kAdjThreads / 32;
+constexpr int kAdjSpread = 6;  // binary orders
 constexpr int kAdjGrads = 48;  // measurements per launch (a longer window runs as several launches)
 
 struct AdjFixParams {
@@ -115,10 +119,11 @@ __device__ __forceinline__ long long warp_sum(long long s) {
 __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_constant__ AdjFixParams p) {
   constexpr int NT = kAdjThreads, NA = kAdjAmps, T = 1 << kAdjBits;
   extern __shared__ __align__(16) unsigned char adj_raw[];
-  __shared__ uint32_t s_mx[2][kAdjWarps], s_mn[2][kAdjWarps], s_any[kAdjWarps];
+  __shared__ uint32_t s_mx[2][kAdjWarps], s_any[kAdjWarps], s_cnt[kAdjWarps];
   __shared__ double s_red[kAdjWarps][3];
   __shared__ int64_t s_slot[NA];
-  __shared__ int s_grown;
+  __shared__ int s_top[2][3];     // largest component of psi and lambda, by phase
+  __shared__ int s_exp[kAdjGrads];  // halvings of both states before each measurement
   longlong2* tp = reinterpret_cast<longlong2*>(adj_raw);
   longlong2* tl = tp + T;
   const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -136,7 +141,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
     for (int i = kAdjThreadBits; i < kv; ++i) off |= (int64_t)((tid >> (i - kAdjThreadBits)) & 1) << (i < low ? i : p.high[i - low]);
     s_slot[tid] = off;
   }
-  if (tid == 0) s_grown = 0;
+  if (tid < 6) s_top[tid / 3][tid % 3] = 0;
   for (int i = tid; i < 3 * p.num_grads; i += NT) s_sum[i] = 0.0;
   const FixOp* fops = p.fix_ops;
   if (p.num_fix_ops <= kFixSmemOps) {
@@ -147,13 +152,12 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
   }
   __syncthreads();
 
-  bool plain = false;  // this tile's fixed-point run failed its headroom check
-  for (int tix = (int)blockIdx.x; tix < p.num_tiles;) {
+  for (int tix = (int)blockIdx.x; tix < p.num_tiles; tix += (int)gridDim.x) {
     int64_t base = (int64_t)tix << low;
     for (int i = 0; i < nh; ++i) base = insert_zero(base, p.high[i]);
     const int64_t at = base | t_off;
     long long a[2 * NA], b[2 * NA];
-    uint32_t mx[2] = {0, 0}, mn[2] = {~0u, ~0u}, any = 0;
+    uint32_t mx[2] = {0, 0}, any = 0;
 #pragma unroll
     for (int u = 0; u < NA; ++u) {
       const bool valid = (tid + NT * u) >> kv == 0;
@@ -173,38 +177,44 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
       const uint32_t h = max((uint32_t)(a[2 * u] >> 32) & 0x7FFFFFFFu, (uint32_t)(a[2 * u + 1] >> 32) & 0x7FFFFFFFu);
       const uint32_t g = max((uint32_t)(b[2 * u] >> 32) & 0x7FFFFFFFu, (uint32_t)(b[2 * u + 1] >> 32) & 0x7FFFFFFFu);
       mx[0] = max(mx[0], h);
-      mn[0] = min(mn[0], h);
       mx[1] = max(mx[1], g);
-      mn[1] = min(mn[1], g);
       any |= (uint32_t)a[2 * u] | (uint32_t)a[2 * u + 1] | (uint32_t)b[2 * u] | (uint32_t)b[2 * u + 1];
     }
     any = __reduce_or_sync(0xffffffffu, any);
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       mx[s] = __reduce_max_sync(0xffffffffu, mx[s]);
-      mn[s] = __reduce_min_sync(0xffffffffu, mn[s]);
-      if (lane == 0) {
-        s_mx[s][warp] = mx[s];
-        s_mn[s][warp] = mn[s];
-      }
+      if (lane == 0) s_mx[s][warp] = mx[s];
     }
     if (lane == 0) s_any[warp] = any;
     __syncthreads();
 #pragma unroll
     for (int w = 0; w < kAdjWarps; ++w) {
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        mx[s] = max(mx[s], s_mx[s][w]);
-        mn[s] = min(mn[s], s_mn[s][w]);
-      }
+      for (int s = 0; s < 2; ++s) mx[s] = max(mx[s], s_mx[s][w]);
       any |= s_any[w];
     }
     const int ea = (int)(mx[0] >> 20), eb = (int)(mx[1] >> 20);
     const bool zero = mx[0] == 0 && mx[1] == 0 && any == 0;
-    const bool fixed = !plain && ea - (int)(mn[0] >> 20) <= kFixRange && eb - (int)(mn[1] >> 20) <= kFixRange &&
-                       ea > 200 && ea < 1800 && eb > 200 && eb < 1800;
-    plain = false;
-    bool redo = false;
+    bool fixed = ea > 200 && ea < 1800 && eb > 200 && eb < 1800;
+    if (fixed) {
+      // a sixteenth of either state within 2^kAdjSpread of its largest
+      uint32_t cnt = 0;
+#pragma unroll
+      for (int u = 0; u < NA; ++u) {
+        const uint32_t h = max((uint32_t)(a[2 * u] >> 32) & 0x7FFFFFFFu, (uint32_t)(a[2 * u + 1] >> 32) & 0x7FFFFFFFu);
+        const uint32_t g = max((uint32_t)(b[2 * u] >> 32) & 0x7FFFFFFFu, (uint32_t)(b[2 * u + 1] >> 32) & 0x7FFFFFFFu);
+        cnt += (int)(h >> 20) >= ea - kAdjSpread ? 1u : 0u;
+        cnt += (int)(g >> 20) >= eb - kAdjSpread ? 0x10000u : 0u;
+      }
+      cnt = __reduce_add_sync(0xffffffffu, cnt);
+      if (lane == 0) s_cnt[warp] = cnt;
+      __syncthreads();
+      cnt = 0;
+#pragma unroll
+      for (int w = 0; w < kAdjWarps; ++w) cnt += s_cnt[w];
+      fixed = 16 * (cnt & 0xFFFFu) >= (1u << kv) && 16 * (cnt >> 16) >= (1u << kv);
+    }
     if (fixed) {
 #pragma unroll
       for (int u = 0; u < NA; ++u) {
@@ -216,7 +226,8 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
       }
       uint32_t pr[4] = {0, 0, 0, 0};
       uint32_t pbase = 0, cx = 0;
-      bool loaded = false;
+      int phase = -1;              // of the registers
+      int halved = 0, na = 0, nb = 0;  // halvings so far: planned, and of each state
       const longlong2* ahead = nullptr;  // the entries of the table being fetched
       for (int o = 0; o < p.num_fix_ops; ++o) {
         const FixOp* op = fops + o;
@@ -242,9 +253,11 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
               a[j] >>= 1;
               b[j] >>= 1;
             }
+            ++halved;
           }
         } else if (w0.x == FIX_GRAD) {
           FixSum g[3] = {};
+          if (tid == 0) s_exp[w0.z] = 2 * halved + na + nb;
           switch (w0.y & 3) {
             case 0: fix_grad<0>(a, b, g); break;
             case 1: fix_grad<1>(a, b, g); break;
@@ -291,20 +304,20 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
           if ((base >> w0.y) & 1) cx ^= (uint32_t)w0.z;
         } else {  // FIX_PHASE, FIX_END
           const int4 w1 = *(reinterpret_cast<const int4*>(op) + 1);
-          if (loaded) {
-            int hmax = 0, hmin = 0;
+          if (phase >= 0) {
 #pragma unroll
             for (int j = 0; j < NA; ++j) {
               const uint32_t s = fix_reg(pbase, pr, j);
               tp[s] = make_longlong2(a[2 * j], a[2 * j + 1]);
               tl[s] = make_longlong2(b[2 * j], b[2 * j + 1]);
-#pragma unroll
-              for (int c = 0; c < 2; ++c) {
-                hmax = max(hmax, max((int)(a[2 * j + c] >> 32), (int)(b[2 * j + c] >> 32)));
-                hmin = min(hmin, min((int)(a[2 * j + c] >> 32), (int)(b[2 * j + c] >> 32)));
-              }
             }
-            if (hmax >= (1 << (kFixLimitBits - 32)) || hmin < -(1 << (kFixLimitBits - 32))) s_grown = 1;
+            const int ta = __reduce_max_sync(0xffffffffu, fix_top(a)), tb = __reduce_max_sync(0xffffffffu, fix_top(b));
+            if (lane == 0) {
+              atomicMax(&s_top[0][phase % 3], ta);
+              atomicMax(&s_top[1][phase % 3], tb);
+            }
+            // the next phase's words: last read before the barrier before this one
+            if (tid < 2) s_top[tid][(phase + 1) % 3] = 0;
           }
           __syncthreads();
           const uint32_t img[6] = {(uint32_t)w0.y, (uint32_t)w0.z, (uint32_t)w0.w,
@@ -328,18 +341,24 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
             b[2 * j] = w.x;
             b[2 * j + 1] = w.y;
           }
-          loaded = true;
+          if (phase >= 0) {
+            const int sa = fix_renorm(s_top[0][phase % 3]), sb = fix_renorm(s_top[1][phase % 3]);
+            fix_shift(a, sa);
+            fix_shift(b, sb);
+            na += sa;
+            nb += sb;
+          }
+          ++phase;
         }
       }
-      redo = s_grown != 0;  // written before the last barrier, as the sums were
-      if (!redo) {
+      {  // the sums were written before the last barrier
         for (int o = tid; o < p.num_fix_ops; o += NT) {
           const FixOp* op = fops + o;
           if (op->kind != FIX_GRAD) continue;
           double f;
           memcpy(&f, &op->a[3], sizeof(f));
           // product of two fixed-point values / 2^64 -> product of the amplitudes
-          const int e = ea + eb - 2 * 1078 + 64 + 2 * op->a[2];
+          const int e = ea + eb - 2 * 1079 + 64 + s_exp[op->a[1]];
           for (int c = 0; c < 3; ++c) {
             const int i = op->a[1] * 3 + c;
             long long h = 0, r = 0;
@@ -351,7 +370,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
             s_sum[i] += scalbn(fma((double)r, 0x1p-21, (double)h) * f, e);
           }
         }
-        const int ep = ea - 1078 + p.shifts + 1075 + p.scale_exp, el = eb - 1078 + p.shifts + 1075 + p.scale_exp;
+        const int ep = ea - 1079 + p.shifts + na + 1075 + p.scale_exp, el = eb - 1079 + p.shifts + nb + 1075 + p.scale_exp;
 #pragma unroll
         for (int u = 0; u < NA; ++u) {
           if ((tid + NT * u) >> kv) continue;
@@ -423,9 +442,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
       }
     }
     __syncthreads();
-    if (tid == 0) s_grown = 0;
-    if (redo) plain = true;
-    else tix += (int)gridDim.x;
+    if (tid < 6) s_top[tid / 3][tid % 3] = 0;
   }
   __syncthreads();
   for (int i = tid; i < 3 * p.num_grads; i += NT) p.partial[(int64_t)i * p.cols + blockIdx.x] = s_sum[i];

@@ -658,7 +658,7 @@ TmaPassParams tma_params(void* amps, int32_t n, const Pass& ps, const Op* ops_de
 // fixed-point kernel.
 template <typename FB>
 int launch_window_fix(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, const void* phase_tab,
-                      const FixOp* fix_ops, int32_t num_fix_ops, int32_t shifts, const longlong2* fix_tab,
+                      const FixOp* fix_ops, int32_t num_fix_ops, int32_t shifts, uint32_t sparse, const longlong2* fix_tab,
                       cudaStream_t stream) {
   if ((reinterpret_cast<uintptr_t>(amps) & 15u) != 0)
     return set_error(DMV_ERR_INVALID, "statevector not 16-byte aligned");
@@ -671,6 +671,7 @@ int launch_window_fix(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, 
   p.fix_tab = fix_tab;
   p.num_fix_ops = num_fix_ops;
   p.shifts = shifts;
+  p.sparse = sparse;
   const size_t smem = ((size_t)16 << 12) + 1024 + (size_t)8 * kFixThreads * 16 + kFixSmemOps * sizeof(FixOp);
   static bool configured = false;
   if (!configured) {
@@ -857,6 +858,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   // Fixed-point passes: the FixOps of every rewritten pass that the kernel takes.
   std::vector<int64_t> fix_first;
   std::vector<int32_t> fix_count, fix_shifts;
+  std::vector<uint32_t> fix_sparse;
   s->fix_ops.clear();
   for (size_t pi = 0; pi < plan.passes.size(); ++pi) {
     const Pass& ps = plan.passes[pi];
@@ -866,9 +868,10 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       RewrittenPass& r = rewritten[(size_t)rewritten_at[pi]];
       const size_t mark = s->fix_ops.size();
       int32_t shifts = 0;
+      uint32_t sparse = 0;
       // FP32 pairs hold the unscaled values of a pass only to 2^40
       bool fixed = fix && tma_eligible<PolF64>(ps) && (rot_ops || r.scale.hi >= kPairScale) &&
-                   build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), 12, s->fix_ops, &shifts);
+                   build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), 12, s->fix_ops, &shifts, &sparse);
       if (fix && !rot_ops && !fixed) {  // FP32 pairs outside the fixed-point kernel: rotations as real 2x2 ops
         s->fix_ops.resize(mark);
         r = RewrittenPass();
@@ -898,6 +901,8 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       fix_first.resize(passes.size(), -1);
       fix_count.resize(passes.size(), 0);
       fix_shifts.resize(passes.size(), 0);
+      fix_sparse.resize(passes.size(), 0);
+      fix_sparse.push_back(sparse);
       fix_first.push_back(fixed ? (int64_t)mark : -1);
       fix_count.push_back((int32_t)(s->fix_ops.size() - mark));
       fix_shifts.push_back(shifts);
@@ -942,6 +947,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   fix_first.resize(passes.size(), -1);
   fix_count.resize(passes.size(), 0);
   fix_shifts.resize(passes.size(), 0);
+  fix_sparse.resize(passes.size(), 0);
   if (!s->fix_ops.empty()) {
     DMV_TRY(s->fix_ops_dev.reserve(s->fix_ops.size() * sizeof(FixOp)));
     DMV_CUDA_TRY(cudaMemcpyAsync(s->fix_ops_dev.ptr, s->fix_ops.data(), s->fix_ops.size() * sizeof(FixOp),
@@ -1070,9 +1076,9 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
         const FixOp* f = static_cast<const FixOp*>(s->fix_ops_dev.ptr) + fix_first[pi];
         const longlong2* ft = static_cast<const longlong2*>(s->phase_tab_fix_dev.ptr);
         if (arith == ARITH_FP32X2)
-          DMV_TRY(launch_window_fix<PolDF>(a, s->n, ps, ops_dev, phase_tab2_dev, f, fix_count[pi], fix_shifts[pi], ft, st));
+          DMV_TRY(launch_window_fix<PolDF>(a, s->n, ps, ops_dev, phase_tab2_dev, f, fix_count[pi], fix_shifts[pi], fix_sparse[pi], ft, st));
         else
-          DMV_TRY(launch_window_fix<PolF64>(a, s->n, ps, ops_dev, phase_tab_dev, f, fix_count[pi], fix_shifts[pi], ft, st));
+          DMV_TRY(launch_window_fix<PolF64>(a, s->n, ps, ops_dev, phase_tab_dev, f, fix_count[pi], fix_shifts[pi], fix_sparse[pi], ft, st));
       } else if (arith == ARITH_FP32X2)
         DMV_TRY(launch_window_tma<PolDF>(a, s->n, ps, ops_dev, phase_ops_dev, st, phase_tab2_dev, df_fmt));
       else if (arith == ARITH_INT64) DMV_TRY(launch_window_tma<PolFX>(a, s->n, ps, ops_dev, phase_ops_dev, st, phase_tab2_dev));

@@ -2,7 +2,7 @@
 tiles whose amplitudes are of one size) and the tiles that leave them: wide
 ranges, zeros, non-finite values, amplitudes that outgrow the integers.
 
-Tolerance: an output is rounded to 2^-56 of its tile's largest component, in
+Tolerance: an output is rounded to 2^-57 of its tile's largest component, in
 FP64 to 2^-53 of itself, so `count` roundings stay below count * 2^-53 of the
 largest amplitude; the gates' own matrices are rounded the same way.
 """
