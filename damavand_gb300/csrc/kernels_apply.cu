@@ -147,6 +147,7 @@ k_apply_window(typename P::G* __restrict__ a, const WindowParams p) {
   const int T = 1 << p.k;
   const int64_t t_off = tile_thread_offset(p.low, p.nh, p.high);
   tile_slot_offsets(p.low, p.nh, p.high, (T + kTileThreads - 1) >> kTileThreadBits, s_slot);
+  prefetch_ops(p.ops, p.num_ops);
   __syncthreads();
   __shared__ int s_red[kTileThreads / 32];
   for (int64_t tix = blockIdx.x; tix < p.num_tiles; tix += gridDim.x) {
@@ -429,6 +430,7 @@ k_window_tma(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ T
   }
   const int64_t t_off = tile_thread_offset(low, nh, p.high);
   tile_slot_offsets(low, nh, p.high, (T + kTileThreads - 1) >> kTileThreadBits, s_slot);
+  prefetch_ops(p.ops, p.num_ops);
   __syncthreads();
   const TileGeom<ES> geom{low, nh, s_high};
   const int lane = (int)(threadIdx.x & 31);
@@ -557,7 +559,7 @@ struct PhaseSlice {
   uint32_t tpos, rpos;  // the fixed-point table's order: the phase's thread and register bits (FixOp::a[6], a[7])
 };
 constexpr int kPhaseTabThreads = 256;
-constexpr int kPhaseTabEntries = 1024;  // per block
+constexpr int kPhaseTabEntries = 256;  // per block: one per thread, the small tables are all latency
 
 // The entries of the phase tables from their terms, in the forms the pass
 // kernels read: FP64 (t, s) with the quadrant packed, FP32 pairs, Q.54 limbs,

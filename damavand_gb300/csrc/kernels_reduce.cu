@@ -207,26 +207,22 @@ k_chunk_mass_f2(const void* src, int n, int chunk_bits, int64_t num_chunks, doub
   for (int j = 0; j < 4; ++j) rsum[j][threadIdx.x] = f2_val(R[j]);
   __syncthreads();
   double* out = partial + (int64_t)blockIdx.x * (n + 1);
-  const int q = threadIdx.x;
-  if (q < chunk_bits) {
+  // one warp per output (a thread adding the 256 sums one by one took 15 us)
+  for (int q = warp; q <= chunk_bits; q += kRedThreads / 32) {
     double acc = 0.;
-    if (q < 8) {
-      for (int t = 0; t < kRedThreads; ++t)
-        if ((t >> q) & 1) acc += tsum[t];
-    } else {
-      for (int t = 0; t < kRedThreads; ++t) acc += rsum[q - 8][t];
+#pragma unroll
+    for (int i = 0; i < kRedThreads / 32; ++i) {
+      const int t = lane + 32 * i;
+      acc += q == chunk_bits ? tsum[t] : q >= 8 ? rsum[q - 8][t] : ((t >> q) & 1) ? tsum[t] : 0.;
     }
-    out[q] = acc;
-  } else if (q == kRedThreads - 1) {
-    double acc = 0.;
-    for (int t = 0; t < kRedThreads; ++t) acc += tsum[t];
-    out[n] = acc;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) out[q == chunk_bits ? n : q] = acc;
   }
   if (threadIdx.x == 0)
     for (int j = 0; j < n - chunk_bits; ++j) out[chunk_bits + j] = hi_acc[j];
 }
 static_assert((1 << kF2ChunkBits) == kRedThreads * kF2Rows, "a chunk is one amplitude per thread and row");
-static_assert(kF2ChunkBits < kRedThreads - 1, "the total's thread is not a per-bit thread");
 
 // ---------------------------------------------------------------------------
 // k_chunk_mass_bulk: the same pass for states of 12 or more qubits, with one
@@ -530,49 +526,108 @@ __global__ void k_segment_scan(double* __restrict__ seg, int64_t num_chunks, dou
   chunk_mass[c] = run;
 }
 
-// Sum the per-CTA partials in CTA order.
-__global__ void k_reduce_partials(const double* __restrict__ partial, int width, int rows,
-                                  double* __restrict__ out) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= width) return;
-  double acc = 0.;
-  for (int r = 0; r < rows; ++r) acc += partial[(int64_t)r * width + q];
-  out[q] = acc;
+// The sum of v over a warp, to every lane, in a fixed order.
+__device__ __forceinline__ double warp_sum_f64(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-// out[r] = sum_c in[r * cols + c], in column order.
-__global__ void k_reduce_rows(const double* __restrict__ in, int64_t rows, int cols, double* __restrict__ out) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
+// Sums of the per-CTA partials, one CTA per column: serial additions are
+// bound by their latency (152 of them took 19 us).
+constexpr int kPartialThreads = 128;
+__global__ void __launch_bounds__(kPartialThreads)
+k_reduce_partials(const double* __restrict__ partial, int width, int rows, double* __restrict__ out) {
+  __shared__ double red[kPartialThreads / 32];
   double acc = 0.;
-  for (int c = 0; c < cols; ++c) acc += in[r * cols + c];
-  out[r] = acc;
-}
-
-// Inclusive prefix of the chunk masses (one CTA, fixed order).
-__global__ void __launch_bounds__(1024)
-k_scan_chunks(const double* __restrict__ mass, int64_t num_chunks, double* __restrict__ incl) {
-  __shared__ double seg[1024];
-  const int64_t per = (num_chunks + blockDim.x - 1) / blockDim.x;
-  const int64_t b = (int64_t)threadIdx.x * per;
-  const int64_t e = min(num_chunks, b + per);
-  double s = 0.;
-  for (int64_t i = b; i < e; ++i) s += mass[i];
-  seg[threadIdx.x] = s;
+  for (int r = threadIdx.x; r < rows; r += kPartialThreads) acc += partial[(int64_t)r * width + blockIdx.x];
+  acc = warp_sum_f64(acc);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  if (threadIdx.x == 0) {  // 1024 serial adds: negligible next to the pass over HBM
-    double run = 0.;
-    for (int t = 0; t < (int)blockDim.x; ++t) {
-      const double x = seg[t];
-      seg[t] = run;
-      run += x;
+  if (threadIdx.x == 0) out[blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
+}
+
+// out[r] = sum_c in[r * cols + c], one warp per row.
+__global__ void k_reduce_rows(const double* __restrict__ in, int64_t rows, int cols, double* __restrict__ out) {
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (r >= rows) return;
+  const int lane = threadIdx.x & 31;
+  double acc = 0.;
+  for (int c = lane; c < cols; c += 32) acc += in[r * cols + c];
+  acc = warp_sum_f64(acc);
+  if (lane == 0) out[r] = acc;
+}
+
+// Inclusive prefix of the chunk masses, kScanBlock of them per CTA: with one
+// CTA per 4096 the 65,536 chunks of 28 qubits take 7 us instead of the 164 of a
+// single CTA with 1024 serial additions (57 us already at 20 qubits, where one
+// CTA is all there is). k_scan_totals gives each CTA's total, and every CTA
+// adds up the ones before its own.
+constexpr int kScanThreads = 1024;
+constexpr int kScanEach = 4;
+constexpr int kScanBlock = kScanThreads * kScanEach;
+
+// This thread's kScanEach masses (0 past the end) and their sum.
+__device__ __forceinline__ double scan_load(const double* mass, int64_t num_chunks, double (&m)[kScanEach]) {
+  const int64_t b = (int64_t)blockIdx.x * kScanBlock + (int64_t)threadIdx.x * kScanEach;
+#pragma unroll
+  for (int j = 0; j < kScanEach; ++j) m[j] = b + j < num_chunks ? mass[b + j] : 0.;
+  return (m[0] + m[1]) + (m[2] + m[3]);
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+k_scan_totals(const double* __restrict__ mass, int64_t num_chunks, double* __restrict__ totals) {
+  __shared__ double red[32];
+  double m[kScanEach];
+  const double s = warp_sum_f64(scan_load(mass, num_chunks, m));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double t = warp_sum_f64(red[threadIdx.x]);
+    if (threadIdx.x == 0) totals[blockIdx.x] = t;
+  }
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+k_scan_chunks(const double* __restrict__ mass, int64_t num_chunks, const double* __restrict__ totals,
+              double* __restrict__ incl) {
+  __shared__ double red[32], before[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double prior = 0.;
+  for (int c = threadIdx.x; c < (int)blockIdx.x; c += kScanThreads) prior += totals[c];
+  prior = warp_sum_f64(prior);
+  double m[kScanEach];
+  double s = scan_load(mass, num_chunks, m);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double up = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += up;
+  }
+  if (lane == 31) red[warp] = s;
+  if (lane == 0) before[warp] = prior;
+  __syncthreads();
+  if (warp == 0) {
+    double t = red[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double up = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += up;
     }
+    // everything before this warp: the warps before it and the CTAs before this one
+    double excl = __shfl_up_sync(0xffffffffu, t, 1);
+    if (lane == 0) excl = 0.;
+    const double p = warp_sum_f64(before[lane]);
+    red[lane] = p + excl;
   }
   __syncthreads();
-  double run = seg[threadIdx.x];
-  for (int64_t i = b; i < e; ++i) {
-    run += mass[i];
-    incl[i] = run;
+  double prev = __shfl_up_sync(0xffffffffu, s, 1);
+  if (lane == 0) prev = 0.;
+  double run = red[warp] + prev;
+  const int64_t b = (int64_t)blockIdx.x * kScanBlock + (int64_t)threadIdx.x * kScanEach;
+#pragma unroll
+  for (int j = 0; j < kScanEach; ++j) {
+    run += m[j];
+    if (b + j < num_chunks) incl[b + j] = run;
   }
 }
 
@@ -1180,7 +1235,7 @@ int chunk_mass_pass(const void* src, int src_kind, int n, DeviceBuffer& reduce_d
   double* partial = static_cast<double*>(reduce_dev.ptr);
   double* sums = partial + partial_elems;
   launch_mass_kernel(src, src_kind, n, cb, num_chunks, grid, partial, stream);
-  k_reduce_partials<<<1, 64, 0, stream>>>(partial, n + 1, grid, sums);
+  k_reduce_partials<<<n + 1, kPartialThreads, 0, stream>>>(partial, n + 1, grid, sums);
   count_launch(2);
   DMV_CUDA_TRY(cudaGetLastError());
   *sums_dev_out = sums;
@@ -1205,11 +1260,13 @@ int sample_prefix_pass(const void* src, int src_kind, int n, DeviceBuffer& prefi
   sp.chunk_bits = bulk ? kMbChunkBits : chunk_bits_for(n);
   sp.num_chunks = int64_t(1) << (n - sp.chunk_bits);
   const int64_t nseg = int64_t(1) << (n - sp.seg_bits);
-  DMV_TRY(prefix.reserve((size_t)(2 * sp.num_chunks + nseg) * sizeof(double) +
+  const int64_t scan_ctas = (sp.num_chunks + kScanBlock - 1) / kScanBlock;
+  DMV_TRY(prefix.reserve((size_t)(2 * sp.num_chunks + scan_ctas + nseg) * sizeof(double) +
                          (size_t)(sp.num_chunks + 1) * sizeof(int32_t)));
   double* mass = static_cast<double*>(prefix.ptr);
   double* incl = mass + sp.num_chunks;
-  double* seg = incl + sp.num_chunks;
+  double* totals = incl + sp.num_chunks;
+  double* seg = totals + scan_ctas;
   int32_t* guide = reinterpret_cast<int32_t*>(seg + nseg);
   if (bulk) {
     const int grid = mass_grid_for(src_kind, n, sp.num_chunks);
@@ -1225,7 +1282,11 @@ int sample_prefix_pass(const void* src, int src_kind, int n, DeviceBuffer& prefi
     }
     count_launch();
   }
-  k_scan_chunks<<<1, 1024, 0, stream>>>(mass, sp.num_chunks, incl);
+  if (scan_ctas > 1) {
+    k_scan_totals<<<(int)scan_ctas, kScanThreads, 0, stream>>>(mass, sp.num_chunks, totals);
+    count_launch();
+  }
+  k_scan_chunks<<<(int)scan_ctas, kScanThreads, 0, stream>>>(mass, sp.num_chunks, totals, incl);
   const int gg = (int)std::max<int64_t>(1, std::min<int64_t>((sp.num_chunks + 256) / 256, (int64_t)sm_count() * 4));
   k_chunk_guide<<<gg, 256, 0, stream>>>(incl, sp.num_chunks, sp.num_chunks, guide);
   count_launch(2);
@@ -1285,7 +1346,7 @@ int launch_chunk_mass_into(const void* src, int src_kind, int n, double* partial
     return set_error(DMV_ERR_INVALID, "launch_chunk_mass_into takes amplitudes (kinds 0, 1)");
   const ChunkMassShape sh = chunk_mass_shape(n);
   launch_mass_kernel(src, src_kind, n, sh.chunk_bits, sh.num_chunks, sh.grid, partial, stream);
-  k_reduce_partials<<<1, 64, 0, stream>>>(partial, n + 1, sh.grid, sums);
+  k_reduce_partials<<<n + 1, kPartialThreads, 0, stream>>>(partial, n + 1, sh.grid, sums);
   count_launch(2);
   DMV_CUDA_TRY(cudaGetLastError());
   return DMV_OK;
@@ -1395,7 +1456,7 @@ int launch_inner_product(dmv_state_s* a, dmv_state_s* b, double* re, double* im)
   else
     k_inner<float2><<<grid, kRedThreads, 0, a->stream>>>(static_cast<const float2*>(a->amps),
                                                         static_cast<const float2*>(b->amps), a->N, partial);
-  k_reduce_partials<<<1, 64, 0, a->stream>>>(partial, 2, grid, sums);
+  k_reduce_partials<<<2, kPartialThreads, 0, a->stream>>>(partial, 2, grid, sums);
   count_launch(2);
   DMV_CUDA_TRY(cudaGetLastError());
   double h[2];
@@ -1497,7 +1558,7 @@ int adjoint_sweep_windows(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, co
 }
 
 int launch_reduce_rows(const double* in, int64_t rows, int cols, double* out, cudaStream_t stream) {
-  k_reduce_rows<<<(int)((rows + 127) / 128), 128, 0, stream>>>(in, rows, cols, out);
+  k_reduce_rows<<<(int)((rows + 3) / 4), 128, 0, stream>>>(in, rows, cols, out);
   count_launch();
   DMV_CUDA_TRY(cudaGetLastError());
   return DMV_OK;
@@ -1603,7 +1664,7 @@ int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const doubl
       rc = launch_adjoint_step_impl(psi, lam, op, last ? 0 : 1, slot, df_raw);
     }
     if (rc != DMV_OK) break;
-    k_reduce_rows<<<(int)((num_params + 127) / 128), 128, 0, s->stream>>>(part, num_params, grid, out);
+    k_reduce_rows<<<(int)((num_params + 3) / 4), 128, 0, s->stream>>>(part, num_params, grid, out);
     count_launch();
     if (cudaMemcpyAsync(grads, out, (size_t)num_params * sizeof(double), cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
         cudaStreamSynchronize(s->stream) != cudaSuccess) {

@@ -461,6 +461,14 @@ __device__ __forceinline__ void tile_phase_fx(longlong2* tile, int T, const Op& 
   }
 }
 
+// Brings a pass's ops into this SM's L1 at once: read one after the other as
+// they are applied, each costs the L2's latency (a 10-qubit state's 90 ops).
+__device__ __forceinline__ void prefetch_ops(const Op* ops, int num_ops) {
+  const char* p = reinterpret_cast<const char*>(ops);
+  for (int i = (int)threadIdx.x * 128; i < num_ops * (int)sizeof(Op); i += (int)blockDim.x * 128)
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + i));
+}
+
 // Every op of a pass on one tile; `base` holds the tile's global index bits
 // (controls outside the tile are read from it). Ends with a barrier after
 // each applied op. `tab` holds the phase tables of OP_PHASE ops in the
