@@ -259,12 +259,12 @@ void phase_entries(const PhaseTables& tabs, std::vector<PhaseEntry>& out) {
 }
 
 void rewrite_passes(const Plan& plan, const std::vector<int64_t>& which, bool rot_ops,
-                    std::vector<RewrittenPass>& out) {
+                    std::vector<RewrittenPass>& out, bool single) {
   out.assign(which.size(), RewrittenPass());
   for (size_t j = 0; j < which.size(); ++j) {
     const Pass& ps = plan.passes[(size_t)which[j]];
     rewrite_pass_rotations(plan.ops.data() + ps.op_begin, ps.op_count, ps.low_bits + ps.num_high, rot_ops,
-                           out[j].ops, out[j].tab, &out[j].scale);
+                           out[j].ops, out[j].tab, &out[j].scale, single);
   }
 }
 
@@ -289,7 +289,7 @@ void phase_tables_f64(const std::vector<PhaseEntry>& in, std::vector<double2>& o
 }
 
 int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot_ops, std::vector<Op>& dst,
-                               PhaseTables& tab, ScaleDD* scale) {
+                               PhaseTables& tab, ScaleDD* scale, bool single) {
   std::vector<DiagTable> tables;  // flushes in time order; tables[0] may sit at the pass start
   bool start_table = false;
   std::vector<Item> items;
@@ -399,7 +399,7 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
         // as the real 2x2 acc f M instead (8 multiply-adds per pair), which
         // gives the state its true scale back.
         (void)Tq;
-        const double w = Sq / Cq;
+        const double w = single ? (double)(float)(Sq / Cq) : Sq / Cq;
         const long double wl = w;
         const double f = (double)(1.0L / std::sqrt(1.0L + wl * wl));
         if (acc.hi * f >= 0x1p-200) {

@@ -18,12 +18,13 @@ struct SlotMap {
   int32_t img[kMaxTileBits];
 };
 
-int rank3(const int32_t* v, int n) {
-  int32_t basis[3] = {0, 0, 0};
+// Rank over GF(2) of the slots v modulo a row of 2^row_bits.
+int row_rank(const int32_t* v, int n, int row_bits) {
+  int32_t basis[4] = {0, 0, 0, 0};
   int r = 0;
   for (int i = 0; i < n; ++i) {
-    int32_t x = v[i] & 7;
-    for (int b = 2; b >= 0; --b)
+    int32_t x = v[i] & ((1 << row_bits) - 1);
+    for (int b = row_bits - 1; b >= 0; --b)
       if ((x >> b) & 1) {
         if (basis[b]) x ^= basis[b];
         else {
@@ -40,18 +41,17 @@ void pack_images(FixOp& op, const int32_t* slot12) {
   for (int i = 0; i < 6; ++i) op.a[i] = slot12[2 * i] | (slot12[2 * i + 1] << 16);
 }
 
-// Thread bits of a phase: the tile bits outside `regs`, the first three chosen
-// so that eight consecutive lanes' 16-byte accesses meet all 32 banks (their
-// slots differ in three independent ways modulo 8), low bits first: those also
-// read consecutive table entries.
-void thread_bits(const SlotMap& m, int tile_bits, uint32_t regs, int32_t* bits) {
+// Thread bits of a phase: the tile bits outside `regs`, the first row_bits
+// chosen so that the lanes of one 128-byte access meet all 32 banks (their
+// slots differ in as many independent ways modulo a row).
+void thread_bits(const SlotMap& m, int tile_bits, int row_bits, uint32_t regs, int32_t* bits) {
   int n = 0;
   uint32_t used = regs;
-  int32_t pick[3];
-  for (int b = 0; b < tile_bits && n < 3; ++b) {
+  int32_t pick[4];
+  for (int b = 0; b < tile_bits && n < row_bits; ++b) {
     if ((used >> b) & 1u) continue;
     pick[n] = m.img[b];
-    if (rank3(pick, n + 1) != n + 1) continue;
+    if (row_rank(pick, n + 1, row_bits) != n + 1) continue;
     bits[n++] = b;
     used |= 1u << b;
   }
@@ -74,13 +74,13 @@ bool split_multiplier(double w, int32_t& hi, int32_t& lo) {
 }  // namespace
 
 bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector<FixOp>& out, int32_t* shifts,
-                    uint32_t* sparse) {
+                    uint32_t* sparse, bool single) {
   const int32_t reg_bits = tile_bits - kThreadBits;
   const uint32_t all_bits = (1u << tile_bits) - 1u;
   const size_t mark = out.size();
   *shifts = 0;
   SlotMap m;
-  for (int b = 0; b < tile_bits; ++b) m.img[b] = fix_slot_host(1 << b);
+  for (int b = 0; b < tile_bits; ++b) m.img[b] = single ? fix_slot8_host(1 << b) : fix_slot_host(1 << b);
   auto blank = [](int32_t kind) {
     FixOp f;
     std::memset(&f, 0, sizeof(f));
@@ -166,6 +166,12 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
         f.a[0] = op.target;  // the register bit once the phase is complete
         const double w = op.m[0];
         if (w != 0.0) least[op.target] = std::min(least[op.target], std::fabs(w));
+        if (single) {
+          const float wf = (float)w;
+          std::memcpy(&f.a[1], &wf, sizeof(wf));
+          taken.push_back(f);
+          continue;
+        }
         if (!split_multiplier(w, f.a[1], f.a[2])) {
           f.a[0] |= kFixComplement << 8;
           if (!split_multiplier(1.0 - w, f.a[1], f.a[2])) {
@@ -197,7 +203,7 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
         regs |= 1u << b;
       }
     int32_t tbits[kThreadBits], slots[kMaxTileBits] = {};
-    thread_bits(m, tile_bits, regs, tbits);
+    thread_bits(m, tile_bits, single ? 4 : 3, regs, tbits);
     FixOp ph = blank(FIX_PHASE);
     for (int i = 0; i < reg_bits; ++i) slots[i] = m.img[reg[i]];
     for (int i = 0; i < kThreadBits; ++i) slots[kMaxFixRegBits + i] = m.img[tbits[i]];

@@ -208,7 +208,7 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
           const int4 w1 = *(reinterpret_cast<const int4*>(op) + 1);
           if (phase >= 0) {
 #pragma unroll
-            for (int j = 0; j < kFixAmps; ++j) ti[fix_reg(pbase, pr, j)] = make_longlong2(r[2 * j], r[2 * j + 1]);
+            for (int j = 0; j < kFixAmps; ++j) *reinterpret_cast<longlong2*>(tile + fix_reg(pbase, pr, j)) = make_longlong2(r[2 * j], r[2 * j + 1]);
             const int top = __reduce_max_sync(0xffffffffu, fix_top(r));
             if (lane == 0) atomicMax(&s_top[phase % 3], top);
             // the next phase's word: last read before the barrier before this one
@@ -217,10 +217,11 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
           __syncthreads();
           const uint32_t img[6] = {(uint32_t)w0.y, (uint32_t)w0.z, (uint32_t)w0.w,
                                    (uint32_t)w1.x, (uint32_t)w1.y, (uint32_t)w1.z};
-          pr[0] = img[0] & 0xFFFFu;
-          pr[1] = img[0] >> 16;
-          pr[2] = img[1] & 0xFFFFu;
-          pr[3] = img[1] >> 16;
+          // as byte offsets
+          pr[0] = (img[0] & 0xFFFFu) << 4;
+          pr[1] = img[0] >> 16 << 4;
+          pr[2] = (img[1] & 0xFFFFu) << 4;
+          pr[3] = img[1] >> 16 << 4;
           cx ^= (uint32_t)op->a[8];
           pbase = cx;
 #pragma unroll
@@ -228,9 +229,10 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
             const uint32_t im = (b & 1) ? img[2 + b / 2] >> 16 : img[2 + b / 2] & 0xFFFFu;
             if ((tid >> b) & 1) pbase ^= im;
           }
+          pbase <<= 4;
 #pragma unroll
           for (int j = 0; j < kFixAmps; ++j) {
-            const longlong2 v = ti[fix_reg(pbase, pr, j)];
+            const longlong2 v = *reinterpret_cast<const longlong2*>(tile + fix_reg(pbase, pr, j));
             r[2 * j] = v.x;
             r[2 * j + 1] = v.y;
           }

@@ -207,8 +207,9 @@ struct ScaleDD {
     lo = l - (hi - p);
   }
 };
+// `single`: w rounded to FP32 (its factor f to match).
 int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot_ops, std::vector<Op>& dst,
-                               PhaseTables& tab, ScaleDD* scale = nullptr);
+                               PhaseTables& tab, ScaleDD* scale = nullptr, bool single = false);
 // The entries of tables, on the host (the debug check; launch_plan has
 // k_phase_tables make them).
 void phase_entries(const PhaseTables& tabs, std::vector<PhaseEntry>& out);
@@ -303,7 +304,7 @@ struct RewrittenPass {
   ScaleDD scale;
 };
 void rewrite_passes(const Plan& plan, const std::vector<int64_t>& which, bool rot_ops,
-                    std::vector<RewrittenPass>& out);
+                    std::vector<RewrittenPass>& out, bool single = false);
 
 // ---------------------------------------------------------------------------
 // Tensor-core window passes (ARITH_TC, complex128 storage).
@@ -400,8 +401,12 @@ inline int32_t fix_slot_host(int32_t l) { return l ^ (((l >> 3) ^ (l >> 6) ^ (l 
 // amplitude that spreads from a nonzero one over z bits stays within that
 // range of it, and z is at most kFixUnreached (a tile of 2^(12-z) nonzero
 // amplitudes rounds every one of 2^12).
+// `single`: complex64 tiles (8-byte elements, fix_slot8), the rotations' w as
+// floats in a[1], no halvings.
 bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector<FixOp>& out, int32_t* shifts,
-                    uint32_t* sparse = nullptr);
+                    uint32_t* sparse = nullptr, bool single = false);
+// Slot of an 8-byte element: the same for the 16 of a row and groups of 4 bits.
+inline int32_t fix_slot8_host(int32_t l) { return l ^ (((l >> 4) ^ (l >> 8)) & 15); }
 constexpr int kFixUnreached = 4;
 constexpr int kFixRange = 12;  // binary orders between a fixed-point tile's largest and smallest amplitude
 // Where make_phase_tables puts each form of the tables' entries (null: nowhere).
@@ -410,6 +415,7 @@ struct PhaseTableForms {
   float4* df = nullptr;
   int4* fx = nullptr;
   longlong2* fix = nullptr;  // in the order of fix_ops
+  float2* f32 = nullptr;     // the same, single precision
 };
 struct DeviceBuffer;
 // Makes the entries of `tabs` on the device (k_phase_tables). `src`, `src_dev`

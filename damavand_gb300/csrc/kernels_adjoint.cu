@@ -307,9 +307,9 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
           if (phase >= 0) {
 #pragma unroll
             for (int j = 0; j < NA; ++j) {
-              const uint32_t s = fix_reg(pbase, pr, j);
-              tp[s] = make_longlong2(a[2 * j], a[2 * j + 1]);
-              tl[s] = make_longlong2(b[2 * j], b[2 * j + 1]);
+              unsigned char* q = adj_raw + fix_reg(pbase, pr, j);
+              *reinterpret_cast<longlong2*>(q) = make_longlong2(a[2 * j], a[2 * j + 1]);
+              *reinterpret_cast<longlong2*>(q + T * 16) = make_longlong2(b[2 * j], b[2 * j + 1]);
             }
             const int ta = __reduce_max_sync(0xffffffffu, fix_top(a)), tb = __reduce_max_sync(0xffffffffu, fix_top(b));
             if (lane == 0) {
@@ -322,9 +322,10 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
           __syncthreads();
           const uint32_t img[6] = {(uint32_t)w0.y, (uint32_t)w0.z, (uint32_t)w0.w,
                                    (uint32_t)w1.x, (uint32_t)w1.y, (uint32_t)w1.z};
-          pr[0] = img[0] & 0xFFFFu;
-          pr[1] = img[0] >> 16;
-          pr[2] = img[1] & 0xFFFFu;
+          // as byte offsets
+          pr[0] = (img[0] & 0xFFFFu) << 4;
+          pr[1] = img[0] >> 16 << 4;
+          pr[2] = (img[1] & 0xFFFFu) << 4;
           cx ^= (uint32_t)op->a[8];
           pbase = cx;
 #pragma unroll
@@ -332,10 +333,12 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
             const uint32_t im = (i & 1) ? img[2 + i / 2] >> 16 : img[2 + i / 2] & 0xFFFFu;
             if ((tid >> i) & 1) pbase ^= im;
           }
+          pbase <<= 4;
 #pragma unroll
           for (int j = 0; j < NA; ++j) {
-            const uint32_t s = fix_reg(pbase, pr, j);
-            const longlong2 v = tp[s], w = tl[s];
+            const unsigned char* q = adj_raw + fix_reg(pbase, pr, j);
+            const longlong2 v = *reinterpret_cast<const longlong2*>(q);
+            const longlong2 w = *reinterpret_cast<const longlong2*>(q + T * 16);
             a[2 * j] = v.x;
             a[2 * j + 1] = v.y;
             b[2 * j] = w.x;

@@ -563,12 +563,12 @@ constexpr int kPhaseTabEntries = 256;  // per block: one per thread, the small t
 
 // The entries of the phase tables from their terms, in the forms the pass
 // kernels read: FP64 (t, s) with the quadrant packed, FP32 pairs, Q.54 limbs,
-// and the fixed-point kernel's Q.62 (cos, sin), each where its pointer is set.
+// the fixed-point kernel's Q.62 (cos, sin) and the complex64 one's, each where
+// its pointer is set.
 // About 60 FP64 operations an entry: 30 us for the 24-qubit, 10-layer
 // forward's 230,000 entries, against 6 ms when the host made and uploaded them.
 __global__ void __launch_bounds__(kPhaseTabThreads)
-k_phase_tables(const PhaseSlice* __restrict__ slices, const PhaseTerm* __restrict__ terms, double2* f64, float4* df,
-               int4* fx, longlong2* fix) {
+k_phase_tables(const PhaseSlice* __restrict__ slices, const PhaseTerm* __restrict__ terms, const PhaseTableForms f) {
   const PhaseSlice sl = slices[blockIdx.x];
   const uint32_t first = blockIdx.y * kPhaseTabEntries;
   const uint32_t end = min(first + (uint32_t)kPhaseTabEntries, 1u << sl.k);
@@ -594,28 +594,31 @@ k_phase_tables(const PhaseSlice* __restrict__ slices, const PhaseTerm* __restric
     sincospi(r * 0x1p-64, &sh, &ch);  // half the angle
     const double t = -sh / ch, sn = 2.0 * sh * ch, cs = fma(-2.0 * sh, sh, 1.0);
     const int64_t at = sl.entry + l;
-    if (f64)
-      f64[at] = make_double2(__hiloint2double(__double2hiint(t) | (int)((q & 1u) << 30), __double2loint(t)),
+    if (f.f64)
+      f.f64[at] = make_double2(__hiloint2double(__double2hiint(t) | (int)((q & 1u) << 30), __double2loint(t)),
                              __hiloint2double(__double2hiint(sn) | (int)((q >> 1) << 30), __double2loint(sn)));
     const double x = (q & 1u) ? sn : cs, y = (q & 1u) ? cs : sn;
     const double re = (q == 1u || q == 2u) ? -x : x, im = q >= 2u ? -y : y;
-    if (df) {
+    if (f.df) {
       const float rh = (float)re, ih = (float)im;
-      df[at] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
+      f.df[at] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
     }
-    if (fx) {
+    if (f.fx) {
       const long long fr = llrint(re * 0x1p54), fi = llrint(im * 0x1p54);
-      fx[at] = make_int4((int)(fr >> 31), (int)(fr & 0x7FFFFFFFll), (int)(fi >> 31), (int)(fi & 0x7FFFFFFFll));
+      f.fx[at] = make_int4((int)(fr >> 31), (int)(fr & 0x7FFFFFFFll), (int)(fi >> 31), (int)(fi & 0x7FFFFFFFll));
     }
-    if (fix) {  // the low words taken as signed
+    if (f.f32)  // two registers to a thread's load
+      f.f32[sl.entry + ((i >> 9) << 9 | (i & 255u) << 1 | ((i >> 8) & 1u))] = make_float2((float)re, (float)im);
+    if (f.fix) {  // the low words taken as signed
       const long long fr = llrint(re * 0x1p62), fi = llrint(im * 0x1p62);
-      fix[sl.entry + i] = make_longlong2(fr + ((fr & 0x80000000ll) << 1), fi + ((fi & 0x80000000ll) << 1));
+      f.fix[sl.entry + i] = make_longlong2(fr + ((fr & 0x80000000ll) << 1), fi + ((fi & 0x80000000ll) << 1));
     }
   }
 }
 
-// The fixed-point window pass of complex128 states.
+// The fixed-point window pass of complex128 states, and the same phases for complex64.
 #include "fix_window.cuh"
+#include "f32_window.cuh"
 
 // TMA kernels by policy: register phases for complex64 (FP32 arithmetic),
 // the shared-memory op loop for complex128 in FP64. The complex128 FP32-pair
@@ -685,6 +688,30 @@ int launch_window_fix(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, 
   if (per_sm < 1) return set_error(DMV_ERR_CUDA, "fixed-point kernel cannot fit %zu bytes of shared memory", smem);
   const int64_t grid = std::min<int64_t>(p.t.num_tiles, (int64_t)per_sm * num_sms());
   k_window_fix<FB><<<(int)grid, kFixThreads, smem, stream>>>(map, p);
+  return DMV_OK;
+}
+
+// A rewritten complex64 pass.
+int launch_window_f32(void* amps, int32_t n, const Pass& ps, const FixOp* fix_ops, int32_t num_fix_ops,
+                      const float2* tab, float out_scale, cudaStream_t stream) {
+  F32PassParams p;
+  p.amps = static_cast<float2*>(amps);
+  p.low = ps.low_bits;
+  p.nh = ps.num_high;
+  for (int i = 0; i < 16; ++i) p.high[i] = i < ps.num_high ? ps.high[i] : 0;
+  p.num_ops = num_fix_ops;
+  p.out_scale = out_scale;
+  p.num_tiles = int64_t(1) << (n - ps.low_bits - ps.num_high);
+  p.ops = fix_ops;
+  p.tab = tab;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(k_window_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF32Smem);
+  (void)attr;  // a refusal shows as the launch's error
+  int per_sm = 0;
+  DMV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_window_f32, kF32Threads, kF32Smem));
+  if (per_sm < 1) return set_error(DMV_ERR_CUDA, "complex64 window kernel cannot fit %zu bytes", kF32Smem);
+  const int64_t grid = std::min<int64_t>(p.num_tiles, (int64_t)per_sm * num_sms());
+  k_window_f32<<<(int)grid, kF32Threads, kF32Smem, stream>>>(p);
   return DMV_OK;
 }
 
@@ -812,8 +839,7 @@ int make_phase_tables(const PhaseTables& tabs, const std::vector<FixOp>& fix_ops
   const dim3 grid((unsigned)slices.size(), (unsigned)(((1 << kmax) + kPhaseTabEntries - 1) / kPhaseTabEntries));
   k_phase_tables<<<grid, kPhaseTabThreads, 0, stream>>>(
       static_cast<const PhaseSlice*>(src_dev.ptr),
-      reinterpret_cast<const PhaseTerm*>(static_cast<const char*>(src_dev.ptr) + sb), forms.f64, forms.df, forms.fx,
-      forms.fix);
+      reinterpret_cast<const PhaseTerm*>(static_cast<const char*>(src_dev.ptr) + sb), forms);
   count_launch();
   DMV_CUDA_TRY(cudaGetLastError());
   return DMV_OK;
@@ -839,7 +865,8 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   const bool c128 = s->precision == DMV_C128;
   const bool rewrite = c128 && ((s->arith == ARITH_FP64 && s->fp64_rewrite) || s->arith == ARITH_FP32X2 ||
                                 s->arith == ARITH_INT64);
-  const bool rot_ops = s->arith == ARITH_FP64;
+  const bool single = !c128 && s->n >= 12;  // complex64 passes as rotations and tables
+  const bool rot_ops = single || s->arith == ARITH_FP64;
   const bool fix = rewrite && s->arith != ARITH_INT64 && s->n >= 12;  // fixed-point passes where the kernel takes them
   s->phase_tabs = PhaseTables();
   // Per staged pass, the product of its OP_ROT factors (1 elsewhere).
@@ -848,38 +875,45 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   // The passes' tables are appended in pass order with the OP_PHASE offsets moved.
   std::vector<RewrittenPass> rewritten;
   std::vector<int64_t> rewritten_at(plan.passes.size(), -1);
-  if (rewrite) {
+  if (rewrite || single) {
     std::vector<int64_t> which;
     for (size_t i = 0; i < plan.passes.size(); ++i)
       if (plan.passes[i].kind == 1) {
         rewritten_at[i] = (int64_t)which.size();
         which.push_back((int64_t)i);
       }
-    rewrite_passes(plan, which, rot_ops || fix, rewritten);
+    rewrite_passes(plan, which, rot_ops || fix, rewritten, single);
   }
   // Fixed-point passes: the FixOps of every rewritten pass that the kernel takes.
   std::vector<int64_t> fix_first;
   std::vector<int32_t> fix_count, fix_shifts;
   std::vector<uint32_t> fix_sparse;
+  std::vector<double> single_scale;  // complex64 passes: the product of their rotation factors
   s->fix_ops.clear();
   for (size_t pi = 0; pi < plan.passes.size(); ++pi) {
     const Pass& ps = plan.passes[pi];
     const int rb = ps.kind == 1 ? window_reg_bits(s, ps) : 0;
-    any_window |= ps.kind == 1;
-    if (rewritten_at[pi] >= 0) {
+    bool fixed = false;
+    const size_t mark = s->fix_ops.size();
+    int32_t shifts = 0;
+    uint32_t sparse = 0;
+    if ((single || fix) && rewritten_at[pi] >= 0) {
       RewrittenPass& r = rewritten[(size_t)rewritten_at[pi]];
-      const size_t mark = s->fix_ops.size();
-      int32_t shifts = 0;
-      uint32_t sparse = 0;
-      // FP32 pairs hold the unscaled values of a pass only to 2^40
-      bool fixed = fix && tma_eligible<PolF64>(ps) && (rot_ops || r.scale.hi >= kPairScale) &&
-                   build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), 12, s->fix_ops, &shifts, &sparse);
-      if (fix && !rot_ops && !fixed) {  // FP32 pairs outside the fixed-point kernel: rotations as real 2x2 ops
-        s->fix_ops.resize(mark);
+      // complex64 states and FP32 pairs hold the unscaled values of a pass only to 2^40
+      const bool in_range = (fix && rot_ops) || r.scale.hi >= kPairScale;
+      const bool eligible = single ? tma_eligible<PolF32>(ps) : tma_eligible<PolF64>(ps);
+      fixed = in_range && eligible &&
+              build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), 12, s->fix_ops, &shifts, &sparse, single);
+      if (single && !fixed) rewritten_at[pi] = -1;  // its gates as complex 2x2s
+      if (!single && !rot_ops && !fixed) {  // FP32 pairs outside the fixed-point kernel: rotations as real 2x2 ops
         r = RewrittenPass();
         rewrite_pass_rotations(plan.ops.data() + ps.op_begin, ps.op_count, ps.low_bits + ps.num_high, false, r.ops,
                                r.tab, &r.scale);
       }
+    }
+    any_window |= ps.kind == 1 && !(single && fixed);
+    if (rewritten_at[pi] >= 0) {
+      const RewrittenPass& r = rewritten[(size_t)rewritten_at[pi]];
       Pass rw = ps;
       rw.op_begin = (int64_t)ops.size();
       rw.op_count = (int64_t)r.ops.size();
@@ -909,7 +943,9 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       fix_count.push_back((int32_t)(s->fix_ops.size() - mark));
       fix_shifts.push_back(shifts);
       passes.push_back(rw);
-      pass_scale.push_back(r.scale);
+      pass_scale.push_back(single ? ScaleDD() : r.scale);
+      single_scale.resize(passes.size(), 1.0);
+      single_scale.back() = r.scale.hi;
       continue;
     }
     if (rb <= 0) {
@@ -950,6 +986,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   fix_count.resize(passes.size(), 0);
   fix_shifts.resize(passes.size(), 0);
   fix_sparse.resize(passes.size(), 0);
+  single_scale.resize(passes.size(), 1.0);
   if (!s->fix_ops.empty()) {
     DMV_TRY(s->fix_ops_dev.reserve(s->fix_ops.size() * sizeof(FixOp)));
     DMV_CUDA_TRY(cudaMemcpyAsync(s->fix_ops_dev.ptr, s->fix_ops.data(), s->fix_ops.size() * sizeof(FixOp),
@@ -963,21 +1000,26 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   int64_t tab_bytes = 0;
   const PhaseTables& tabs = s->phase_tabs;
   if (tabs.entries > 0) {
-    const size_t bytes = (size_t)tabs.entries * 16;  // every form has 16 bytes an entry
-    if (s->arith != ARITH_FP32X2) {
-      DMV_TRY(s->phase_tab_dev.reserve(bytes));
-      phase_tab_dev = s->phase_tab_dev.ptr;
-    }
-    if (s->arith == ARITH_FP32X2 || s->arith == ARITH_INT64) {
-      DMV_TRY(s->phase_tab2_dev.reserve(bytes));
-      phase_tab2_dev = s->phase_tab2_dev.ptr;
-    }
-    if (!s->fix_ops.empty()) DMV_TRY(s->phase_tab_fix_dev.reserve(bytes));
+    const size_t bytes = (size_t)tabs.entries * 16;  // every complex128 form has 16 bytes an entry
     PhaseTableForms forms;
-    forms.f64 = static_cast<double2*>(s->arith == ARITH_FP32X2 ? nullptr : s->phase_tab_dev.ptr);
-    forms.df = static_cast<float4*>(s->arith == ARITH_FP32X2 ? s->phase_tab2_dev.ptr : nullptr);
-    forms.fx = static_cast<int4*>(s->arith == ARITH_INT64 ? s->phase_tab2_dev.ptr : nullptr);
-    forms.fix = static_cast<longlong2*>(s->fix_ops.empty() ? nullptr : s->phase_tab_fix_dev.ptr);
+    if (single) {
+      DMV_TRY(s->phase_tab_fix_dev.reserve((size_t)tabs.entries * sizeof(float2)));
+      forms.f32 = static_cast<float2*>(s->phase_tab_fix_dev.ptr);
+    } else {
+      if (s->arith != ARITH_FP32X2) {
+        DMV_TRY(s->phase_tab_dev.reserve(bytes));
+        phase_tab_dev = s->phase_tab_dev.ptr;
+      }
+      if (s->arith == ARITH_FP32X2 || s->arith == ARITH_INT64) {
+        DMV_TRY(s->phase_tab2_dev.reserve(bytes));
+        phase_tab2_dev = s->phase_tab2_dev.ptr;
+      }
+      if (!s->fix_ops.empty()) DMV_TRY(s->phase_tab_fix_dev.reserve(bytes));
+      forms.f64 = static_cast<double2*>(s->arith == ARITH_FP32X2 ? nullptr : s->phase_tab_dev.ptr);
+      forms.df = static_cast<float4*>(s->arith == ARITH_FP32X2 ? s->phase_tab2_dev.ptr : nullptr);
+      forms.fx = static_cast<int4*>(s->arith == ARITH_INT64 ? s->phase_tab2_dev.ptr : nullptr);
+      forms.fix = static_cast<longlong2*>(s->fix_ops.empty() ? nullptr : s->phase_tab_fix_dev.ptr);
+    }
     DMV_TRY(make_phase_tables(tabs, s->fix_ops, forms, s->phase_src, s->phase_src_dev, s->stream));
     tab_bytes = (int64_t)s->phase_src.size();
   }
@@ -1025,6 +1067,10 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   // values could have grown past 2^200 (FP32 pairs: 2^40, twice that stays in
   // FP32's range with the pairs' 48 bits).
   ScaleDD owed;
+  double stored = 1.0;  // complex64
+  int64_t last_single = -1;
+  for (size_t pi = 0; pi < passes.size(); ++pi)
+    if (single && fix_first[pi] >= 0) last_single = (int64_t)pi;
   const double owed_min = rot_ops ? 0x1p-200 : kPairScale;
   for (size_t pi = 0; pi < passes.size(); ++pi) {
     if (pi > 0) {
@@ -1073,7 +1119,14 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       const int64_t tok = prof_begin(DMV_KERNEL_WINDOW, s->stream, (double)(2 * S), fmas);
       void* a = s->amps;
       cudaStream_t st = s->stream;
-      if (s->precision == DMV_C64) DMV_TRY(launch_window_tma<PolF32>(a, s->n, ps, ops_dev, phase_ops_dev, st));
+      if (single && fix_first[pi] >= 0) {
+        // the stored state is the true one times `stored`, in [1, 2) until the last such pass makes it 1
+        const double raw = stored / single_scale[pi];
+        const double out = (int64_t)pi == last_single ? 1.0 / raw : std::ldexp(1.0, -std::ilogb(raw));
+        stored = raw * out;
+        DMV_TRY(launch_window_f32(a, s->n, ps, static_cast<const FixOp*>(s->fix_ops_dev.ptr) + fix_first[pi],
+                                  fix_count[pi], static_cast<const float2*>(s->phase_tab_fix_dev.ptr), (float)out, st));
+      } else if (s->precision == DMV_C64) DMV_TRY(launch_window_tma<PolF32>(a, s->n, ps, ops_dev, phase_ops_dev, st));
       else if (fix_first[pi] >= 0) {
         const FixOp* f = static_cast<const FixOp*>(s->fix_ops_dev.ptr) + fix_first[pi];
         const longlong2* ft = static_cast<const longlong2*>(s->phase_tab_fix_dev.ptr);
