@@ -215,6 +215,14 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
     ph.a[7] = (int32_t)rpos;
     ph.a[8] = flip;
     flip = 0;
+    // at most one table, then rotations on register bits 0, 1, ... once each
+    {
+      const size_t t0 = taken[0].kind == FIX_TABLE ? 1 : 0;
+      bool simple = taken.size() - t0 <= (size_t)reg_bits;
+      for (size_t i = t0; i < taken.size(); ++i)
+        simple = simple && taken[i].kind == FIX_ROT && (taken[i].a[0] & 15) == reg[i - t0];
+      if (simple) ph.a[9] = kFixSimple | (t0 ? kFixSimpleTable : 0) | (int32_t)(taken.size() - t0);
+    }
     out.push_back(ph);
     for (FixOp& f : taken) {
       if (f.kind == FIX_ROT || f.kind == FIX_GRAD) {
@@ -242,6 +250,7 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
   pack_images(end, slots);
   end.a[8] = flip;
   out.push_back(end);
+  if (single) return true;
   // Each table's first entries load from the moment the one before it is done.
   std::vector<FixOp> body(out.begin() + (std::ptrdiff_t)mark, out.end());
   out.resize(mark);

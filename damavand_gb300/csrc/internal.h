@@ -367,7 +367,7 @@ void set_tc_convert_mode(int32_t mode);
 // ---------------------------------------------------------------------------
 enum FixKind : int32_t {
   FIX_PHASE = 0,  // registers out, registers in: a[0..5] the images (fix_slot(A e_b)) of the 4 register bits, then of
-                  // the 8 thread bits, two 16-bit words each; a[8]: c ^= a[8] first. Host only: a[6] the tile bits of the
+                  // the 8 thread bits, two 16-bit words each; a[8]: c ^= a[8] first; a[9]: kFixSimple. Host only: a[6] the tile bits of the
                   // 8 thread bits, a[7] of the 4 register bits, 4 bits each
   FIX_XOR = 1,    // slot offset c ^= a[1] on tiles where qubit a[0] is 1
   FIX_ROT = 2,    // OP_ROT on register bit a[0] & 3: a[0] also holds kFixComplement and kFixShift; a[1], a[2]: the
@@ -381,6 +381,10 @@ enum FixKind : int32_t {
 };
 constexpr int32_t kFixComplement = 4;  // the multiplier is 1 - w
 constexpr int32_t kFixShift = 8;       // then every amplitude is halved
+// FIX_PHASE's a[9] when its ops are at most one FIX_TABLE, then one FIX_ROT on
+// each of register bits 0, 1, ... (their number in the low bits).
+constexpr int32_t kFixSimple = 16;
+constexpr int32_t kFixSimpleTable = 8;  // with a table
 struct alignas(16) FixOp {
   int32_t kind;
   int32_t a[11];
