@@ -15,9 +15,11 @@
 // An autotuner picks the tile size, the number of always-local low qubits
 // and the tiles per item by timing graph runs of the batch itself.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
+#include "fix_ops.cuh"
 #include "internal.h"
 #include "policies.cuh"
 
@@ -33,7 +35,15 @@ struct BatchPass {
   int64_t amp_offset;  // first amplitude of the circuit in the arena
   int64_t op_begin;    // first op in the batch op array
   int32_t fmt;         // FP32-pair batches: bit 0 reads, bit 1 writes the pair form (not its
-  int32_t pad;         // circuit's first / last pass), so the passes between skip the conversions
+                       // circuit's first / last pass), so the passes between skip the conversions
+  // Rewritten FP64 passes (k_batch_fix):
+  int32_t fix_count;   // fixed-point ops, 0: FP64 only
+  int64_t fix_begin;
+  int32_t shifts;
+  uint32_t sparse;
+  int32_t out_exp;     // the circuit leaves the pass times out_frac 2^out_exp
+  int32_t pad;
+  double out_frac;
 };
 
 struct BatchItem {
@@ -126,6 +136,122 @@ k_batch(typename P::G* __restrict__ arena, const BatchPass* __restrict__ passes,
   }
 }
 
+// The queue of k_batch over rewritten FP64 passes (rotations, phase tables,
+// exchanges): tiles of 2^12 amplitudes that qualify run in the fixed-point
+// arithmetic of fix_ops.cuh, the others in FP64. Applied as complex 2x2s in
+// FP64, 8 multiply-adds per amplitude and gate, the batch was bound by them.
+constexpr size_t kBatchFixSmem = ((size_t)16 << 12) + kFixStage + (size_t)kFixSmemOps * sizeof(FixOp);
+
+__global__ void __launch_bounds__(kFixThreads, 2)
+k_batch_fix(double2* __restrict__ arena, const BatchPass* __restrict__ passes, const BatchItem* __restrict__ items,
+            int64_t num_items, const Op* __restrict__ ops, const double2* __restrict__ tab,
+            const FixOp* __restrict__ fix_ops, const longlong2* __restrict__ fix_tab, unsigned long long* counters,
+            long long spin_limit) {
+  constexpr int NT = kFixThreads;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ long long s_item;
+  __shared__ int s_stop;
+  __shared__ int64_t s_slot[kFixAmps];
+  __shared__ uint32_t s_scan[4][NT / 32];
+  __shared__ int s_top[3];
+  const int tid = (int)threadIdx.x;
+  longlong2* ti = reinterpret_cast<longlong2*>(smem_raw);
+  double2* td = reinterpret_cast<double2*>(smem_raw);
+  longlong2* stage = ti + (1 << 12) + tid;
+  FixOp* sops = reinterpret_cast<FixOp*>(ti + (1 << 12) + 8 * NT);
+  if (tid < 3) s_top[tid] = 0;
+  for (;;) {
+    if (tid == 0) {
+      const long long it = (long long)atomicAdd(&counters[0], 1ull);
+      int stop = it >= num_items ? 1 : 0;
+      if (!stop && items[it].wait_count > 0) {
+        const unsigned long long* done = counters + 2 + items[it].circuit;
+        const unsigned long long need = (unsigned long long)items[it].wait_count;
+        long long spins = 0;
+        while (ld_acquire_u64(done) < need) {
+          if (++spins > spin_limit || *(volatile unsigned long long*)&counters[1] != 0ull) {
+            stop = 2;
+            break;
+          }
+          __nanosleep(1000);
+        }
+      }
+      if (stop == 2) atomicExch(&counters[1], 1ull);
+      s_item = it;
+      s_stop = stop;
+    }
+    __syncthreads();
+    if (s_stop) break;
+    const BatchItem item = items[s_item];
+    const BatchPass& ps = passes[item.pass];
+    double2* a = arena + ps.amp_offset;
+    const int k = ps.k, low = ps.low, nh = ps.nh, T = 1 << k;
+    const int num_fix = ps.fix_count;
+    int64_t t_off = 0;
+    for (int i = 0; i < min(k, kFixThreadBits); ++i)
+      t_off |= (int64_t)((tid >> i) & 1) << (i < low ? i : ps.high[i - low]);
+    if (tid < kFixAmps) {
+      int64_t off = 0;
+      for (int i = kFixThreadBits; i < k; ++i)
+        off |= (int64_t)((tid >> (i - kFixThreadBits)) & 1) << (i < low ? i : ps.high[i - low]);
+      s_slot[tid] = off;
+    }
+    const FixOp* fops = fix_ops + ps.fix_begin;
+    if (num_fix <= kFixSmemOps) {
+      int4* dst = reinterpret_cast<int4*>(sops);
+      const int4* src = reinterpret_cast<const int4*>(fops);
+      for (int i = tid; i < num_fix * 3; i += NT) dst[i] = src[i];
+      fops = sops;
+    }
+    __syncthreads();
+    for (int64_t tix = item.tile_begin; tix < item.tile_end; ++tix) {
+      int64_t base = tix << low;
+      for (int i = 0; i < nh; ++i) base = insert_zero(base, ps.high[i]);
+      double2* at = a + (base | t_off);
+      long long r[2 * kFixAmps];
+      // L2-coherent loads: another SM wrote these amplitudes in the previous pass.
+#pragma unroll
+      for (int u = 0; u < kFixAmps; ++u) {
+        longlong2 v = make_longlong2(0, 0);
+        if (tid + NT * u < T) v = __ldcg(reinterpret_cast<const longlong2*>(at + s_slot[u]));
+        r[2 * u] = v.x;
+        r[2 * u + 1] = v.y;
+      }
+      const FixScan scan = fix_scan(r, s_scan);
+      if (num_fix > 0 && scan.fixed(ps.sparse)) {
+        fix_put(r, smem_raw, scan.emax());
+        const int renorm = fix_run(r, smem_raw, stage, fops, num_fix, fix_tab, base, s_top);
+        const int e = scan.emax() - 1079 + ps.shifts + renorm + 1075 + ps.out_exp;
+        const double f = ps.out_frac;
+#pragma unroll
+        for (int u = 0; u < kFixAmps; ++u) {
+          double2 v = make_double2(fix_to_double(r[2 * u], e), fix_to_double(r[2 * u + 1], e));
+          if (f != 1.0) v = make_double2(v.x * f, v.y * f);
+          at[s_slot[u]] = v;
+        }
+      } else if (!scan.zero()) {
+#pragma unroll
+        for (int u = 0; u < kFixAmps; ++u)
+          if (tid + NT * u < T) ti[tid + NT * u] = make_longlong2(r[2 * u], r[2 * u + 1]);
+        __syncthreads();
+        tile_apply_ops<PolF64>(td, T, ops + ps.op_begin, ps.num_ops, base, tab);
+        const double f = scalbn(ps.out_frac, ps.out_exp);
+#pragma unroll
+        for (int u = 0; u < kFixAmps; ++u)
+          if (tid + NT * u < T) {
+            const double2 v = td[tid + NT * u];
+            at[s_slot[u]] = make_double2(v.x * f, v.y * f);
+          }
+      }
+      __syncthreads();
+      if (tid < 3) s_top[tid] = 0;
+    }
+    __threadfence();  // publish this item's amplitudes before counting it done
+    __syncthreads();
+    if (tid == 0) atomicAdd(&counters[2 + item.circuit], 1ull);
+  }
+}
+
 template <typename G>
 __global__ void k_batch_init(G* arena, const int64_t* offsets, int count) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -161,6 +287,8 @@ struct dmv_batch_s {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   bool use_graph = true;
+  bool rewrite = false;     // passes as rotations, tables and exchanges (k_batch_fix)
+  DeviceBuffer fix_ops_dev, tab_dev, fix_tab_dev, tab_src_dev;
   bool all_unitary = true;  // block fixed point needs unitary ops everywhere
   long long spin_limit = kDefaultSpinLimit;
   bool poison_next_plan = false;  // test hook: one item waits for a count that never arrives
@@ -184,6 +312,8 @@ void destroy_graph(dmv_batch_s* b) {
 int batch_plan(dmv_batch_s* b) {
   std::vector<BatchPass> passes;
   std::vector<Op> ops;
+  std::vector<FixOp> fix_ops;
+  PhaseTables tabs;
   std::vector<std::vector<int32_t>> pass_ids((size_t)b->count);
   std::vector<std::vector<int64_t>> pass_tiles((size_t)b->count);
   b->max_k = 0;
@@ -192,6 +322,7 @@ int batch_plan(dmv_batch_s* b) {
     PlanOptions opt = b->opt;
     opt.windows_only = true;
     DMV_TRY(build_plan(b->gates[(size_t)c], b->n[(size_t)c], b->precision, opt, plan));
+    double stored = 1.0;  // the circuit's stored amplitudes / the true ones
     for (const Pass& p : plan.passes) {
       BatchPass bp;
       std::memset(&bp, 0, sizeof(bp));
@@ -202,7 +333,38 @@ int batch_plan(dmv_batch_s* b) {
       for (int i = 0; i < p.num_high; ++i) bp.high[i] = p.high[i];
       bp.amp_offset = b->offsets[(size_t)c];
       bp.op_begin = (int64_t)ops.size();
-      for (int64_t o = 0; o < p.op_count; ++o) ops.push_back(plan.ops[(size_t)(p.op_begin + o)]);
+      bp.out_frac = 1.0;
+      if (b->rewrite) {
+        RewrittenPass r;
+        rewrite_pass_rotations(plan.ops.data() + p.op_begin, p.op_count, bp.k, true, r.ops, r.tab, &r.scale);
+        bp.fix_begin = (int64_t)fix_ops.size();
+        if (bp.k == 12 && build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), 12, fix_ops, &bp.shifts, &bp.sparse))
+          bp.fix_count = (int32_t)((int64_t)fix_ops.size() - bp.fix_begin);
+        if (tabs.entries + r.tab.entries > INT32_MAX) {
+          b->rewrite = false;
+          return batch_plan(b);
+        }
+        for (Op& op : r.ops)
+          if (op.cls == OP_PHASE) op.fh[0] += (int32_t)tabs.entries;
+        for (int64_t i = bp.fix_begin; i < (int64_t)fix_ops.size(); ++i)
+          if (fix_ops[(size_t)i].kind == FIX_TABLE || fix_ops[(size_t)i].kind == FIX_FETCH)
+            fix_ops[(size_t)i].a[0] += (int32_t)tabs.entries;
+        for (PhaseTable t : r.tab.tables) {
+          t.entry += tabs.entries;
+          t.first_term += (int32_t)tabs.terms.size();
+          tabs.tables.push_back(t);
+        }
+        tabs.terms.insert(tabs.terms.end(), r.tab.terms.begin(), r.tab.terms.end());
+        tabs.entries += r.tab.entries;
+        const double raw = stored / r.scale.hi;
+        if (&p == &plan.passes.back()) bp.out_frac = 1.0 / raw;
+        else bp.out_exp = -std::ilogb(raw);
+        stored = std::ldexp(raw, bp.out_exp);
+        bp.num_ops = (int32_t)r.ops.size();
+        ops.insert(ops.end(), r.ops.begin(), r.ops.end());
+      } else {
+        for (int64_t o = 0; o < p.op_count; ++o) ops.push_back(plan.ops[(size_t)(p.op_begin + o)]);
+      }
       b->max_k = std::max(b->max_k, bp.k);
       if (b->precision == DMV_C128 && b->arith == ARITH_FP32X2) {
         const size_t pi = (size_t)(&p - plan.passes.data());
@@ -255,6 +417,29 @@ int batch_plan(dmv_batch_s* b) {
   DMV_TRY(b->passes_dev.reserve(std::max<size_t>(1, passes.size()) * sizeof(BatchPass)));
   DMV_TRY(b->items_dev.reserve(std::max<size_t>(1, items.size()) * sizeof(BatchItem)));
   DMV_TRY(b->ops_dev.reserve(std::max<size_t>(1, ops.size()) * sizeof(Op)));
+  if (b->rewrite) {
+    const size_t bytes = (size_t)std::max<int64_t>(1, tabs.entries) * 16;
+    if (b->fix_ops_dev.reserve(std::max<size_t>(1, fix_ops.size()) * sizeof(FixOp)) != DMV_OK ||
+        b->tab_dev.reserve(bytes) != DMV_OK || b->fix_tab_dev.reserve(bytes) != DMV_OK) {
+      // no room for the tables: complex 2x2s
+      clear_error();
+      b->tab_dev.release();
+      b->fix_tab_dev.release();
+      b->rewrite = false;
+      return batch_plan(b);
+    }
+    if (!fix_ops.empty())
+      DMV_CUDA_TRY(cudaMemcpy(b->fix_ops_dev.ptr, fix_ops.data(), fix_ops.size() * sizeof(FixOp), cudaMemcpyHostToDevice));
+    if (tabs.entries > 0) {
+      PhaseTableForms forms;
+      forms.f64 = static_cast<double2*>(b->tab_dev.ptr);
+      forms.fix = static_cast<longlong2*>(b->fix_tab_dev.ptr);
+      std::vector<unsigned char> src;
+      DMV_TRY(make_phase_tables(tabs, fix_ops, forms, src, b->tab_src_dev, b->stream));
+      DMV_CUDA_TRY(cudaStreamSynchronize(b->stream));
+      b->tab_src_dev.release();
+    }
+  }
   if (!passes.empty())
     DMV_CUDA_TRY(cudaMemcpy(b->passes_dev.ptr, passes.data(), passes.size() * sizeof(BatchPass), cudaMemcpyHostToDevice));
   if (!items.empty())
@@ -295,6 +480,36 @@ int batch_launch_kernel(dmv_batch_s* b) {
   return DMV_OK;
 }
 
+int batch_launch_fix(dmv_batch_s* b) {
+  DMV_CUDA_TRY(cudaFuncSetAttribute(k_batch_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchFixSmem));
+  int per_sm = 0;
+  DMV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_fix, kFixThreads, kBatchFixSmem));
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (per_sm < 1) return set_error(DMV_ERR_CUDA, "batch kernel does not fit (%zu bytes of shared memory)", kBatchFixSmem);
+  b->grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * sms, b->num_items));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)b->grid);
+  cfg.blockDim = dim3(kFixThreads);
+  cfg.dynamicSmemBytes = kBatchFixSmem;
+  cfg.stream = b->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  DMV_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_batch_fix, static_cast<double2*>(b->arena),
+                                  static_cast<const BatchPass*>(b->passes_dev.ptr),
+                                  static_cast<const BatchItem*>(b->items_dev.ptr), b->num_items,
+                                  static_cast<const Op*>(b->ops_dev.ptr), static_cast<const double2*>(b->tab_dev.ptr),
+                                  static_cast<const FixOp*>(b->fix_ops_dev.ptr),
+                                  static_cast<const longlong2*>(b->fix_tab_dev.ptr),
+                                  static_cast<unsigned long long*>(b->counters_dev.ptr), b->spin_limit));
+  count_launch();
+  return DMV_OK;
+}
+
 // The whole run as stream work: counters and arena reset, |0...0> per
 // circuit, the persistent kernel, then the per-circuit Pauli-Z reductions.
 int batch_enqueue(dmv_batch_s* b) {
@@ -313,6 +528,7 @@ int batch_enqueue(dmv_batch_s* b) {
     if (b->precision == DMV_C64) DMV_TRY(batch_launch_kernel<PolF32>(b));
     else if (b->arith == ARITH_FP32X2) DMV_TRY(batch_launch_kernel<PolDF>(b));
     else if (b->arith == ARITH_INT64 && b->all_unitary) DMV_TRY(batch_launch_kernel<PolFX>(b));
+    else if (b->rewrite) DMV_TRY(batch_launch_fix(b));
     else DMV_TRY(batch_launch_kernel<PolF64>(b));
   }
   double* red = static_cast<double*>(b->reduce_dev.ptr);
@@ -388,9 +604,13 @@ extern "C" int dmv_batch_create(int32_t num_circuits, const int32_t* num_qubits,
   dmv_batch_s* b = new dmv_batch_s();
   b->count = num_circuits;
   b->precision = precision;
-  // Batches apply every fused 2x2 directly: the rotation/phase-table rewrite of
-  // single states builds one table per pass, which many small circuits cannot
-  // amortise (config-4-like batches: ~22k tables, 2.9 GB, for 512 circuits).
+  // The default arithmetic takes the single states' rewrite and its tables (made
+  // once, on the device); the others apply every fused 2x2 directly.
+  b->rewrite = precision == DMV_C128 && arithmetic == DMV_ARITH_FP64;
+  if (b->rewrite) {
+    b->opt.low_bits = 4;
+    b->opt.search_windows = true;
+  }
   b->arith = arithmetic == DMV_ARITH_FP64_DIRECT ? (int32_t)ARITH_FP64 : arithmetic;
   int64_t off = 0;
   for (int32_t c = 0; c < num_circuits; ++c) {
@@ -465,6 +685,10 @@ extern "C" int dmv_batch_destroy(dmv_batch_t b) {
   b->counters_dev.release();
   b->offsets_dev.release();
   b->reduce_dev.release();
+  b->fix_ops_dev.release();
+  b->tab_dev.release();
+  b->fix_tab_dev.release();
+  b->tab_src_dev.release();
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->stream) cudaStreamDestroy(b->stream);

@@ -185,4 +185,168 @@ __device__ __forceinline__ uint32_t fix_reg(uint32_t base, const uint32_t (&pr)[
   return s;
 }
 
+// ---------------------------------------------------------------------------
+// A tile of 2^12 amplitudes by 256 threads (fix_window.cuh, batch.cu).
+// ---------------------------------------------------------------------------
+constexpr int kFixThreads = 256;
+constexpr int kFixThreadBits = 8;
+constexpr int kFixAmps = 16;  // per thread
+constexpr size_t kFixStage = (size_t)8 * kFixThreads * 16;  // table entries on their way
+
+// What decides how a tile runs.
+struct FixScan {
+  uint32_t mx, mn, any, cnt;  // largest and smallest nonzero amplitude (top words), low words, nonzero amplitudes
+  __device__ int emax() const { return (int)(mx >> 20); }
+  __device__ bool zero() const { return mx == 0 && any == 0; }
+  // In range, with no more than the pass's (`sparse`) numbers of unreached
+  // qubits: log2 (4096 / nonzero amplitudes).
+  __device__ bool fixed(uint32_t sparse) const {
+    const int unreached = 12 - (31 - __clz((int)cnt | 1));
+    return emax() - (int)(mn >> 20) <= kFixRange && emax() > 200 && emax() < 1800 && ((sparse >> unreached) & 1u);
+  }
+};
+
+// Over the CTA, of amplitudes raw (double bits); s: 4 x 8 words of shared memory.
+__device__ __forceinline__ FixScan fix_scan(const long long (&raw)[2 * kFixAmps], uint32_t (*s)[kFixThreads / 32]) {
+  uint32_t mx = 0, mn = ~0u, any = 0, cnt = 0;
+#pragma unroll
+  for (int u = 0; u < kFixAmps; ++u) {
+    const uint32_t h = max((uint32_t)(raw[2 * u] >> 32) & 0x7FFFFFFFu, (uint32_t)(raw[2 * u + 1] >> 32) & 0x7FFFFFFFu);
+    const uint32_t lo = (uint32_t)raw[2 * u] | (uint32_t)raw[2 * u + 1];
+    mx = max(mx, h);
+    any |= lo;
+    if (h | lo) {
+      mn = min(mn, h);
+      ++cnt;
+    }
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  any = __reduce_or_sync(0xffffffffu, any);
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if ((threadIdx.x & 31) == 0) {
+    const int w = (int)threadIdx.x >> 5;
+    s[0][w] = mx;
+    s[1][w] = mn;
+    s[2][w] = any;
+    s[3][w] = cnt;
+  }
+  __syncthreads();
+  cnt = 0;
+#pragma unroll
+  for (int w = 0; w < kFixThreads / 32; ++w) {
+    mx = max(mx, s[0][w]);
+    mn = min(mn, s[1][w]);
+    any |= s[2][w];
+    cnt += s[3][w];
+  }
+  return FixScan{mx, mn, any, cnt};
+}
+
+// The tile's amplitudes (thread tid holds tid + 256 u) into its slots as integers.
+__device__ __forceinline__ void fix_put(const long long (&raw)[2 * kFixAmps], unsigned char* tile, int emax) {
+  longlong2* ti = reinterpret_cast<longlong2*>(tile);
+#pragma unroll
+  for (int u = 0; u < kFixAmps; ++u)
+    ti[fix_slot(threadIdx.x + kFixThreads * u)] = make_longlong2(fix_from_double(__longlong_as_double(raw[2 * u]), emax),
+                                                                 fix_from_double(__longlong_as_double(raw[2 * u + 1]), emax));
+}
+
+// Every op of a pass on the tile in its slots; leaves amplitude tid + 256 u in
+// r[2u], r[2u + 1] and returns the halvings beyond the planned ones. `stage`:
+// this thread's place in kFixStage bytes; s_top: three words, zero.
+__device__ __forceinline__ int fix_run(long long (&r)[2 * kFixAmps], unsigned char* tile, longlong2* stage,
+                                       const FixOp* ops, int num_ops, const longlong2* tab, int64_t base, int* s_top) {
+  const int tid = (int)threadIdx.x, lane = tid & 31;
+        uint32_t pr[4] = {0, 0, 0, 0};
+        uint32_t pbase = 0, cx = 0;
+        int phase = -1;  // of the registers
+        int renorm = 0;  // further halvings so far
+        const longlong2* ahead = nullptr;  // the entries of the table being fetched
+        int4 nxt = *reinterpret_cast<const int4*>(ops);
+        for (int o = 0; o < num_ops; ++o) {
+          const FixOp* op = ops + o;
+          const int4 w0 = nxt;
+          if (o + 1 < num_ops) nxt = *reinterpret_cast<const int4*>(op + 1);
+          if (w0.x == FIX_ROT) {
+            switch (w0.y & 3) {
+              case 0: fix_rot_form<kFixAmps, 0>(r, w0.y, w0.z, w0.w); break;
+              case 1: fix_rot_form<kFixAmps, 1>(r, w0.y, w0.z, w0.w); break;
+              case 2: fix_rot_form<kFixAmps, 2>(r, w0.y, w0.z, w0.w); break;
+              default: fix_rot_form<kFixAmps, 3>(r, w0.y, w0.z, w0.w); break;
+            }
+            if (w0.y & kFixShift) {
+  #pragma unroll
+              for (int j = 0; j < 2 * kFixAmps; ++j) r[j] >>= 1;
+            }
+          } else if (w0.x == FIX_TABLE) {
+            // groups of four entries: wait for this one, then start the one after the next
+  #pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              if (g < 3) fix_copy_wait<1>();
+              else fix_copy_wait<0>();
+              longlong2 t[4];
+  #pragma unroll
+              for (int j = 0; j < 4; ++j) t[j] = stage[kFixThreads * (4 * (g & 1) + j)];
+  #pragma unroll
+              for (int j = 0; j < 4; ++j) fix_phase(r[2 * (4 * g + j)], r[2 * (4 * g + j) + 1], t[j]);
+              if (g < 2) {
+  #pragma unroll
+                for (int j = 0; j < 4; ++j) fix_copy16(stage + kFixThreads * (4 * g + j), ahead + kFixThreads * (4 * g + 8 + j));
+                fix_copy_commit();
+              }
+            }
+          } else if (w0.x == FIX_FETCH) {
+            ahead = tab + fix_slice(op, base, 12) + tid;
+  #pragma unroll
+            for (int g = 0; g < 2; ++g) {
+  #pragma unroll
+              for (int j = 0; j < 4; ++j) fix_copy16(stage + kFixThreads * (4 * g + j), ahead + kFixThreads * (4 * g + j));
+              fix_copy_commit();
+            }
+          } else if (w0.x == FIX_XOR) {
+            if ((base >> w0.y) & 1) cx ^= (uint32_t)w0.z;
+          } else {  // FIX_PHASE, FIX_END
+            const int4 w1 = *(reinterpret_cast<const int4*>(op) + 1);
+            if (phase >= 0) {
+  #pragma unroll
+              for (int j = 0; j < kFixAmps; ++j) *reinterpret_cast<longlong2*>(tile + fix_reg(pbase, pr, j)) = make_longlong2(r[2 * j], r[2 * j + 1]);
+              const int top = __reduce_max_sync(0xffffffffu, fix_top(r));
+              if (lane == 0) atomicMax(&s_top[phase % 3], top);
+              // the next phase's word: last read before the barrier before this one
+              if (tid == 0) s_top[(phase + 1) % 3] = 0;
+            }
+            __syncthreads();
+            const uint32_t img[6] = {(uint32_t)w0.y, (uint32_t)w0.z, (uint32_t)w0.w,
+                                     (uint32_t)w1.x, (uint32_t)w1.y, (uint32_t)w1.z};
+            // as byte offsets
+            pr[0] = (img[0] & 0xFFFFu) << 4;
+            pr[1] = img[0] >> 16 << 4;
+            pr[2] = (img[1] & 0xFFFFu) << 4;
+            pr[3] = img[1] >> 16 << 4;
+            cx ^= (uint32_t)op->a[8];
+            pbase = cx;
+  #pragma unroll
+            for (int b = 0; b < 8; ++b) {
+              const uint32_t im = (b & 1) ? img[2 + b / 2] >> 16 : img[2 + b / 2] & 0xFFFFu;
+              if ((tid >> b) & 1) pbase ^= im;
+            }
+            pbase <<= 4;
+  #pragma unroll
+            for (int j = 0; j < kFixAmps; ++j) {
+              const longlong2 v = *reinterpret_cast<const longlong2*>(tile + fix_reg(pbase, pr, j));
+              r[2 * j] = v.x;
+              r[2 * j + 1] = v.y;
+            }
+            if (phase >= 0) {
+              const int sh = fix_renorm(s_top[phase % 3]);
+              fix_shift(r, sh);
+              renorm += sh;
+            }
+            ++phase;
+          }
+        }
+  return renorm;
+}
+
 }  // namespace dmv

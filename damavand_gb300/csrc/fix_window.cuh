@@ -28,10 +28,6 @@
 // stored norm grows at most 2 sqrt 2 times (kFixShift halves it), so no sum
 // leaves 63 bits.
 
-constexpr int kFixThreads = 256;
-constexpr int kFixThreadBits = 8;
-constexpr int kFixAmps = 16;       // amplitudes per thread: (2^12 tile) / 256
-
 struct FixPassParams {
   TmaPassParams t;
   const FixOp* fix_ops;
@@ -47,7 +43,7 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
   constexpr int NT = kFixThreads;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_mx[NT / 32], s_mn[NT / 32], s_any[NT / 32], s_cnt[NT / 32];
+  __shared__ uint32_t s_scan[4][NT / 32];
   __shared__ int s_high[16];
   __shared__ int64_t s_slot[kFixAmps];
   __shared__ int s_top[3];  // largest component, by phase
@@ -107,143 +103,20 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
     const int64_t base = geom.base(tix);
     const int64_t next = tix + gridDim.x;
     long long r[2 * kFixAmps];
-    // largest and smallest amplitude (top words of their larger component)
-    uint32_t mx = 0, mn = ~0u, any = 0, cnt = 0;
 #pragma unroll
     for (int u = 0; u < kFixAmps; ++u) {
       const longlong2 v = ti[tid + NT * u];
       r[2 * u] = v.x;
       r[2 * u + 1] = v.y;
-      const uint32_t h = max((uint32_t)(v.x >> 32) & 0x7FFFFFFFu, (uint32_t)(v.y >> 32) & 0x7FFFFFFFu);
-      const uint32_t lo = (uint32_t)v.x | (uint32_t)v.y;
-      mx = max(mx, h);
-      any |= lo;
-      if (h | lo) {
-        mn = min(mn, h);
-        ++cnt;
-      }
     }
-    cnt = __reduce_add_sync(0xffffffffu, cnt);
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    mn = __reduce_min_sync(0xffffffffu, mn);
-    any = __reduce_or_sync(0xffffffffu, any);
-    if (lane == 0) {
-      s_mx[tid >> 5] = mx;
-      s_mn[tid >> 5] = mn;
-      s_any[tid >> 5] = any;
-      s_cnt[tid >> 5] = cnt;
-    }
-    __syncthreads();
-    cnt = 0;
-#pragma unroll
-    for (int w = 0; w < NT / 32; ++w) {
-      mx = max(mx, s_mx[w]);
-      mn = min(mn, s_mn[w]);
-      any |= s_any[w];
-      cnt += s_cnt[w];
-    }
-    const int emax = (int)(mx >> 20);
-    const bool zero = mx == 0 && any == 0;
-    // qubits of the tile that the state has not reached: log2 (4096 / nonzero amplitudes)
-    const int unreached = k - (31 - __clz((int)cnt | 1));
-    const bool fixed = emax - (int)(mn >> 20) <= kFixRange && emax > 200 && emax < 1800 &&
-                       ((fp.sparse >> unreached) & 1u);
+    const FixScan scan = fix_scan(r, s_scan);
+    const int emax = scan.emax();
+    const bool zero = scan.zero(), fixed = scan.fixed(fp.sparse);
     int e_out = 0;
     const bool store = !zero;
     if (fixed) {
-#pragma unroll
-      for (int u = 0; u < kFixAmps; ++u)
-        ti[fix_slot((uint32_t)(tid + NT * u))] =
-            make_longlong2(fix_from_double(__longlong_as_double(r[2 * u]), emax),
-                           fix_from_double(__longlong_as_double(r[2 * u + 1]), emax));
-      uint32_t pr[4] = {0, 0, 0, 0};
-      uint32_t pbase = 0, cx = 0;
-      int phase = -1;  // of the registers
-      int renorm = 0;  // further halvings so far
-      const longlong2* ahead = nullptr;  // the entries of the table being fetched
-      int4 nxt = *reinterpret_cast<const int4*>(ops);
-      for (int o = 0; o < fp.num_fix_ops; ++o) {
-        const FixOp* op = ops + o;
-        const int4 w0 = nxt;
-        if (o + 1 < fp.num_fix_ops) nxt = *reinterpret_cast<const int4*>(op + 1);
-        if (w0.x == FIX_ROT) {
-          switch (w0.y & 3) {
-            case 0: fix_rot_form<kFixAmps, 0>(r, w0.y, w0.z, w0.w); break;
-            case 1: fix_rot_form<kFixAmps, 1>(r, w0.y, w0.z, w0.w); break;
-            case 2: fix_rot_form<kFixAmps, 2>(r, w0.y, w0.z, w0.w); break;
-            default: fix_rot_form<kFixAmps, 3>(r, w0.y, w0.z, w0.w); break;
-          }
-          if (w0.y & kFixShift) {
-#pragma unroll
-            for (int j = 0; j < 2 * kFixAmps; ++j) r[j] >>= 1;
-          }
-        } else if (w0.x == FIX_TABLE) {
-          // groups of four entries: wait for this one, then start the one after the next
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            if (g < 3) fix_copy_wait<1>();
-            else fix_copy_wait<0>();
-            longlong2 t[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) t[j] = stage[NT * (4 * (g & 1) + j)];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) fix_phase(r[2 * (4 * g + j)], r[2 * (4 * g + j) + 1], t[j]);
-            if (g < 2) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) fix_copy16(stage + NT * (4 * g + j), ahead + NT * (4 * g + 8 + j));
-              fix_copy_commit();
-            }
-          }
-        } else if (w0.x == FIX_FETCH) {
-          ahead = fp.fix_tab + fix_slice(op, base, k) + tid;
-#pragma unroll
-          for (int g = 0; g < 2; ++g) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) fix_copy16(stage + NT * (4 * g + j), ahead + NT * (4 * g + j));
-            fix_copy_commit();
-          }
-        } else if (w0.x == FIX_XOR) {
-          if ((base >> w0.y) & 1) cx ^= (uint32_t)w0.z;
-        } else {  // FIX_PHASE, FIX_END
-          const int4 w1 = *(reinterpret_cast<const int4*>(op) + 1);
-          if (phase >= 0) {
-#pragma unroll
-            for (int j = 0; j < kFixAmps; ++j) *reinterpret_cast<longlong2*>(tile + fix_reg(pbase, pr, j)) = make_longlong2(r[2 * j], r[2 * j + 1]);
-            const int top = __reduce_max_sync(0xffffffffu, fix_top(r));
-            if (lane == 0) atomicMax(&s_top[phase % 3], top);
-            // the next phase's word: last read before the barrier before this one
-            if (tid == 0) s_top[(phase + 1) % 3] = 0;
-          }
-          __syncthreads();
-          const uint32_t img[6] = {(uint32_t)w0.y, (uint32_t)w0.z, (uint32_t)w0.w,
-                                   (uint32_t)w1.x, (uint32_t)w1.y, (uint32_t)w1.z};
-          // as byte offsets
-          pr[0] = (img[0] & 0xFFFFu) << 4;
-          pr[1] = img[0] >> 16 << 4;
-          pr[2] = (img[1] & 0xFFFFu) << 4;
-          pr[3] = img[1] >> 16 << 4;
-          cx ^= (uint32_t)op->a[8];
-          pbase = cx;
-#pragma unroll
-          for (int b = 0; b < 8; ++b) {
-            const uint32_t im = (b & 1) ? img[2 + b / 2] >> 16 : img[2 + b / 2] & 0xFFFFu;
-            if ((tid >> b) & 1) pbase ^= im;
-          }
-          pbase <<= 4;
-#pragma unroll
-          for (int j = 0; j < kFixAmps; ++j) {
-            const longlong2 v = *reinterpret_cast<const longlong2*>(tile + fix_reg(pbase, pr, j));
-            r[2 * j] = v.x;
-            r[2 * j + 1] = v.y;
-          }
-          if (phase >= 0) {
-            const int sh = fix_renorm(s_top[phase % 3]);
-            fix_shift(r, sh);
-            renorm += sh;
-          }
-          ++phase;
-        }
-      }
+      fix_put(r, tile, emax);
+      const int renorm = fix_run(r, tile, stage, ops, fp.num_fix_ops, fp.fix_tab, base, s_top);
       e_out = emax - 1079 + fp.shifts + renorm + 1075;
     } else if (!zero) {
       using V = typename FB::T;

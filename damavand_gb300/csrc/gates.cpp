@@ -175,6 +175,13 @@ struct PGate {
   int32_t param, generator;  // adjoint tags (PlanOptions::param_of), else -1 / 0
 };
 
+// What the window search reads of a gate.
+struct SGate {
+  uint64_t qs, target;  // its qubits
+  int16_t t, c;
+  bool exchange;
+};
+
 Op make_op(const PGate& g, int32_t target_pos, int32_t ctrl, int32_t ctrl_kind) {
   Op op;
   std::memset(&op, 0, sizeof(op));
@@ -193,15 +200,13 @@ inline uint64_t qbit(int32_t q) { return q >= 0 ? (uint64_t(1) << q) : 0; }
 
 // Depth of a gate in its window: the number of non-exchange gates on the
 // longest chain of taken gates that ends with it. `depth` holds it per qubit.
-inline bool is_exchange(const PGate& g) { return g.m[2] == 1. && g.m[4] == 1. && classify(g.m) == OP_SWAP; }
-inline int32_t gate_depth(const PGate& g, const int32_t* depth) {
-  const int32_t d = g.control >= 0 ? std::max(depth[g.target], depth[g.control]) : depth[g.target];
-  return is_exchange(g) ? d : d + 1;
+inline int32_t gate_depth(const SGate& g, const int32_t* depth) {
+  const int32_t d = g.c >= 0 ? std::max(depth[g.t], depth[g.c]) : depth[g.t];
+  return g.exchange ? d : d + 1;
 }
-inline void raise_depth(const PGate& g, int32_t* depth) {
-  const int32_t d = gate_depth(g, depth);
-  depth[g.target] = d;
-  if (g.control >= 0) depth[g.control] = d;
+inline void set_depth(const SGate& g, int32_t d, int32_t* depth) {
+  depth[g.t] = d;
+  if (g.c >= 0) depth[g.c] = d;
 }
 
 struct Window {
@@ -227,7 +232,7 @@ struct Window {
 // in complex64 67 and 62 ms. The search takes 2 ms of host time there.
 constexpr double kPassCost = 8.0;
 
-Window next_window(const std::vector<PGate>& fg, const std::vector<int64_t>& pending, int32_t n, int32_t k,
+Window next_window(const std::vector<SGate>& sg, const std::vector<int64_t>& pending, int32_t n, int32_t k,
                    int32_t low, bool search) {
   Window first;
   first.local = (uint64_t(1) << low) - 1;
@@ -235,8 +240,8 @@ Window next_window(const std::vector<PGate>& fg, const std::vector<int64_t>& pen
   int32_t nlocal = low;
   for (int64_t gi : pending) {
     if (nlocal >= k) break;
-    const int32_t t = fg[(size_t)gi].target;
-    if (!(first.local & qbit(t))) { first.local |= qbit(t); ++nlocal; }
+    const uint64_t t = sg[(size_t)gi].target;
+    if (!(first.local & t)) { first.local |= t; ++nlocal; }
   }
   for (int32_t q = 0; q < n && nlocal < k; ++q)
     if (!(first.local & qbit(q))) { first.local |= qbit(q); ++nlocal; }
@@ -255,19 +260,18 @@ Window next_window(const std::vector<PGate>& fg, const std::vector<int64_t>& pen
     int32_t depth[64] = {};
     for (int64_t gi : pending) {
       if (!(local & ~blocked)) break;  // every local qubit blocked
-      const PGate& g = fg[(size_t)gi];
-      const uint64_t qs = qbit(g.target) | qbit(g.control);
-      if ((qs & blocked) || !(local & qbit(g.target))) {
-        blocked |= qs;
+      const SGate& g = sg[(size_t)gi];
+      if ((g.qs & blocked) || !(local & g.target)) {
+        blocked |= g.qs;
         continue;
       }
       const int32_t d = gate_depth(g, depth);
-      raise_depth(g, depth);
+      set_depth(g, d, depth);
       if ((size_t)d >= work.size()) {
         work.resize((size_t)d + 1, 0);
         moves.resize((size_t)d + 1, 0);
       }
-      if (is_exchange(g)) ++moves[(size_t)d];
+      if (g.exchange) ++moves[(size_t)d];
       else ++work[(size_t)d];
     }
     double w = 0.0, x = 0.0;
@@ -358,9 +362,14 @@ int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
   //    pending; a gate left pending blocks its qubits.
   std::vector<int64_t> pending(fg.size());
   for (size_t i = 0; i < fg.size(); ++i) pending[i] = (int64_t)i;
+  std::vector<SGate> sg;
+  sg.reserve(fg.size());
+  for (const PGate& g : fg)
+    sg.push_back(SGate{qbit(g.target) | qbit(g.control), qbit(g.target), (int16_t)g.target, (int16_t)g.control,
+                       classify(g.m) == OP_SWAP});
   std::vector<int64_t> keep, take;
   while (!pending.empty()) {
-    const Window win = next_window(fg, pending, n, k, low, opt.search_windows);
+    const Window win = next_window(sg, pending, n, k, low, opt.search_windows);
     const uint64_t local = win.local;
 
     keep.clear();
@@ -369,14 +378,15 @@ int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
     int32_t depth[64] = {};
     for (size_t idx = 0; idx < pending.size(); ++idx) {
       const int64_t gi = pending[idx];
-      const PGate& g = fg[(size_t)gi];
-      const uint64_t qs = qbit(g.target) | qbit(g.control);
+      const SGate& g = sg[(size_t)gi];
+      const uint64_t qs = g.qs;
       if (blocked == all_mask) { keep.insert(keep.end(), pending.begin() + (int64_t)idx, pending.end()); break; }
-      if ((qs & blocked) || !(local & qbit(g.target)) || gate_depth(g, depth) > win.max_depth) {
+      const int32_t d = gate_depth(g, depth);
+      if ((qs & blocked) || !(local & g.target) || d > win.max_depth) {
         blocked |= qs;
         keep.push_back(gi);
       } else {
-        raise_depth(g, depth);
+        set_depth(g, d, depth);
         take.push_back(gi);
       }
     }

@@ -677,7 +677,7 @@ int launch_window_fix(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, 
   p.num_fix_ops = num_fix_ops;
   p.shifts = shifts;
   p.sparse = sparse;
-  const size_t smem = ((size_t)16 << 12) + 1024 + (size_t)8 * kFixThreads * 16 + kFixSmemOps * sizeof(FixOp);
+  const size_t smem = ((size_t)16 << 12) + 1024 + kFixStage + kFixSmemOps * sizeof(FixOp);
   static bool configured = false;
   if (!configured) {
     DMV_CUDA_TRY(cudaFuncSetAttribute(k_window_fix<FB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
