@@ -221,16 +221,18 @@ struct Window {
 // taken, in FP64 multiply-adds per amplitude: 2 per non-exchange gate (a
 // rotation), 3 per level of depth (each level of rotations has to apply the
 // diagonal factors left by the one before: one phase table), and kPassCost
-// for the pass itself (the state read and written once; about 2.5 in FP64 at
-// HBM's rate, far more where the arithmetic is faster). A deep window saves
-// passes and a shallow one phase tables, because a window's edge loses a
-// qubit per level: kPassCost 8 is near both optima. On the 28-qubit, 20-layer
-// ladder the search takes 78 passes (6 low qubits, first targets met: those
-// scatter the window over the qubits, where few gates meet) to 27 with 4 low
-// qubits. Measured forwards, before and after: 28 qubits in FP64 1041 and 879
-// ms, 26 in FP32 pairs 183 and 128 ms, 25 on the tensor cores 80 and 56 ms, 27
-// in complex64 67 and 62 ms. The search takes 2 ms of host time there.
-constexpr double kPassCost = 8.0;
+// for the pass itself. A deep window saves passes and a shallow one phase
+// tables, because a window's edge loses a qubit per level. Where the arithmetic
+// is fast (fixed point, FP32, tensor cores) a pass's reading, converting and
+// writing of the state costs as much as 15 rotations, so deep windows win: cost
+// 32 against 8 measured 9.3 and 9.8 ms at 24 qubits, 61 and 72 at 26 in FP32
+// pairs, 54 and 59 at 25 on the tensor cores, 32.6 and 35 at 27 in complex64
+// (28 in fixed point: 318 and 315). States of fewer tiles than SMs are bound
+// by a tile's latency: 8. On the 28-qubit, 20-layer ladder the search takes 78
+// passes (6 low qubits, first targets met: those scatter the window over the
+// qubits, where few gates meet) to 27 with 4 low qubits, in 1 ms of host time.
+constexpr double kPassCost = 32.0, kPassCostFewTiles = 8.0;
+constexpr int32_t kFewTilesQubits = 20;
 
 Window next_window(const std::vector<SGate>& sg, const std::vector<int64_t>& pending, int32_t n, int32_t k,
                    int32_t low, bool search) {
@@ -247,6 +249,7 @@ Window next_window(const std::vector<SGate>& sg, const std::vector<int64_t>& pen
     if (!(first.local & qbit(q))) { first.local |= qbit(q); ++nlocal; }
   if (!search || k >= n) return first;
 
+  const double pass_cost = n < kFewTilesQubits ? kPassCostFewTiles : kPassCost;
   Window best = first;
   double best_score = -1.0;
   std::vector<int32_t> work, moves;  // non-exchange and exchange gates taken, per depth
@@ -278,7 +281,7 @@ Window next_window(const std::vector<SGate>& sg, const std::vector<int64_t>& pen
     for (size_t d = 0; d < work.size(); ++d) {
       w += 2.0 * work[d];
       x += 0.2 * moves[d];
-      const double score = (w + x) / (w + 3.0 * (double)d + kPassCost);
+      const double score = (w + x) / (w + 3.0 * (double)d + pass_cost);
       if (score > best_score && w + x > 0.0) {
         best_score = score;
         best.local = local;
