@@ -230,6 +230,7 @@ k_batch_fix(double2* __restrict__ arena, const BatchPass* __restrict__ passes, c
           at[s_slot[u]] = v;
         }
       } else if (!scan.zero()) {
+        prefetch_ops(ops + ps.op_begin, ps.num_ops);
 #pragma unroll
         for (int u = 0; u < kFixAmps; ++u)
           if (tid + NT * u < T) ti[tid + NT * u] = make_longlong2(r[2 * u], r[2 * u + 1]);

@@ -155,15 +155,10 @@ bool permute(DiagTable& d, const Op& op) {
       t.mask ^= flip;
     }
   }
-  // terms whose masks became equal are one term
-  std::vector<PhaseTerm> old;
-  old.swap(d.terms);
+  // an invertible map of the masks: different ones stay different
   d.supp = 0;
-  for (const PhaseTerm& t : old) {
-    if (t.turn == 0) continue;
-    d.add(t.mask, t.turn);
-    d.supp |= t.mask & ((1u << kPhaseGlobalBit) - 1u);
-  }
+  for (const PhaseTerm& t : d.terms)
+    if (t.turn != 0) d.supp |= t.mask & ((1u << kPhaseGlobalBit) - 1u);
   return true;
 }
 

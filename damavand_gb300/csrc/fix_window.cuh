@@ -122,6 +122,7 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
       using V = typename FB::T;
       static_assert(sizeof(V) == 16, "the tile is converted in place");
       V* tv = reinterpret_cast<V*>(tile);
+      prefetch_ops(p.ops, p.num_ops);
       if constexpr (!std::is_same<V, double2>::value) {
 #pragma unroll
         for (int u = 0; u < kFixAmps; ++u)

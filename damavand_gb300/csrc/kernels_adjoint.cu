@@ -384,6 +384,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
     } else if (!zero) {
       double2* dp = reinterpret_cast<double2*>(tp);
       double2* dl = reinterpret_cast<double2*>(tl);
+      prefetch_ops(p.ops, p.num_ops);
 #pragma unroll
       for (int u = 0; u < NA; ++u) {
         tp[tid + NT * u] = make_longlong2(a[2 * u], a[2 * u + 1]);
