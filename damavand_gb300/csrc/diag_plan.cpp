@@ -164,6 +164,15 @@ bool permute(DiagTable& d, const Op& op) {
 
 inline double cabs(double re, double im) { return std::hypot(re, im); }
 
+// 1 / sqrt(s + sl) as y + yl, good to about 2^-100 (long double would do, but
+// is emulated on the host this runs on).
+void inv_sqrt(double s, double sl, double& y, double& yl) {
+  y = 1.0 / std::sqrt(s);
+  const double y2 = y * y, y2l = std::fma(y, y, -y2);
+  const double t = std::fma(-s, y2, 1.0) - s * y2l - sl * y2;  // 1 - (s + sl) y^2
+  yl = 0.5 * y * t;
+}
+
 // U = D1 R D2 (see the file comment). Returns false when the product does not
 // reproduce U to kZyzTol in every entry.
 bool zyz(const double m[8], double& T, double& S, double& C, int64_t& t1, int64_t& t2, int64_t& tg) {
@@ -171,9 +180,13 @@ bool zyz(const double m[8], double& T, double& S, double& C, int64_t& t1, int64_
   // c and s each rounded once from a wider quotient: dividing both by one
   // rounded double r biased c^2 + s^2 (by about 3e-17 per rotation on the
   // benchmark's unitaries, a norm drift of 1e-14 over 600 rotations).
-  const long double rl = std::hypot((long double)ra, (long double)rb);
-  if (!(rl > 0.0L)) return false;
-  const double c = (double)((long double)ra / rl), s = (double)((long double)rb / rl);
+  const double pa = ra * ra, pb = rb * rb, r2 = pa + pb;
+  if (!(r2 > 0.0)) return false;
+  const double r2l = (pa > pb ? pb - (r2 - pa) : pa - (r2 - pb)) + std::fma(ra, ra, -pa) + std::fma(rb, rb, -pb);
+  double y, yl;
+  inv_sqrt(r2, r2l, y, yl);
+  const double ca = ra * y, sa = rb * y;
+  const double c = ca + (std::fma(ra, y, -ca) + ra * yl), s = sa + (std::fma(rb, y, -sa) + rb * yl);
   const double a1 = std::atan2(m[1], m[0]), a2 = std::atan2(m[5], m[4]);
   const double g2 = std::atan2(m[3], m[2]) + M_PI - a1;
   const double e[8] = {c * std::cos(a1),        c * std::sin(a1),
@@ -395,8 +408,10 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
         // gives the state its true scale back.
         (void)Tq;
         const double w = single ? (double)(float)(Sq / Cq) : Sq / Cq;
-        const long double wl = w;
-        const double f = (double)(1.0L / std::sqrt(1.0L + wl * wl));
+        const double w2 = std::fma(w, w, 1.0);
+        double f, fl;
+        inv_sqrt(w2, std::fma(w, w, 1.0 - w2), f, fl);
+        f += fl;
         if (acc.hi * f >= 0x1p-200) {
           r.cls = OP_ROT;
           r.m[0] = w;
@@ -404,8 +419,8 @@ int64_t rewrite_pass_rotations(const Op* src, int64_t count, int32_t k, bool rot
           r.ml[0] = (float)(w - (double)r.mh[0]);
           acc.mul(f);
         } else {
-          const long double F = ((long double)acc.hi + (long double)acc.lo) * (long double)f;
-          const double one = (double)F, ww = (double)(F * wl);
+          acc.mul(f);
+          const double one = acc.hi + acc.lo, ww = acc.hi * w + (std::fma(acc.hi, w, -(acc.hi * w)) + acc.lo * w);
           r.cls = OP_REAL;
           r.m[0] = one;
           r.m[2] = -ww;
