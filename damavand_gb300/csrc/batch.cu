@@ -10,7 +10,8 @@
 // on items claimed before it by CTAs that are already running, so the wait
 // always ends; it is nevertheless bounded, after which the kernel raises an
 // error flag and every CTA returns. The arena reset, the kernel and the
-// per-circuit Pauli-Z reductions are captured in one CUDA graph.
+// circuits' Pauli-Z reductions (one pass over all of them) are captured in one
+// CUDA graph.
 //
 // An autotuner picks the tile size, the number of always-local low qubits
 // and the tiles per item by timing graph runs of the batch itself.
@@ -280,7 +281,10 @@ struct dmv_batch_s {
   void* arena = nullptr;
   cudaStream_t stream = nullptr;
   DeviceBuffer passes_dev, items_dev, ops_dev, counters_dev, offsets_dev, reduce_dev;
-  std::vector<int64_t> red_partial, red_sums;  // per-circuit offsets (doubles) into reduce_dev
+  // Pauli-Z reductions: reduce_dev holds the sums (one column per circuit and qubit, and its total), then the
+  // partials; mass_dev the circuits' BatchMass and the circuit of each CTA and column.
+  DeviceBuffer mass_dev;
+  int32_t mass_ctas = 0, mass_columns = 0;
   int64_t num_items = 0, num_passes = 0, num_ops = 0;
   int32_t max_k = 0;
   PlanOptions opt;
@@ -512,7 +516,7 @@ int batch_launch_fix(dmv_batch_s* b) {
 }
 
 // The whole run as stream work: counters and arena reset, |0...0> per
-// circuit, the persistent kernel, then the per-circuit Pauli-Z reductions.
+// circuit, the persistent kernel, then the Pauli-Z reductions.
 int batch_enqueue(dmv_batch_s* b) {
   DMV_CUDA_TRY(cudaMemsetAsync(b->counters_dev.ptr, 0, (size_t)(2 + b->count) * sizeof(unsigned long long), b->stream));
   DMV_CUDA_TRY(cudaMemsetAsync(b->arena, 0, (size_t)b->total_amps * b->amp_size(), b->stream));
@@ -533,11 +537,11 @@ int batch_enqueue(dmv_batch_s* b) {
     else DMV_TRY(batch_launch_kernel<PolF64>(b));
   }
   double* red = static_cast<double*>(b->reduce_dev.ptr);
-  for (int32_t c = 0; c < b->count; ++c) {
-    const char* base = static_cast<const char*>(b->arena) + (size_t)b->offsets[(size_t)c] * b->amp_size();
-    DMV_TRY(launch_chunk_mass_into(base, b->precision == DMV_C128 ? 0 : 1, b->n[(size_t)c],
-                                   red + b->red_partial[(size_t)c], red + b->red_sums[(size_t)c], b->stream));
-  }
+  const char* md = static_cast<const char*>(b->mass_dev.ptr);
+  const int32_t* of_cta = reinterpret_cast<const int32_t*>(md + (size_t)b->count * sizeof(BatchMass));
+  DMV_TRY(launch_batch_mass(reinterpret_cast<const BatchMass*>(md), of_cta, b->mass_ctas, of_cta + b->mass_ctas,
+                            b->mass_columns, b->arena, b->precision == DMV_C128 ? 0 : 1, red + b->mass_columns, red,
+                            b->stream));
   return DMV_OK;
 }
 
@@ -656,15 +660,28 @@ extern "C" int dmv_batch_create(int32_t num_circuits, const int32_t* num_qubits,
       rc = set_error(DMV_ERR_CUDA, "offset upload failed");
       break;
     }
+    std::vector<BatchMass> mass;
+    std::vector<int32_t> of;  // the circuit of each CTA, then of each column
     int64_t red = 0;
     for (int32_t c = 0; c < num_circuits; ++c) {
-      const ChunkMassShape sh = chunk_mass_shape(b->n[(size_t)c]);
-      b->red_partial.push_back(red);
-      red += sh.partial_elems;
-      b->red_sums.push_back(red);
-      red += b->n[(size_t)c] + 1;
+      const int32_t n = b->n[(size_t)c];
+      const int32_t ctas = batch_mass_ctas(n);
+      mass.push_back(BatchMass{b->offsets[(size_t)c], red, n, b->mass_ctas, ctas, b->mass_columns});
+      red += (int64_t)ctas * (n + 1);
+      b->mass_ctas += ctas;
+      b->mass_columns += n + 1;
+      of.insert(of.end(), (size_t)ctas, c);
     }
-    if ((rc = b->reduce_dev.reserve((size_t)red * sizeof(double))) != DMV_OK) break;
+    for (int32_t c = 0; c < num_circuits; ++c) of.insert(of.end(), (size_t)b->n[(size_t)c] + 1, c);
+    if ((rc = b->reduce_dev.reserve((size_t)(red + b->mass_columns) * sizeof(double))) != DMV_OK) break;
+    const size_t mb = mass.size() * sizeof(BatchMass);
+    if ((rc = b->mass_dev.reserve(mb + of.size() * sizeof(int32_t))) != DMV_OK) break;
+    if (cudaMemcpy(b->mass_dev.ptr, mass.data(), mb, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(static_cast<char*>(b->mass_dev.ptr) + mb, of.data(), of.size() * sizeof(int32_t),
+                   cudaMemcpyHostToDevice) != cudaSuccess) {
+      rc = set_error(DMV_ERR_CUDA, "reduction plan upload failed");
+      break;
+    }
     rc = batch_plan(b);
   } while (false);
   if (rc != DMV_OK) {
@@ -686,6 +703,7 @@ extern "C" int dmv_batch_destroy(dmv_batch_t b) {
   b->counters_dev.release();
   b->offsets_dev.release();
   b->reduce_dev.release();
+  b->mass_dev.release();
   b->fix_ops_dev.release();
   b->tab_dev.release();
   b->fix_tab_dev.release();
@@ -764,15 +782,14 @@ extern "C" int dmv_batch_expect_z(dmv_batch_t b, double* out) {
   clear_error();
   if (!b || !out) return set_error(DMV_ERR_INVALID, "null batch or output");
   DMV_CUDA_TRY(cudaStreamSynchronize(b->stream));
-  DMV_TRY(check_window_status());  // a mass pass whose chunk load wait gave up
-  int64_t pos = 0;
+  std::vector<double> h((size_t)b->mass_columns);
+  DMV_CUDA_TRY(cudaMemcpy(h.data(), b->reduce_dev.ptr, h.size() * sizeof(double), cudaMemcpyDeviceToHost));
+  int64_t pos = 0, col = 0;
   for (int32_t c = 0; c < b->count; ++c) {
     const int n = b->n[(size_t)c];
-    std::vector<double> h((size_t)n + 1);
-    DMV_CUDA_TRY(cudaMemcpy(h.data(), static_cast<double*>(b->reduce_dev.ptr) + b->red_sums[(size_t)c],
-                            h.size() * sizeof(double), cudaMemcpyDeviceToHost));
-    for (int q = 0; q < n; ++q) out[pos + q] = h[(size_t)n] - 2.0 * h[(size_t)q];
+    for (int q = 0; q < n; ++q) out[pos + q] = h[(size_t)(col + n)] - 2.0 * h[(size_t)(col + q)];
     pos += n;
+    col += n + 1;
   }
   return DMV_OK;
 }

@@ -535,16 +535,16 @@ uint32_t tma_wait_limit();
 // The device word those waits set to 1 when they give up.
 int* tma_status_word();
 
-// Pauli-Z mass reduction into caller-provided device buffers: `partial`
-// holds partial_elems doubles, `sums` n+1 (mass with bit q set for q < n,
-// then the total).
-struct ChunkMassShape {
-  int chunk_bits;
-  int64_t num_chunks;
-  int grid;
-  int64_t partial_elems;
+// Pauli-Z mass reduction of every circuit of a batch in one pass: circuit c's
+// CTAs first_cta .. + ctas leave n + 1 sums each at `partial`, and columns
+// first_column .. + n of `sums` get the mass with bit q set (q < n), then the total.
+struct BatchMass {
+  int64_t amp_offset;
+  int64_t partial;  // doubles
+  int32_t n, first_cta, ctas, first_column;
 };
-ChunkMassShape chunk_mass_shape(int n);
-int launch_chunk_mass_into(const void* src, int src_kind, int n, double* partial, double* sums,
-                           cudaStream_t stream);
+int batch_mass_ctas(int n);
+int launch_batch_mass(const BatchMass* circuits, const int32_t* circuit_of_cta, int ctas, const int32_t* circuit_of_column,
+                      int columns, const void* arena, int src_kind, double* partial, double* sums,
+                      cudaStream_t stream);
 }  // namespace dmv

@@ -156,8 +156,8 @@ constexpr int kF2ChunkBits = 12;
 // the chunk-index bits. Per CTA: partial[cta * (n+1) + q] = mass with bit q
 // set (q < n), partial[cta * (n+1) + n] = the total.
 template <int SRC>
-__global__ void __launch_bounds__(kRedThreads)
-k_chunk_mass_f2(const void* src, int n, int chunk_bits, int64_t num_chunks, double* __restrict__ partial) {
+__device__ __forceinline__ void chunk_mass_f2(const void* src, int n, int chunk_bits, int64_t num_chunks, int cta,
+                                              int grid, double* __restrict__ partial) {
   __shared__ F2 red[kRedThreads / 32];
   __shared__ double tsum[kRedThreads];
   __shared__ double rsum[4][kRedThreads];
@@ -168,7 +168,7 @@ k_chunk_mass_f2(const void* src, int n, int chunk_bits, int64_t num_chunks, doub
   for (int r = 0; r < kF2Rows; ++r) v[r] = F2{0.f, 0.f};
   if (threadIdx.x < 34) hi_acc[threadIdx.x] = 0.;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int64_t ch = blockIdx.x; ch < num_chunks; ch += gridDim.x) {
+  for (int64_t ch = cta; ch < num_chunks; ch += grid) {
     const int64_t base = ch << chunk_bits;
     F2 mine{0.f, 0.f};
 #pragma unroll
@@ -206,7 +206,7 @@ k_chunk_mass_f2(const void* src, int n, int chunk_bits, int64_t num_chunks, doub
 #pragma unroll
   for (int j = 0; j < 4; ++j) rsum[j][threadIdx.x] = f2_val(R[j]);
   __syncthreads();
-  double* out = partial + (int64_t)blockIdx.x * (n + 1);
+  double* out = partial + (int64_t)cta * (n + 1);
   // one warp per output (a thread adding the 256 sums one by one took 15 us)
   for (int q = warp; q <= chunk_bits; q += kRedThreads / 32) {
     double acc = 0.;
@@ -222,6 +222,26 @@ k_chunk_mass_f2(const void* src, int n, int chunk_bits, int64_t num_chunks, doub
   if (threadIdx.x == 0)
     for (int j = 0; j < n - chunk_bits; ++j) out[chunk_bits + j] = hi_acc[j];
 }
+template <int SRC>
+__global__ void __launch_bounds__(kRedThreads)
+k_chunk_mass_f2(const void* src, int n, int chunk_bits, int64_t num_chunks, double* __restrict__ partial) {
+  chunk_mass_f2<SRC>(src, n, chunk_bits, num_chunks, (int)blockIdx.x, (int)gridDim.x, partial);
+}
+
+// The pass over every circuit of a batch at once (its states are too small to
+// fill the chip one after the other): CTA by CTA from `work`, then the columns'
+// sums (k_batch_mass_sums), one CTA for each.
+template <int SRC>
+__global__ void __launch_bounds__(kRedThreads)
+k_batch_mass(const BatchMass* __restrict__ circuits, const int32_t* __restrict__ circuit_of,
+             const void* __restrict__ arena, double* __restrict__ partial) {
+  using G = typename std::conditional<SRC == 0, double2, float2>::type;
+  const BatchMass m = circuits[circuit_of[blockIdx.x]];
+  const int cb = min(kF2ChunkBits, m.n);
+  chunk_mass_f2<SRC>(static_cast<const G*>(arena) + m.amp_offset, m.n, cb, int64_t(1) << (m.n - cb),
+                     (int)blockIdx.x - m.first_cta, m.ctas, partial + m.partial);
+}
+
 static_assert((1 << kF2ChunkBits) == kRedThreads * kF2Rows, "a chunk is one amplitude per thread and row");
 
 // ---------------------------------------------------------------------------
@@ -541,6 +561,21 @@ k_reduce_partials(const double* __restrict__ partial, int width, int rows, doubl
   __shared__ double red[kPartialThreads / 32];
   double acc = 0.;
   for (int r = threadIdx.x; r < rows; r += kPartialThreads) acc += partial[(int64_t)r * width + blockIdx.x];
+  acc = warp_sum_f64(acc);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) out[blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
+}
+
+// The same for every circuit of a batch: CTA b sums column b of all circuits' columns.
+__global__ void __launch_bounds__(kPartialThreads)
+k_batch_mass_sums(const BatchMass* __restrict__ circuits, const int32_t* __restrict__ circuit_of_column,
+                  const double* __restrict__ partial, double* __restrict__ out) {
+  __shared__ double red[kPartialThreads / 32];
+  const BatchMass m = circuits[circuit_of_column[blockIdx.x]];
+  const int q = (int)blockIdx.x - m.first_column;
+  double acc = 0.;
+  for (int r = threadIdx.x; r < m.ctas; r += kPartialThreads) acc += partial[m.partial + (int64_t)r * (m.n + 1) + q];
   acc = warp_sum_f64(acc);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
@@ -1179,8 +1214,7 @@ int mass_grid_for(int src_kind, int n, int64_t num_chunks) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(num_chunks, (int64_t)sm_count() * per_sm));
 }
 
-// Opts the bulk-staged pass into its shared memory (once per process; done
-// before any graph capture by the batch engine's setup).
+// Opts the bulk-staged pass into its shared memory (once per process).
 template <int SRC>
 void mass_bulk_attributes() {
   static const cudaError_t attr = cudaFuncSetAttribute(
@@ -1329,24 +1363,17 @@ int run_sampler(const void* src, int src_kind, int n, DeviceBuffer& prefix, Devi
 
 }  // namespace
 
-ChunkMassShape chunk_mass_shape(int n) {
-  ChunkMassShape sh;
-  sh.chunk_bits = mass_chunk_bits_for(n);
-  sh.num_chunks = int64_t(1) << (n - sh.chunk_bits);
-  sh.grid = mass_grid_for(0, n, sh.num_chunks);  // the same grid for complex64
-  mass_bulk_attributes<0>();
-  mass_bulk_attributes<1>();
-  sh.partial_elems = (int64_t)sh.grid * (n + 1);
-  return sh;
+int batch_mass_ctas(int n) {
+  const int64_t chunks = int64_t(1) << std::max(0, n - kF2ChunkBits);
+  return (int)std::min<int64_t>(chunks, (int64_t)sm_count() * 8);
 }
 
-int launch_chunk_mass_into(const void* src, int src_kind, int n, double* partial, double* sums,
-                           cudaStream_t stream) {
-  if (src_kind != 0 && src_kind != 1)
-    return set_error(DMV_ERR_INVALID, "launch_chunk_mass_into takes amplitudes (kinds 0, 1)");
-  const ChunkMassShape sh = chunk_mass_shape(n);
-  launch_mass_kernel(src, src_kind, n, sh.chunk_bits, sh.num_chunks, sh.grid, partial, stream);
-  k_reduce_partials<<<n + 1, kPartialThreads, 0, stream>>>(partial, n + 1, sh.grid, sums);
+int launch_batch_mass(const BatchMass* circuits, const int32_t* circuit_of_cta, int ctas, const int32_t* circuit_of_column,
+                      int columns, const void* arena, int src_kind, double* partial, double* sums,
+                      cudaStream_t stream) {
+  if (src_kind == 0) k_batch_mass<0><<<ctas, kRedThreads, 0, stream>>>(circuits, circuit_of_cta, arena, partial);
+  else k_batch_mass<1><<<ctas, kRedThreads, 0, stream>>>(circuits, circuit_of_cta, arena, partial);
+  k_batch_mass_sums<<<columns, kPartialThreads, 0, stream>>>(circuits, circuit_of_column, partial, sums);
   count_launch(2);
   DMV_CUDA_TRY(cudaGetLastError());
   return DMV_OK;

@@ -111,3 +111,24 @@ def test_pair_states_off_the_integers(built_lib, oracle_mod, start):
     want = oracle_forward_any_control(oracle_mod, n, gates, psi)
     got = _run(n, gates, psi, ARITH_FP32X2)
     assert np.max(np.abs(got - want)) <= 2 * len(gates) * 2.0 ** -47 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("shape", ["ladder", "ring", "random"])
+@pytest.mark.parametrize("n", [12, 13, 17])
+def test_complex64_shapes(built_lib, oracle_mod, n, shape):
+    """The complex64 passes on the same shapes; each output is rounded to 2^-24 of itself, the
+    rotations' and tables' entries likewise."""
+    from damavand_gb300 import workloads as wl
+    rng = np.random.default_rng(40 + n)
+    gates = {"ladder": lambda: wl.ladder_circuit(n, 6, 1, False), "ring": lambda: wl.ring_ansatz(n, 6, 2),
+             "random": lambda: wl.random_circuit(n, 12, rng)}[shape]()
+    psi = random_state(n, rng)
+    want = oracle_forward_any_control(oracle_mod, n, gates, psi)
+    st = new_state(n, 1)
+    try:
+        load_state(st, psi)
+        apply_gates(st, gates, 1)
+        got = st.numpy().astype(np.complex128)
+    finally:
+        free_state(st)
+    assert np.max(np.abs(got - want)) <= 2 * len(gates) * 2.0 ** -24 * np.max(np.abs(want))
