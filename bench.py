@@ -42,12 +42,14 @@ sys.path.insert(0, REPO)
 
 METRIC = "30-qubit gate applies/s + HBM GB/s; adjoint vs param-shift grads/s at 1e-10"
 UNIT = "gate-applies/s"
-DTYPES = {"fp64": "f64 (complex128 storage, IEEE FP64 arithmetic; fused passes as real rotations, one "
-                  "multiply-add per output with their factors multiplied back once, and per-amplitude phase "
-                  "tables)",
+DTYPES = {"fp64": "f64 (complex128 storage; fused passes as real rotations with their factors multiplied back "
+                  "once, and per-amplitude phase tables; tiles of like-sized amplitudes in 64-bit fixed point, "
+                  "57 bits under the tile's largest component, the others in IEEE FP64; error against 64-bit "
+                  "values below plain FP64's)",
           "fp64-direct": "f64 (complex128 storage, IEEE FP64 arithmetic; every fused 2x2 as a full complex "
                          "multiply-add)",
-          "fp32x2": "f32x2 (complex128 storage, FP32-pair arithmetic, ~48-bit)",
+          "fp32x2": "f32x2 (complex128 storage, FP32-pair arithmetic, ~48-bit; tiles of like-sized amplitudes in "
+                    "64-bit fixed point as fp64's)",
           "int64": "int64 (complex128 storage, block fixed point: 54-bit fraction per tile, exact products)",
           "tc": "int64 (complex128 storage, block fixed point: 56-bit fraction per tile; fused gates as dense "
                 "5-qubit blocks, exact products of FP16 digits on the tcgen05 tensor cores)"}
@@ -57,6 +59,9 @@ INT_MAD_PEAK_T = 18.85
 # (0.504 T FMA/s = 1.0 TFLOP/s); complex128 arithmetic is bounded by it.
 FP64_FMA_PEAK_T = 0.504
 FP32_FMA_PEAK_T = 35.9
+# 32 x 32 -> 64-bit (or high-word) integer products: one per warp and SM quarter every 4.0 cycles, measured with
+# independent chains.
+INT_WIDE_PEAK_T = 9.68
 # dram__bytes_read.sum + dram__bytes_write.sum per launch divided by the amplitudes of
 # the captured case: one ncu capture per kernel on a smaller state of the same ladder
 # workload (dram__bytes.sum.per_second x gpu__time_duration.sum: k_window_tma<PolF64>
@@ -64,16 +69,15 @@ FP32_FMA_PEAK_T = 35.9
 # 476.1 MB at 2^24; k_apply_window<PolDF> 492.7 MB and k_apply_window<PolFX> 493.1 MB at
 # 2^24). Traffic is the state read plus written once per pass, so it scales with the
 # number of amplitudes.
-NCU_TRAFFIC_PER_AMPLITUDE = {("window", "c128"): 479.1e6 / (1 << 24),
-                             ("window", "c64"): 1012.4e6 / (1 << 26),
+NCU_TRAFFIC_PER_AMPLITUDE = {("window", "c128"): 482.2e6 / (1 << 24),
+                             ("window", "c64"): 2086.6e6 / (1 << 27),
                              ("window", "c128", "tc"): 476.1e6 / (1 << 24),
-                             ("window", "c128", "fp32x2"): 492.7e6 / (1 << 24),
                              ("window", "c128", "int64"): 493.1e6 / (1 << 24)}
 # The kernel that runs a fused window pass, by arithmetic and precision.
-WINDOW_KERNEL = {("fp64", "c128"): "k_window_tma<PolF64>", ("fp64-direct", "c128"): "k_window_tma<PolF64>",
-                 ("fp32x2", "c128"): "k_apply_window<PolDF>",
+WINDOW_KERNEL = {("fp64", "c128"): "k_window_fix<PolF64>", ("fp64-direct", "c128"): "k_window_tma<PolF64>",
+                 ("fp32x2", "c128"): "k_window_fix<PolDF>",
                  ("int64", "c128"): "k_apply_window<PolFX>", ("tc", "c128"): "k_window_tc",
-                 ("fp32", "c64"): "k_window_phases<PolF32>"}
+                 ("fp32", "c64"): "k_window_f32"}
 
 
 def load_peaks():
@@ -636,12 +640,17 @@ def rooflines(fam, n, arith, prec="c128"):
     roofline = {"bound": "hbm", "kernel": kernel, "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic, "peak_source": peak_kind,
                 "algorithmic_bytes_per_launch": per_launch_bytes, "avg_launch_ms": avg_launch_s * 1e3}
-    # The same kernel against the arithmetic ceiling it meets on GB300: FP64
-    # multiply-adds for IEEE FP64 arithmetic, FP32 operations for FP32-pair arithmetic.
+    # The same kernel against the arithmetic ceiling it meets on GB300: integer
+    # products for the fixed-point passes, FP64 multiply-adds for direct FP64.
     rate = d["arith_ops"] / (d["ms"] / 1e3) / 1e12 if d["ms"] else 0.0
-    if arith in ("fp64", "fp64-direct"):
+    if prec == "c128" and arith in ("fp64", "fp32x2"):
+        ra = {"bound": "int-wide", "achieved": rate, "peak": INT_WIDE_PEAK_T, "unit": "T product/s",
+              "frac": rate / INT_WIDE_PEAK_T,
+              "peak_source": "measured (32 x 32-bit product chain kernel on a GB300); counts the passes' "
+                             "products: 3 per rotation output, 6 per component and phase table"}
+    elif arith == "fp64-direct":
         ra = {"bound": "fp64", "achieved": rate, "peak": FP64_FMA_PEAK_T, "unit": "T FMA/s",
-              "frac": rate / FP64_FMA_PEAK_T, "peak_source": "measured (FP64 FMA chain kernel on this pool's GB300)"}
+              "frac": rate / FP64_FMA_PEAK_T, "peak_source": "measured (FP64 FMA chain kernel on a GB300)"}
     elif arith == "tc":
         tpeak, tkind = load_tensor_peak()
         ra = {"bound": "tensor", "achieved": rate, "peak": tpeak, "unit": "TFLOP/s",
@@ -651,10 +660,10 @@ def rooflines(fam, n, arith, prec="c128"):
     elif arith == "int64":
         ra = {"bound": "int-mad", "achieved": rate, "peak": INT_MAD_PEAK_T, "unit": "T IMAD/s",
               "frac": rate / INT_MAD_PEAK_T,
-              "peak_source": "measured (32-bit IMAD chain kernel on this pool's GB300); counts IMAD.WIDE limb products"}
+              "peak_source": "measured (32-bit IMAD chain kernel on a GB300); counts IMAD.WIDE limb products"}
     else:
         ra = {"bound": "fp32", "achieved": rate, "peak": FP32_FMA_PEAK_T, "unit": "T op/s",
-              "frac": rate / FP32_FMA_PEAK_T, "peak_source": "measured (FP32 FMA chain kernel on this pool's GB300)"}
+              "frac": rate / FP32_FMA_PEAK_T, "peak_source": "measured (FP32 FMA chain kernel on a GB300)"}
     total_bytes = sum(v["bytes"] for v in fam.values())
     total_ms = sum(v["ms"] for v in fam.values())
     return roofline, ra, (total_bytes / (total_ms / 1e3) / 1e9 if total_ms else None)

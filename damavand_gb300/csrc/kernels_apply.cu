@@ -798,6 +798,14 @@ double op_multiply_adds(const Op& op, int64_t N, int arith) {
   return per_pair * pairs * (op.ctrl_kind != CTRL_NONE ? 0.5 : 1.0);
 }
 
+// The same for the passes in register phases: 32 x 32-bit products of the
+// fixed-point pass (3 per rotation output, 6 per component and table), FP32
+// multiply-adds of the complex64 one (1 and 2).
+double phase_pass_products(const Op& op, int64_t N, bool single) {
+  const double reals = 2.0 * (double)N;
+  return op.cls == OP_ROT ? reals * (single ? 1. : 3.) : op.cls == OP_PHASE ? reals * (single ? 2. : 6.) : 0.;
+}
+
 // Register bits of a window pass that runs in register phases (complex64
 // passes on the TMA kernel), 0 otherwise.
 int window_reg_bits(const dmv_state_s* s, const Pass& ps) {
@@ -1114,8 +1122,10 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       bytes += b;
     } else {
       double fmas = 0.;
-      for (int64_t o = 0; o < ps.op_count; ++o)
-        fmas += op_multiply_adds(ops[(size_t)(ps.op_begin + o)], s->N, arith);
+      for (int64_t o = 0; o < ps.op_count; ++o) {
+        const Op& op = ops[(size_t)(ps.op_begin + o)];
+        fmas += fix_first[pi] >= 0 ? phase_pass_products(op, s->N, single) : op_multiply_adds(op, s->N, arith);
+      }
       const int64_t tok = prof_begin(DMV_KERNEL_WINDOW, s->stream, (double)(2 * S), fmas);
       void* a = s->amps;
       cudaStream_t st = s->stream;
