@@ -89,10 +89,11 @@ class Circuit:
         self.set_arithmetic(arithmetic)
 
     def set_arithmetic(self, arithmetic: str) -> None:
-        """Arithmetic on the complex128 amplitudes (complex64 ignores it): 'fp64' (IEEE FP64;
-        fused passes apply real rotations and phase tables), 'fp64-direct' (IEEE FP64,
+        """Arithmetic on the complex128 amplitudes (complex64 ignores it): 'fp64' (fused
+        passes as real rotations and phase tables, in 64-bit fixed point on tiles of
+        like-sized amplitudes and IEEE FP64 elsewhere), 'fp64-direct' (IEEE FP64,
         every fused 2x2 as a full complex multiply-add), 'fp32x2' (FP32-pair error-free
-        arithmetic, ~1e-13 normwise on deep circuits), 'int64' (block fixed point with exact
+        arithmetic where 'fp64' is IEEE FP64, below 1e-13 normwise on deep circuits), 'int64' (block fixed point with exact
         integer products) or 'tc' (the same block fixed point, fused gates applied as dense
         5-qubit blocks by exact digit products on the tensor cores)."""
         modes = {"fp64": _lib.ARITH_FP64, "fp64-direct": _lib.ARITH_FP64_DIRECT, "fp32x2": _lib.ARITH_FP32X2,

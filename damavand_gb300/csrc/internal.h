@@ -186,8 +186,8 @@ void split_matrix(Op& op);
 // `rot_ops` true: rotations as OP_ROT (the FP64 kernels: two multiply-adds
 // per component, the state left divided by each rotation's factor f, whose
 // product over the pass is multiplied into *scale); false: as OP_REAL 2x2 ops
-// (with their FP32-pair, Q.54 and FP32 forms), for the other arithmetics,
-// which read the tables converted by phase_entry_value.
+// (with their FP32-pair, Q.54 and FP32 forms), for the int64 arithmetic and
+// for FP32 pairs outside the fixed-point passes.
 // A product of many factors kept to about 2^-100 relative (error-free
 // products through fma), for the OP_ROT factors.
 struct ScaleDD {

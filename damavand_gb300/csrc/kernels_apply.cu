@@ -12,13 +12,16 @@
 //    of the pass to it, and writes it back: one read and one write of the
 //    statevector for the whole window of gates. A control qubit outside the
 //    tile is constant over the tile and is tested once per tile.
-//  * k_window_tma: the same pass for full-size tiles (2^12 complex128 or
-//    2^13 complex64 amplitudes with at least three high qubits). One
-//    persistent CTA per SM; tiles move HBM <-> shared memory by TMA
-//    (cp.async.bulk.tensor over a per-pass 5-D tensor map), three buffers
-//    deep: tile i+1 loads and tile i-1 drains while tile i computes. The ops
-//    run in register phases (phases.cuh), so the tile crosses shared memory
-//    once per phase instead of once per op.
+//  * k_window_fix (fix_window.cuh), k_window_f32 (f32_window.cuh): a rewritten
+//    pass over 2^12-amplitude tiles in register phases, complex128 in 64-bit
+//    fixed point and complex64 in FP32: what nearly every pass runs on.
+//  * k_window_tma, k_window_phases: passes over such tiles with ops those do
+//    not take (controlled non-exchanges, non-unitary matrices), complex128 in
+//    FP64 and complex64; tiles move by TMA (cp.async.bulk.tensor over a
+//    per-pass 5-D tensor map).
+//  * k_window_tc (tc_window.cuh): complex128 passes as dense blocks on the
+//    tensor cores.
+//  * k_phase_tables: the phase tables' entries from their terms.
 #include <cuda.h>
 #include <cuda_fp16.h>
 

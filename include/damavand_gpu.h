@@ -53,23 +53,27 @@ enum { DMV_C128 = 0, DMV_C64 = 1 };
 
 /* Arithmetic of complex128 gate application (complex64 always computes in FP32).
  * The amplitudes are IEEE complex128 in device memory between calls in every mode.
- * DMV_ARITH_FP64: IEEE FP64 arithmetic (default). Fused window passes on the
- *   TMA kernel write each uncontrolled unitary 2x2 as diagonal x real rotation
- *   x diagonal, apply the rotation as a scaled matrix with one FP64
- *   multiply-add per output (2 per amplitude instead of 8; the product of the
- *   scale factors is multiplied back into the state once per forward) and
- *   collect the diagonals of a pass into a few per-amplitude phase tables,
- *   each applied with three shears (3 multiply-adds per amplitude).
+ * DMV_ARITH_FP64: the default. Fused window passes write each uncontrolled
+ *   unitary 2x2 as diagonal x real rotation x diagonal, apply the rotation as
+ *   a scaled matrix (the product of the scale factors is multiplied back into
+ *   the state once per forward) and collect the diagonals of a pass into a few
+ *   per-amplitude phase tables. Tiles of 2^12 amplitudes within 2^12 of one
+ *   another run in 64-bit fixed point, 57 bits for the tile's largest
+ *   component, one rounding per output; every other tile (and pass, and state
+ *   below 12 qubits) in IEEE FP64. Measured errors against 64-bit values are
+ *   below those of FP64 throughout.
  * DMV_ARITH_FP64_DIRECT: IEEE FP64 with every fused 2x2 applied as a full
  *   complex multiply-add (8 per amplitude for a general matrix).
- * The FP32-pair and int64 arithmetics below take the same rotation and phase
- * table rewrite of their fused passes, with each rotation a real 2x2.
+ * The FP32-pair and int64 arithmetics below take the same rewrite of their
+ * fused passes.
  * DMV_ARITH_FP32X2: the FP64 amplitudes are split into FP32 pairs (about 48
  *   significant bits) inside each kernel and combined with error-free
  *   transformations, then stored back as FP64; GB300 runs FP32 ~71x faster
- *   than FP64. Between the window passes of one gate list the state keeps the
- *   pair form (the same 16 bytes per amplitude); it is IEEE complex128 again
- *   when the call returns. Measured error on deep circuits ~1e-13 normwise.
+ *   than FP64. Tiles that DMV_ARITH_FP64 would run in fixed point do so here
+ *   as well. Where all passes of a gate list are in pairs the state keeps that
+ *   form between them (the same 16 bytes per amplitude); it is IEEE complex128
+ *   again when the call returns. Measured error on deep circuits below 1e-13
+ *   normwise.
  * DMV_ARITH_INT64: each tile (or pair) is converted to int64 fixed point with
  *   one shared exponent (54 fraction bits for its largest components) and
  *   multiplied exactly in 31-bit limbs on the integer pipe, with one rounding
@@ -81,8 +85,8 @@ enum { DMV_C128 = 0, DMV_C64 = 1 };
  *   (7 per 56-bit integer, FP16) on the tensor cores (tcgen05.mma, FP32
  *   accumulators in tensor memory, every sum exact), rounded once per
  *   output. Passes it does not take run as DMV_ARITH_INT64. Single states
- *   only (batches accept FP64, FP64_DIRECT, FP32X2 and INT64; a batch applies
- *   every fused 2x2 directly, as DMV_ARITH_FP64_DIRECT does). */
+ *   only (batches accept FP64, FP64_DIRECT, FP32X2 and INT64; the last three
+ *   apply every fused 2x2 directly). */
 enum { DMV_ARITH_FP64 = 0, DMV_ARITH_FP32X2 = 1, DMV_ARITH_INT64 = 2, DMV_ARITH_TC = 3, DMV_ARITH_FP64_DIRECT = 4 };
 
 /* Gate kinds (numbering shared with the oracle). DMV_GATE_MATRIX takes an
@@ -191,8 +195,8 @@ int dmv_last_plan_stats(int64_t* num_passes, int64_t* num_fused_ops, int64_t* by
  * blocks and their exchange stages (zeros for other arithmetics). */
 int dmv_last_tc_stats(dmv_state_t s, int64_t* tc_passes, int64_t* blocks, int64_t* exchanges);
 /* Bytes the last gate application on `s` copied from the host to the device
- * (the plan's op list, phase tables, tensor-core stages and digit matrices),
- * and of those the phase tables of the FP64 rotation passes. No reference
+ * (the plan's op lists, the terms of its phase tables, tensor-core stages and
+ * digit matrices), and of those the terms. No reference
  * counterpart. */
 int dmv_last_upload_bytes(dmv_state_t s, int64_t* total, int64_t* phase_tables);
 /* Plans a gate list without touching a GPU (host only): the number of HBM
