@@ -231,12 +231,11 @@ k_batch_fix(double2* __restrict__ arena, const BatchPass* __restrict__ passes, c
           at[s_slot[u]] = v;
         }
       } else if (!scan.zero()) {
-        prefetch_ops(ops + ps.op_begin, ps.num_ops);
 #pragma unroll
         for (int u = 0; u < kFixAmps; ++u)
           if (tid + NT * u < T) ti[tid + NT * u] = make_longlong2(r[2 * u], r[2 * u + 1]);
-        __syncthreads();
-        tile_apply_ops<PolF64>(td, T, ops + ps.op_begin, ps.num_ops, base, tab);
+        tile_apply_ops_staged<PolF64>(td, T, ops + ps.op_begin, ps.num_ops, base, tab, ti + (1 << 12), (int)kFixStage);
+        __syncthreads();  // (no ops: the tile's threads)
         const double f = scalbn(ps.out_frac, ps.out_exp);
 #pragma unroll
         for (int u = 0; u < kFixAmps; ++u)

@@ -122,14 +122,12 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
       using V = typename FB::T;
       static_assert(sizeof(V) == 16, "the tile is converted in place");
       V* tv = reinterpret_cast<V*>(tile);
-      prefetch_ops(p.ops, p.num_ops);
       if constexpr (!std::is_same<V, double2>::value) {
 #pragma unroll
         for (int u = 0; u < kFixAmps; ++u)
           tv[tid + NT * u] = FB::in(make_double2(__longlong_as_double(r[2 * u]), __longlong_as_double(r[2 * u + 1])));
       }
-      __syncthreads();
-      tile_apply_ops<FB>(tv, T, p.ops, p.num_ops, base, p.phase_tab);
+      tile_apply_ops_staged<FB>(tv, T, p.ops, p.num_ops, base, p.phase_tab, ti + T, (int)kFixStage);
 #pragma unroll
       for (int u = 0; u < kFixAmps; ++u) {
         const double2 v = FB::out(tv[tid + NT * u]);

@@ -384,15 +384,21 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
     } else if (!zero) {
       double2* dp = reinterpret_cast<double2*>(tp);
       double2* dl = reinterpret_cast<double2*>(tl);
-      prefetch_ops(p.ops, p.num_ops);
 #pragma unroll
       for (int u = 0; u < NA; ++u) {
         tp[tid + NT * u] = make_longlong2(a[2 * u], a[2 * u + 1]);
         tl[tid + NT * u] = make_longlong2(b[2 * u], b[2 * u + 1]);
       }
-      __syncthreads();
+      constexpr int kFit = (int)(kAdjStage / sizeof(Op));  // ops staged at a time
       for (int o = 0; o < p.num_ops; ++o) {
-        const Op& op = p.ops[o];
+        if (o % kFit == 0) {
+          __syncthreads();
+          const int4* src = reinterpret_cast<const int4*>(p.ops + o);
+          int4* dst = reinterpret_cast<int4*>(tl + T);
+          for (int i = tid; i < min(kFit, p.num_ops - o) * (int)(sizeof(Op) / sizeof(int4)); i += NT) dst[i] = src[i];
+          __syncthreads();
+        }
+        const Op& op = reinterpret_cast<const Op*>(tl + T)[o % kFit];
         if (op.ctrl_kind == CTRL_GLOBAL && !((base >> op.ctrl) & 1)) continue;  // uniform per tile
         if (op.cls == OP_GRAD) {
           double gx = 0.0, gy = 0.0, gz = 0.0;
@@ -436,6 +442,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
         }
         __syncthreads();
       }
+      __syncthreads();
       const double f = scalbn(1.0, p.scale_exp);
 #pragma unroll
       for (int u = 0; u < NA; ++u) {

@@ -131,6 +131,7 @@ struct WindowParams {
   int64_t num_tiles;
   const Op* ops;
   const void* tab;   // phase tables of the pass's OP_PHASE ops, in the policy's form
+  int32_t stage_bytes;  // shared memory behind the tile for the ops, 0: read from HBM
 };
 
 static_assert(kWindowThreads == kTileThreads, "tile staging assumes 512 threads");
@@ -150,7 +151,6 @@ k_apply_window(typename P::G* __restrict__ a, const WindowParams p) {
   const int T = 1 << p.k;
   const int64_t t_off = tile_thread_offset(p.low, p.nh, p.high);
   tile_slot_offsets(p.low, p.nh, p.high, (T + kTileThreads - 1) >> kTileThreadBits, s_slot);
-  prefetch_ops(p.ops, p.num_ops);
   __syncthreads();
   __shared__ int s_red[kTileThreads / 32];
   for (int64_t tix = blockIdx.x; tix < p.num_tiles; tix += gridDim.x) {
@@ -166,7 +166,8 @@ k_apply_window(typename P::G* __restrict__ a, const WindowParams p) {
       if constexpr (FMT & 1) tile_load<PolRaw<P>, false>(tile, reinterpret_cast<const V*>(a), base, T, t_off, s_slot);
       else tile_load<P, false>(tile, a, base, T, t_off, s_slot);
       __syncthreads();
-      tile_apply_ops<P>(tile, T, p.ops, p.num_ops, base, p.tab);
+      if (p.stage_bytes) tile_apply_ops_staged<P>(tile, T, p.ops, p.num_ops, base, p.tab, tile + T, p.stage_bytes);
+      else tile_apply_ops<P>(tile, T, p.ops, p.num_ops, base, p.tab);
       if constexpr (FMT & 2) tile_store<PolRaw<P>>(tile, reinterpret_cast<V*>(a), base, T, t_off, s_slot);
       else tile_store<P>(tile, a, base, T, t_off, s_slot);
     }
@@ -187,7 +188,10 @@ int launch_window_fmt(void* amps, int32_t n, const Pass& ps, const Op* ops_dev, 
   p.num_tiles = int64_t(1) << (n - p.k);
   p.ops = ops_dev + ps.op_begin;
   p.tab = tab;
-  const size_t smem = (size_t(1) << p.k) * sizeof(V);
+  const size_t tile = (size_t(1) << p.k) * sizeof(V);
+  // A state of one tile has the SM to itself: its ops go to shared memory.
+  p.stage_bytes = p.num_tiles == 1 ? (int32_t)(std::min<size_t>((size_t)p.num_ops, 128) * sizeof(Op)) : 0;
+  const size_t smem = tile + (size_t)p.stage_bytes;
   static size_t configured = 0;
   if (smem > configured) {
     DMV_CUDA_TRY(cudaFuncSetAttribute(k_apply_window<P, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -433,7 +437,6 @@ k_window_tma(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ T
   }
   const int64_t t_off = tile_thread_offset(low, nh, p.high);
   tile_slot_offsets(low, nh, p.high, (T + kTileThreads - 1) >> kTileThreadBits, s_slot);
-  prefetch_ops(p.ops, p.num_ops);
   __syncthreads();
   const TileGeom<ES> geom{low, nh, s_high};
   const int lane = (int)(threadIdx.x & 31);

@@ -461,14 +461,6 @@ __device__ __forceinline__ void tile_phase_fx(longlong2* tile, int T, const Op& 
   }
 }
 
-// Brings a pass's ops into this SM's L1 at once: read one after the other as
-// they are applied, each costs the L2's latency (a 10-qubit state's 90 ops).
-__device__ __forceinline__ void prefetch_ops(const Op* ops, int num_ops) {
-  const char* p = reinterpret_cast<const char*>(ops);
-  for (int i = (int)threadIdx.x * 128; i < num_ops * (int)sizeof(Op); i += (int)blockDim.x * 128)
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + i));
-}
-
 // Every op of a pass on one tile; `base` holds the tile's global index bits
 // (controls outside the tile are read from it). Ends with a barrier after
 // each applied op. `tab` holds the phase tables of OP_PHASE ops in the
@@ -518,6 +510,26 @@ __device__ __forceinline__ void tile_apply_ops(typename P::T* tile, int T, const
       default: tile_op<P, OP_GENERAL>(tile, T, op); break;
     }
     __syncthreads();
+  }
+}
+
+// The same with the ops copied to `stage` (shared memory, `bytes` of it) first,
+// as many at a time as fit: read one after the other from L2 as they are
+// applied, every op costs its latency, which is most of a small tile's time (a
+// 10-qubit state's 90 ops: 73 us, 54 so). All threads call it; `stage` may be
+// in use until the first barrier.
+template <typename P>
+__device__ __forceinline__ void tile_apply_ops_staged(typename P::T* tile, int T, const Op* ops, int num_ops,
+                                                      int64_t base, const void* tab, void* stage, int bytes) {
+  const int fit = bytes / (int)sizeof(Op);
+  for (int o = 0; o < num_ops; o += fit) {
+    const int n = min(fit, num_ops - o);
+    __syncthreads();
+    const int4* src = reinterpret_cast<const int4*>(ops + o);
+    int4* dst = static_cast<int4*>(stage);
+    for (int i = (int)threadIdx.x; i < n * (int)(sizeof(Op) / sizeof(int4)); i += (int)blockDim.x) dst[i] = src[i];
+    __syncthreads();
+    tile_apply_ops<P>(tile, T, static_cast<const Op*>(stage), n, base, tab);
   }
 }
 
