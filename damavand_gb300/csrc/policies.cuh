@@ -521,6 +521,7 @@ __device__ __forceinline__ void tile_apply_ops(typename P::T* tile, int T, const
 template <typename P>
 __device__ __forceinline__ void tile_apply_ops_staged(typename P::T* tile, int T, const Op* ops, int num_ops,
                                                       int64_t base, const void* tab, void* stage, int bytes) {
+  static_assert(sizeof(Op) % sizeof(int4) == 0, "ops are copied in 16-byte words");
   const int fit = bytes / (int)sizeof(Op);
   for (int o = 0; o < num_ops; o += fit) {
     const int n = min(fit, num_ops - o);
