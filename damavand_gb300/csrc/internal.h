@@ -275,6 +275,7 @@ struct PlanOptions {
   int32_t tile_bits = 12;  // log2 amplitudes per tile
   int32_t low_bits = 6;    // always-local low qubits (coalesced chunks)
   bool search_windows = false;  // choose each window by a search (next_window) instead of the first targets met
+  double pass_cost = 0.0;       // next_window's cost of a pass, 0: by the number of qubits
   bool windows_only = false;  // every pass a window pass (the batched kernel runs only those)
   // Adjoint sweeps: when set, no gates are merged and the op made from
   // gates[i] carries param_of[i] / generator_of[i] (Op::param, Op::generator).
@@ -489,14 +490,24 @@ void release_adjoint(dmv_state_s* s);
 int ensure_pinned(dmv_state_s* s, size_t bytes);
 
 // Planner settings for a state: tiles of 2^12 amplitudes (the TMA window
-// kernel's register phases hold 8 per thread of 512).
-inline PlanOptions plan_options_for(const dmv_state_s* s, int32_t fusion) {
-  (void)s;
+// kernel's register phases hold 8 per thread of 512). `sweep`: a gradient's.
+//
+// On the tensor cores a pass's cost is the digit split and recombination of the
+// state at every size, so the search counts it as on large states. Up to 16
+// qubits it has little to choose from and the first targets met do as well: on
+// random circuits of 13 to 16 qubits the search takes 1.07 of their time with a
+// pass at 8 and 1.01 at 32, on ladders and rings as long; at 17 to 19 qubits
+// and 32 it takes 0.97 and 0.93.
+inline PlanOptions plan_options_for(const dmv_state_s* s, int32_t fusion, bool sweep = false) {
   PlanOptions opt;
   opt.fusion = fusion;
   opt.tile_bits = 12;
   opt.low_bits = 4;  // a 128-byte row of complex64, two of complex128
   opt.search_windows = true;
+  if (!sweep && s->precision == DMV_C128 && s->arith == ARITH_TC) {
+    opt.search_windows = s->n > 16;
+    opt.pass_cost = 32.0;
+  }
   return opt;
 }
 

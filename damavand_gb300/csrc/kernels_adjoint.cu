@@ -512,7 +512,7 @@ int adjoint_sweep_fix(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, const 
     slot.push_back(p ? slots : -1);
     gen.push_back(p ? rotation_generator(g.kind) : 0);
   }
-  PlanOptions opt = plan_options_for(s, DMV_FUSE_WINDOW);
+  PlanOptions opt = plan_options_for(s, DMV_FUSE_WINDOW, true);
   opt.tile_bits = kAdjBits;
   opt.windows_only = true;
   std::vector<int32_t> run_of;

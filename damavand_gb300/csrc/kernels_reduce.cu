@@ -1565,7 +1565,7 @@ int launch_adjoint_step_impl(dmv_state_s* psi, dmv_state_s* lam, const Op& op, i
 int adjoint_sweep_windows(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, const std::vector<Gate>& gates,
                           double* part, int64_t cols, DeviceBuffer& ops_buf) {
   Plan plan;
-  DMV_TRY(build_adjoint_plan(gates, s->n, s->precision, plan_options_for(s, DMV_FUSE_WINDOW), plan));
+  DMV_TRY(build_adjoint_plan(gates, s->n, s->precision, plan_options_for(s, DMV_FUSE_WINDOW, true), plan));
   if (!plan.ops.empty()) {
     DMV_TRY(ops_buf.reserve(plan.ops.size() * sizeof(Op)));
     DMV_CUDA_TRY(cudaMemcpyAsync(ops_buf.ptr, plan.ops.data(), plan.ops.size() * sizeof(Op), cudaMemcpyHostToDevice,
