@@ -235,7 +235,7 @@ constexpr double kPassCost = 32.0, kPassCostFewTiles = 8.0;
 constexpr int32_t kFewTilesQubits = 20;
 
 Window next_window(const std::vector<SGate>& sg, const std::vector<int64_t>& pending, int32_t n, int32_t k,
-                   int32_t low, bool search, double pass_cost) {
+                   int32_t low, bool search) {
   Window first;
   first.local = (uint64_t(1) << low) - 1;
   first.max_depth = INT32_MAX;
@@ -249,7 +249,7 @@ Window next_window(const std::vector<SGate>& sg, const std::vector<int64_t>& pen
     if (!(first.local & qbit(q))) { first.local |= qbit(q); ++nlocal; }
   if (!search || k >= n) return first;
 
-  if (pass_cost <= 0.0) pass_cost = n < kFewTilesQubits ? kPassCostFewTiles : kPassCost;
+  const double pass_cost = n < kFewTilesQubits ? kPassCostFewTiles : kPassCost;
   Window best = first;
   double best_score = -1.0;
   std::vector<int32_t> work, moves;  // non-exchange and exchange gates taken, per depth
@@ -372,7 +372,7 @@ int build_plan(const std::vector<Gate>& gates, int32_t n, int32_t precision,
                        classify(g.m) == OP_SWAP});
   std::vector<int64_t> keep, take;
   while (!pending.empty()) {
-    const Window win = next_window(sg, pending, n, k, low, opt.search_windows, opt.pass_cost);
+    const Window win = next_window(sg, pending, n, k, low, opt.search_windows);
     const uint64_t local = win.local;
 
     keep.clear();

@@ -275,7 +275,6 @@ struct PlanOptions {
   int32_t tile_bits = 12;  // log2 amplitudes per tile
   int32_t low_bits = 6;    // always-local low qubits (coalesced chunks)
   bool search_windows = false;  // choose each window by a search (next_window) instead of the first targets met
-  double pass_cost = 0.0;       // next_window's cost of a pass, 0: by the number of qubits
   bool windows_only = false;  // every pass a window pass (the batched kernel runs only those)
   // Adjoint sweeps: when set, no gates are merged and the op made from
   // gates[i] carries param_of[i] / generator_of[i] (Op::param, Op::generator).
@@ -489,24 +488,31 @@ constexpr size_t kKeepAdjointBytes = size_t(64) << 20;
 void release_adjoint(dmv_state_s* s);
 int ensure_pinned(dmv_state_s* s, size_t bytes);
 
+constexpr int32_t kSearchQubits = 20;
 // Planner settings for a state: tiles of 2^12 amplitudes (the TMA window
 // kernel's register phases hold 8 per thread of 512). `sweep`: a gradient's.
 //
+// complex64 passes are rewritten (rotations, phase tables) from kSearchQubits
+// qubits on. Below, the passes of a few states overlap and the host's time per
+// forward shows, which the search and the rewrite raise (17 qubits, 1290 gates:
+// 289 us): three states in turn take 189 us per forward without and 316 with
+// them at that size, 230 and 289 at 19 qubits and 15 layers, 31 and 66 at 13
+// and 15, although one state alone gains (537 and 289 us at 17 qubits). Above,
+// the device's time decides: 763 and 405 us at 21 qubits and 16 layers.
+//
 // On the tensor cores a pass's cost is the digit split and recombination of the
-// state at every size, so the search counts it as on large states. Up to 16
-// qubits it has little to choose from and the first targets met do as well: on
-// random circuits of 13 to 16 qubits the search takes 1.07 of their time with a
-// pass at 8 and 1.01 at 32, on ladders and rings as long; at 17 to 19 qubits
-// and 32 it takes 0.97 and 0.93.
+// state. Below 20 qubits the search has little to choose from: at 13 to 19 it
+// takes 0.98 of the time of the first targets met on ladders and rings but 1.03
+// on random circuits, 1.25 at worst; at 20 to 23 qubits 0.88 and 0.97.
 inline PlanOptions plan_options_for(const dmv_state_s* s, int32_t fusion, bool sweep = false) {
   PlanOptions opt;
   opt.fusion = fusion;
   opt.tile_bits = 12;
   opt.low_bits = 4;  // a 128-byte row of complex64, two of complex128
   opt.search_windows = true;
-  if (!sweep && s->precision == DMV_C128 && s->arith == ARITH_TC) {
-    opt.search_windows = s->n > 16;
-    opt.pass_cost = 32.0;
+  if (!sweep && s->n < kSearchQubits && (s->precision == DMV_C64 || s->arith == ARITH_TC)) {
+    opt.search_windows = false;
+    opt.low_bits = 6;  // rows of 512 and 1024 bytes
   }
   return opt;
 }

@@ -879,7 +879,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   const bool c128 = s->precision == DMV_C128;
   const bool rewrite = c128 && ((s->arith == ARITH_FP64 && s->fp64_rewrite) || s->arith == ARITH_FP32X2 ||
                                 s->arith == ARITH_INT64);
-  const bool single = !c128 && s->n >= 12;  // complex64 passes as rotations and tables
+  const bool single = !c128 && s->n >= kSearchQubits;  // complex64 passes as rotations and tables
   const bool rot_ops = single || s->arith == ARITH_FP64;
   const bool fix = rewrite && s->arith != ARITH_INT64 && s->n >= 12;  // fixed-point passes where the kernel takes them
   s->phase_tabs = PhaseTables();

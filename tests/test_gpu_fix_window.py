@@ -114,7 +114,7 @@ def test_pair_states_off_the_integers(built_lib, oracle_mod, start):
 
 
 @pytest.mark.parametrize("shape", ["ladder", "ring", "random"])
-@pytest.mark.parametrize("n", [12, 13, 17])
+@pytest.mark.parametrize("n", [12, 13, 17, 20, 21])
 def test_complex64_shapes(built_lib, oracle_mod, n, shape):
     """The complex64 passes on the same shapes; each output is rounded to 2^-24 of itself, the
     rotations' and tables' entries likewise."""
