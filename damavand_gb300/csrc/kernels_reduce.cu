@@ -598,6 +598,14 @@ __global__ void k_reduce_rows(const double* __restrict__ in, int64_t rows, int c
 // single CTA with 1024 serial additions (57 us already at 20 qubits, where one
 // CTA is all there is). k_scan_totals gives each CTA's total, and every CTA
 // adds up the ones before its own.
+//
+// The samplers search these prefixes, so they must not decrease and a chunk of
+// no mass must repeat its predecessor's, although sums of different shapes
+// round differently. So a border is one number for both its sides. Between
+// CTAs it is the sum of the totals before it, always in the same shape: more
+// terms of it nonnegative, none of it smaller. Between threads it is the
+// largest of the nonempty threads' prefixes up to there, and a thread's own
+// chunks stay between its two borders.
 constexpr int kScanThreads = 1024;
 constexpr int kScanEach = 4;
 constexpr int kScanBlock = kScanThreads * kScanEach;
@@ -623,23 +631,46 @@ k_scan_totals(const double* __restrict__ mass, int64_t num_chunks, double* __res
   }
 }
 
+// Prefixes are compared by their bits: at least 0, they order as integers, a
+// NaN above all, and the FP64 pipe is left out of it.
+__device__ __forceinline__ bool scan_less(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ double scan_max(double a, double b) { return scan_less(a, b) ? b : a; }
+__device__ __forceinline__ bool scan_some(double mass) { return (__double_as_longlong(mass) << 1) != 0; }
+
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_chunks(const double* __restrict__ mass, int64_t num_chunks, const double* __restrict__ totals,
               double* __restrict__ incl) {
-  __shared__ double red[32], before[32];
+  __shared__ double red[32], low[32], high[32], top[32], border[2];
+  __shared__ int last[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double prior = 0.;
-  for (int c = threadIdx.x; c < (int)blockIdx.x; c += kScanThreads) prior += totals[c];
-  prior = warp_sum_f64(prior);
+  // the CTA's two borders; warps without a total skip the sums
+  double below = 0., above = 0.;
+  if (gridDim.x > 1 && warp * 32 <= (int)blockIdx.x) {
+    for (int c = threadIdx.x; c <= (int)blockIdx.x; c += kScanThreads) {
+      const double t = totals[c];
+      if (c < (int)blockIdx.x) below += t;
+      above += t;
+    }
+    below = warp_sum_f64(below);
+    above = warp_sum_f64(above);
+  }
   double m[kScanEach];
   double s = scan_load(mass, num_chunks, m);
+  const bool some = scan_some(s);
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const double up = __shfl_up_sync(0xffffffffu, s, o);
     if (lane >= o) s += up;
   }
+  const unsigned full = __ballot_sync(0xffffffffu, some);
   if (lane == 31) red[warp] = s;
-  if (lane == 0) before[warp] = prior;
+  if (lane == 0) {
+    low[warp] = below;
+    high[warp] = above;
+    last[warp] = full ? 31 - __clz((int)full) : -1;
+  }
   __syncthreads();
   if (warp == 0) {
     double t = red[lane];
@@ -648,20 +679,54 @@ k_scan_chunks(const double* __restrict__ mass, int64_t num_chunks, const double*
       const double up = __shfl_up_sync(0xffffffffu, t, o);
       if (lane >= o) t += up;
     }
-    // everything before this warp: the warps before it and the CTAs before this one
-    double excl = __shfl_up_sync(0xffffffffu, t, 1);
-    if (lane == 0) excl = 0.;
-    const double p = warp_sum_f64(before[lane]);
-    red[lane] = p + excl;
+    red[lane] = t;  // (this warp reads its own word only)
+    if (gridDim.x > 1) {
+      below = warp_sum_f64(low[lane]);
+      above = warp_sum_f64(high[lane]);
+    }
+    if (lane == 0) {
+      border[0] = below;
+      border[1] = above;
+    }
   }
   __syncthreads();
-  double prev = __shfl_up_sync(0xffffffffu, s, 1);
-  if (lane == 0) prev = 0.;
-  double run = red[warp] + prev;
+  below = border[0];
+  above = border[1];
+  const double before = warp > 0 ? red[warp - 1] : 0.;
+  const unsigned warps = __ballot_sync(0xffffffffu, last[lane] >= 0);  // the warps with mass
+  // this thread's upper border: its prefix, or `above` where no mass follows in the CTA
+  double upper = below;
+  if (some) {
+    upper = scan_max(below, below + (before + s));
+    if (gridDim.x > 1) {
+      if (scan_less(above, upper)) upper = above;
+      if (31 - __clz((int)warps) == warp && last[warp] == lane) upper = above;
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double up = __shfl_up_sync(0xffffffffu, upper, o);
+    if (lane >= o) upper = scan_max(up, upper);
+  }
+  if (lane == 31) top[warp] = upper;
+  __syncthreads();
+  double floor_w = lane < warp ? top[lane] : below;  // the warp's lower border
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) floor_w = scan_max(floor_w, __shfl_xor_sync(0xffffffffu, floor_w, o));
+  double lower = __shfl_up_sync(0xffffffffu, upper, 1);
+  lower = lane == 0 ? floor_w : scan_max(floor_w, lower);
+  upper = scan_max(floor_w, upper);
   const int64_t b = (int64_t)blockIdx.x * kScanBlock + (int64_t)threadIdx.x * kScanEach;
+  double run = lower;
 #pragma unroll
   for (int j = 0; j < kScanEach; ++j) {
-    run += m[j];
+    bool more = false;  // mass in a later chunk of the thread
+#pragma unroll
+    for (int i = j + 1; i < kScanEach; ++i) more = more || scan_some(m[i]);
+    if (scan_some(m[j])) {
+      run += m[j];
+      if (!more || scan_less(upper, run)) run = upper;
+    }
     if (b + j < num_chunks) incl[b + j] = run;
   }
 }
@@ -774,9 +839,10 @@ __global__ void k_chunk_guide(const double* __restrict__ incl, int64_t num_chunk
 // prefix levels: the chunk by binary search on the chunk prefixes, the segment
 // by a ballot over the chunk's segment prefixes, the element by a scan of the
 // segment (lane sums, a shuffle scan, then each lane's own elements in order).
-// Where rounding between the levels leaves no element of the chosen segment
-// reaching u*total, the segment's last element of nonzero probability is taken
-// (the chosen segment has nonzero mass, so one exists).
+// The levels' sums round differently. Where no segment of the chunk reaches
+// u*total, the last one of nonzero mass is taken (the chunk has some: its prefix
+// is above its predecessor's); where no element of nonzero probability of the
+// segment does, the last such element.
 template <int SRC>
 __global__ void __launch_bounds__(kRedThreads)
 k_sample_warp(const void* src, int seg_bits, int chunk_bits, int64_t num_chunks, const double* __restrict__ chunk_incl,
@@ -810,8 +876,11 @@ k_sample_warp(const void* src, int seg_bits, int chunk_bits, int64_t num_chunks,
     }
     const double before = lo > 0 ? chunk_incl[lo - 1] : 0.;
     const double* sp = seg_incl + lo * spc;
-    const unsigned segs = __ballot_sync(0xffffffffu, lane < spc && xsi <= before + sp[lane < spc ? lane : 0]);
-    const int sg = segs ? __ffs((int)segs) - 1 : spc - 1;
+    const double mine_sp = sp[lane < spc ? lane : 0];
+    const double prev_sp = __shfl_up_sync(0xffffffffu, mine_sp, 1);
+    const unsigned segs = __ballot_sync(0xffffffffu, lane < spc && xsi <= before + mine_sp);
+    const unsigned some = __ballot_sync(0xffffffffu, lane < spc && mine_sp > (lane > 0 ? prev_sp : 0.));
+    const int sg = segs ? __ffs((int)segs) - 1 : some ? 31 - __clz((int)some) : spc - 1;
     const double sbefore = sg > 0 ? before + sp[sg - 1] : before;
     const int64_t base = ((lo * spc + sg) << seg_bits) + (int64_t)lane * E;
     const int mine = lane * E < S ? E : 0;
@@ -836,7 +905,7 @@ k_sample_warp(const void* src, int seg_bits, int chunk_bits, int64_t num_chunks,
       if (e < mine) {
         run += p[e];
         if (p[e] > 0.) last_nz = e;
-        if (hit < 0 && xsi <= run) hit = e;
+        if (hit < 0 && p[e] > 0. && xsi <= run) hit = e;
       }
     }
     const unsigned hits = __ballot_sync(0xffffffffu, hit >= 0);
