@@ -62,6 +62,14 @@ constexpr size_t kAdjSmem = ((size_t)2 << kAdjBits) * 16 + kAdjStage + (size_t)k
 // unit is 2^-44 of a product, and a gradient is no larger than the rounding of
 // a sum of that many terms (dropping it left 7.5e-14 of the 22-qubit gradient
 // where FP64 leaves 8e-15).
+//
+// How large it gets. A phase starts with components below 2^58 (fix_renorm), and
+// the stored norm at most doubles until the next (`grown` from 1/sqrt 2 to
+// sqrt 2). So over a thread's 16 components of each state the sum is at most
+// 16 2^116 4 / 2^64 = 2^58, and over a tile's 2^12 it is 2^66, which 64 bits do
+// not hold: what leaves the thread is in units of 2^(64 + kGradShift), at most
+// 2^62 over the tile.
+constexpr int kGradShift = 4;
 struct FixSum {
   long long h;
   unsigned f;
@@ -265,8 +273,10 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
           }
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            const long long h = warp_sum(g[c].h);
-            const unsigned f = __reduce_add_sync(0xffffffffu, g[c].f >> 5);  // f < 8 x 2^26
+            const long long h = warp_sum(g[c].h >> kGradShift);
+            // units of 2^-26 of g.h: f < 8 x 2^26, so the sum is below 2^31
+            const unsigned fr = g[c].f + (((unsigned)g[c].h & ((1u << kGradShift) - 1u)) << 26);
+            const unsigned f = __reduce_add_sync(0xffffffffu, fr >> 5);
             if (lane == 0) {
               const int at_w = (w0.z * 3 + c) * kAdjWarps + warp;
               s_acc[at_w] = h;
@@ -361,7 +371,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
           double f;
           memcpy(&f, &op->a[3], sizeof(f));
           // product of two fixed-point values / 2^64 -> product of the amplitudes
-          const int e = ea + eb - 2 * 1079 + 64 + s_exp[op->a[1]];
+          const int e = ea + eb - 2 * 1079 + 64 + kGradShift + s_exp[op->a[1]];
           for (int c = 0; c < 3; ++c) {
             const int i = op->a[1] * 3 + c;
             long long h = 0, r = 0;
@@ -370,7 +380,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adjoint_fix(const __grid_con
               h += s_acc[i * kAdjWarps + w];
               r += s_frac[i * kAdjWarps + w];
             }
-            s_sum[i] += scalbn(fma((double)r, 0x1p-21, (double)h) * f, e);
+            s_sum[i] += scalbn(fma((double)r, 0x1p-25, (double)h) * f, e);
           }
         }
         const int ep = ea - 1079 + p.shifts + na + 1075 + p.scale_exp, el = eb - 1079 + p.shifts + nb + 1075 + p.scale_exp;
