@@ -55,30 +55,28 @@ __device__ __forceinline__ long long fix_wide(int a, int b) {
 }
 
 // x m / 2^64 = high + low for |x| < 2^62 and the multiplier m = mh 2^32 + ml
-// (0 <= mh < 2^31, ml signed). x's low word is taken as signed too, so low
-// stays within 2^30 + 2^29; the two truncated middle products average to the
-// 1 that is added. Three bare products: with the sums inside the 64-bit
-// multiply-adds a rotation took 24 cycles per warp output and SM quarter, so
-// 20; volatile keeps the compiler from hoisting products of other pairs,
-// which spills (23 without it).
+// (0 <= mh < 2^31, ml signed). x's low word is taken as signed too, so the sum
+// of the middle products stays below 2^62 + 2^61 and low within 2^30 + 2^29. It
+// is rounded once, so 0 times anything, and anything times 0, is exactly 0: two
+// truncated products with the mean of their errors added as a constant left +-1
+// in the place of amplitudes that a circuit keeps at zero, and took longer (28
+// qubits: 328 ms, 315 so). The high product stays bare: with all three in one
+// chain of 64-bit multiply-adds a rotation took 24 cycles per warp output and
+// SM quarter, against 20 for the truncated products. volatile keeps the
+// compiler from hoisting products of other pairs, which spills.
 __device__ __forceinline__ void fix_mul(long long x, int mh, int ml, long long& high, int& low) {
   const int xl = (int)x, xh = (int)(x >> 32) + (int)((unsigned)xl >> 31);
-  int q1, q2;
-  asm volatile("mul.hi.s32 %0, %1, %2;" : "=r"(q1) : "r"(xl), "r"(mh));
-  asm volatile("mul.hi.s32 %0, %1, %2;" : "=r"(q2) : "r"(xh), "r"(ml));
+  long long mid;
+  asm volatile("mul.wide.s32 %0, %1, %2;" : "=l"(mid) : "r"(xl), "r"(mh));
+  asm volatile("mad.wide.s32 %0, %1, %2, %0;" : "+l"(mid) : "r"(xh), "r"(ml));
   asm volatile("mul.wide.s32 %0, %1, %2;" : "=l"(high) : "r"(xh), "r"(mh));
-  low = q1 + q2 + 1;
+  low = (int)(mid >> 32) + (int)((unsigned)mid >> 31);
 }
 
-// x + q and x - q for a 32-bit q.
+// x + q for a 32-bit q.
 __device__ __forceinline__ long long fix_add(long long x, int q) {
   unsigned l = (unsigned)x, h = (unsigned)(x >> 32);
   asm("{add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;}" : "+r"(l), "+r"(h) : "r"(q), "r"(q >> 31));
-  return (long long)((unsigned long long)h << 32 | l);
-}
-__device__ __forceinline__ long long fix_sub(long long x, int q) {
-  unsigned l = (unsigned)x, h = (unsigned)(x >> 32);
-  asm("{sub.cc.u32 %0, %0, %2;\n\tsubc.u32 %1, %1, %3;}" : "+r"(l), "+r"(h) : "r"(q), "r"(q >> 31));
   return (long long)((unsigned long long)h << 32 | l);
 }
 
@@ -126,11 +124,11 @@ __device__ __forceinline__ void fix_rot(long long (&r)[2 * NA], int mh, int ml) 
       fix_mul(x0, mh, ml, h0, q0);
       fix_mul(x1, mh, ml, h1, q1);
       if constexpr (COMP) {
-        a = fix_add(x0 - x1 + h1, q1);
-        b = fix_sub(x1 + x0 - h0, q0);
+        a = x0 - x1 + h1 + (long long)q1;
+        b = x1 + x0 - h0 - (long long)q0;
       } else {
-        a = fix_sub(x0 - h1, q1);
-        b = fix_add(x1 + h0, q0);
+        a = x0 - h1 - (long long)q1;
+        b = x1 + h0 + (long long)q0;
       }
     }
   }
