@@ -153,7 +153,7 @@ k_batch_fix(double2* __restrict__ arena, const BatchPass* __restrict__ passes, c
   __shared__ long long s_item;
   __shared__ int s_stop;
   __shared__ int64_t s_slot[kFixAmps];
-  __shared__ uint32_t s_scan[4][NT / 32];
+  __shared__ uint32_t s_scan[5][NT / 32];
   __shared__ int s_top[3];
   const int tid = (int)threadIdx.x;
   longlong2* ti = reinterpret_cast<longlong2*>(smem_raw);
@@ -219,7 +219,7 @@ k_batch_fix(double2* __restrict__ arena, const BatchPass* __restrict__ passes, c
         r[2 * u + 1] = v.y;
       }
       const FixScan scan = fix_scan(r, s_scan);
-      if (num_fix > 0 && scan.fixed(ps.sparse)) {
+      if (num_fix > 0 && scan.fixed(ps.sparse) && scan.heavy()) {
         fix_put(r, smem_raw, scan.emax());
         const int renorm = fix_run(r, smem_raw, stage, fops, num_fix, fix_tab, base, s_top);
         const int e = scan.emax() - 1079 + ps.shifts + renorm + 1075 + ps.out_exp;

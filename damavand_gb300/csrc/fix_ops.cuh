@@ -194,6 +194,7 @@ constexpr size_t kFixStage = (size_t)8 * kFixThreads * 16;  // table entries on 
 // What decides how a tile runs.
 struct FixScan {
   uint32_t mx, mn, any, cnt;  // largest and smallest nonzero amplitude (top words), low words, nonzero amplitudes
+  uint32_t mass;              // sum of the squares of the amplitudes' larger components, in 2^-18 M^2 (fixed)
   __device__ int emax() const { return (int)(mx >> 20); }
   __device__ bool zero() const { return mx == 0 && any == 0; }
   // In range, with no more than the pass's (`sparse`) numbers of unreached
@@ -202,9 +203,20 @@ struct FixScan {
     const int unreached = 12 - (31 - __clz((int)cnt | 1));
     return emax() - (int)(mn >> 20) <= kFixRange && emax() > 200 && emax() < 1800 && ((sparse >> unreached) & 1u);
   }
+  // Whether the amplitudes outweigh the rounding of the fixed point. With
+  // u = 2^-57 M, M the power of two above the largest component, a rotation
+  // leaves an error of variance 0.09 u^2 in a component (the rounding of one
+  // product and the part of it that is left out) and a table 0.3 u^2; in FP64
+  // it is 0.045 and 0.06 times 2^-104 x^2 in a component x. At three or four
+  // rotations to a table the two are even where the squares of 2^13 components
+  // add up to 22 M^2, or 16 M^2 over each amplitude's larger one, which is the
+  // line, in proportion to the nonzero amplitudes: zeros round to zero. Dense
+  // random tiles have 100 to 400 M^2, one that a single amplitude dominates 1
+  // to 2: 360 small rotations left 2.5e-15 of such a tile, in FP64 3.8e-16.
+  __device__ bool heavy() const { return mass >= ((16u << 18) >> 12) * cnt; }
 };
 
-// Over the CTA, of amplitudes raw (double bits); s: 4 x 8 words of shared memory.
+// Over the CTA, of amplitudes raw (double bits); s: 5 x 8 words of shared memory.
 __device__ __forceinline__ FixScan fix_scan(const long long (&raw)[2 * kFixAmps], uint32_t (*s)[kFixThreads / 32]) {
   uint32_t mx = 0, mn = ~0u, any = 0, cnt = 0;
 #pragma unroll
@@ -222,12 +234,23 @@ __device__ __forceinline__ FixScan fix_scan(const long long (&raw)[2 * kFixAmps]
   mn = __reduce_min_sync(0xffffffffu, mn);
   any = __reduce_or_sync(0xffffffffu, any);
   cnt = __reduce_add_sync(0xffffffffu, cnt);
+  // the squares, in units of the warp's largest exponent: floats in [0, 2)
+  float q = 0.f;
+  const int unit = ((int)(mx >> 20) - 127) << 20;
+#pragma unroll
+  for (int u = 0; u < kFixAmps; ++u) {
+    const int h = max((int)(raw[2 * u] >> 32) & 0x7FFFFFFF, (int)(raw[2 * u + 1] >> 32) & 0x7FFFFFFF);
+    const float f = __int_as_float(max(h - unit, 0) << 3);
+    q = fmaf(f, f, q);
+  }
+  uint32_t mass = __reduce_add_sync(0xffffffffu, (uint32_t)(q * 65536.f));  // 2^9 2^2 2^16 at most
   if ((threadIdx.x & 31) == 0) {
     const int w = (int)threadIdx.x >> 5;
     s[0][w] = mx;
     s[1][w] = mn;
     s[2][w] = any;
     s[3][w] = cnt;
+    s[4][w] = mass;
   }
   __syncthreads();
   cnt = 0;
@@ -238,7 +261,10 @@ __device__ __forceinline__ FixScan fix_scan(const long long (&raw)[2 * kFixAmps]
     any |= s[2][w];
     cnt += s[3][w];
   }
-  return FixScan{mx, mn, any, cnt};
+  mass = 0;
+#pragma unroll
+  for (int w = 0; w < kFixThreads / 32; ++w) mass += s[4][w] >> min(2 * ((mx >> 20) - (s[0][w] >> 20)), 31u);
+  return FixScan{mx, mn, any, cnt, mass};
 }
 
 // The tile's amplitudes (thread tid holds tid + 256 u) into its slots as integers.

@@ -6,14 +6,16 @@
 // amplitudes is turned into integers under one exponent: the largest
 // component gets 57 bits, and a rotation output x0 - w x1 (the same f M form
 // as OP_ROT) is three integer multiply-adds and one rounding to the last bit,
-// 2^-57 of the tile's largest component: less than FP64 rounds a component of
-// the tile's average size by. The ops run in register phases (build_fix_pass):
+// 2^-57 of the tile's largest component: in the norm of the tile, as long as it
+// is no more than a few times its average (FixScan::heavy), less than FP64's
+// roundings. The ops run in register phases (build_fix_pass):
 // 256 threads hold 16 amplitudes each, the tile crosses shared memory once per
 // phase, exchanges cost nothing (they re-index the tile).
 //
 // Which tiles. Fixed point keeps less of a component the smaller it is, so a
 // tile runs in it only when every amplitude is within 2^kFixRange of its
-// largest one (entangled states: all but one tile in a few hundred). Any
+// largest one (entangled states: all but one tile in a few hundred) and their
+// squares are not those of a few (FixScan::heavy). Any
 // other tile (product states, exact zeros, infinities, NaN) takes the pass's
 // ops in shared memory in the arithmetic FB (FP64, or FP32 pairs for states of
 // that arithmetic). A tile of zeros is left as it is.
@@ -43,7 +45,7 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
   constexpr int NT = kFixThreads;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_scan[4][NT / 32];
+  __shared__ uint32_t s_scan[5][NT / 32];
   __shared__ int s_high[16];
   __shared__ int64_t s_slot[kFixAmps];
   __shared__ int s_top[3];  // largest component, by phase
@@ -111,7 +113,9 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
     }
     const FixScan scan = fix_scan(r, s_scan);
     const int emax = scan.emax();
-    const bool zero = scan.zero(), fixed = scan.fixed(fp.sparse);
+    const bool zero = scan.zero();
+    // FP32 pairs round more coarsely than any fixed-point tile
+    const bool fixed = scan.fixed(fp.sparse) && (!std::is_same<FB, PolF64>::value || scan.heavy());
     int e_out = 0;
     const bool store = !zero;
     if (fixed) {
