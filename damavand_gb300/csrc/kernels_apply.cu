@@ -1175,6 +1175,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   s->last_ops = (int64_t)plan.ops.size();
   s->last_phase_tab_bytes = tab_bytes;
   s->last_upload_bytes = s->last_phase_tab_bytes + (any_window ? (int64_t)(ops.size() * sizeof(Op)) : 0) +
+                         (int64_t)(s->fix_ops.size() * sizeof(FixOp)) +
                          (any_phases ? (int64_t)(s->phase_ops.size() * sizeof(PhaseOp)) : 0) +
                          (tc ? (int64_t)(s->tc_stages.size() * sizeof(TcStage) + s->tc_u.size() * 2) : 0);
   s->last_bytes = bytes;
