@@ -863,7 +863,8 @@ int make_phase_tables(const PhaseTables& tabs, const std::vector<FixOp>& fix_ops
 // leaves out.
 constexpr double kPairScale = 0x1p-40;
 
-int launch_plan(dmv_state_s* s, const Plan& plan) {
+// `rewritten_form` false: every fused 2x2 as it is, no phase tables.
+int launch_plan_form(dmv_state_s* s, const Plan& plan, bool rewritten_form) {
   // The launches: every pass, except that a register-phase pass with more
   // ops than the kernel's op table holds runs as several launches over the
   // same qubits. Ops are copied so the phase scheduler may reorder them.
@@ -877,9 +878,10 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
   // The FP32-pair and int64 arithmetics take the same rewrite with the rotations
   // as real 2x2 ops and the tables in their own forms.
   const bool c128 = s->precision == DMV_C128;
-  const bool rewrite = c128 && ((s->arith == ARITH_FP64 && s->fp64_rewrite) || s->arith == ARITH_FP32X2 ||
-                                s->arith == ARITH_INT64);
-  const bool single = !c128 && s->n >= kSearchQubits;  // complex64 passes as rotations and tables
+  const bool rewrite = rewritten_form && c128 &&
+                       ((s->arith == ARITH_FP64 && s->fp64_rewrite) || s->arith == ARITH_FP32X2 ||
+                        s->arith == ARITH_INT64);
+  const bool single = rewritten_form && !c128 && s->n >= kSearchQubits;  // complex64 passes as rotations and tables
   const bool rot_ops = single || s->arith == ARITH_FP64;
   const bool fix = rewrite && s->arith != ARITH_INT64 && s->n >= 12;  // fixed-point passes where the kernel takes them
   s->phase_tabs = PhaseTables();
@@ -934,7 +936,7 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
       PhaseTables& all = s->phase_tabs;
       const int64_t tab_base = all.entries;
       if (tab_base + r.tab.entries > INT32_MAX)
-        return set_error(DMV_ERR_UNSUPPORTED, "gate list: too many phase tables for one call");
+        return set_error(DMV_ERR_OOM, "gate list: too many phase tables for one call");
       for (Op op : r.ops) {
         if (op.cls == OP_PHASE) op.fh[0] += (int32_t)tab_base;
         ops.push_back(op);
@@ -1180,6 +1182,17 @@ int launch_plan(dmv_state_s* s, const Plan& plan) {
                          (tc ? (int64_t)(s->tc_stages.size() * sizeof(TcStage) + s->tc_u.size() * 2) : 0);
   s->last_bytes = bytes;
   return DMV_OK;
+}
+
+// Where there is no room for the rewritten passes' tables and ops (all of it is
+// reserved before the first launch), the gates run as they are.
+int launch_plan(dmv_state_s* s, const Plan& plan) {
+  const int rc = launch_plan_form(s, plan, true);
+  if (rc != DMV_ERR_OOM) return rc;
+  clear_error();
+  for (DeviceBuffer* b : {&s->phase_tab_dev, &s->phase_tab2_dev, &s->phase_tab_fix_dev, &s->fix_ops_dev, &s->phase_src_dev})
+    b->release();
+  return launch_plan_form(s, plan, false);
 }
 
 // The state times a real factor: the product of the FP64 rotations' factors
