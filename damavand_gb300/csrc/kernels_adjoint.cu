@@ -499,8 +499,9 @@ struct AdjGrad {
 }  // namespace
 
 // The reverse sweep (see the file comment) from psi and lam, which it uses up.
-// *done is false, and nothing ran, for gate lists it does not take: controls
-// other than CNOT's, non-unitary matrices.
+// *done is false, and nothing ran, for gate lists it does not take (controls
+// other than CNOT's, non-unitary matrices) and where its ops and tables, all
+// reserved before the first launch, find no memory.
 int adjoint_sweep_fix(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, const std::vector<Gate>& gates, double* grads,
                       bool* done) {
   *done = false;
@@ -605,6 +606,10 @@ int adjoint_sweep_fix(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, const 
   std::vector<double> sums(rows);
   do {
     if ((rc = work.reserve(ops_bytes + fops_bytes + part_bytes + out_bytes)) != DMV_OK) break;
+    if (tabs.entries > 0) {
+      if ((rc = tab.reserve((size_t)tabs.entries * 16)) != DMV_OK) break;
+      if ((rc = fix_tab.reserve((size_t)tabs.entries * 16)) != DMV_OK) break;
+    }
     char* wp = static_cast<char*>(work.ptr);
     double* part = reinterpret_cast<double*>(wp + ops_bytes + fops_bytes);
     double* out = reinterpret_cast<double*>(wp + ops_bytes + fops_bytes + part_bytes);
@@ -614,8 +619,6 @@ int adjoint_sweep_fix(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, const 
       break;
     }
     if (tabs.entries > 0) {
-      if ((rc = tab.reserve((size_t)tabs.entries * 16)) != DMV_OK) break;
-      if ((rc = fix_tab.reserve((size_t)tabs.entries * 16)) != DMV_OK) break;
       PhaseTableForms forms;
       forms.f64 = static_cast<double2*>(tab.ptr);
       forms.fix = static_cast<longlong2*>(fix_tab.ptr);
@@ -654,6 +657,11 @@ int adjoint_sweep_fix(dmv_state_s* s, dmv_state_s* psi, dmv_state_s* lam, const 
     }
     if (cudaStreamSynchronize(s->stream) != cudaSuccess) rc = set_error(DMV_ERR_CUDA, "adjoint sweep failed");
   } while (false);
+  if (rc == DMV_ERR_OOM) {
+    clear_error();
+    for (DeviceBuffer* b : {&src, &work, &tab, &fix_tab}) b->release();
+    return DMV_OK;
+  }
   DMV_TRY(rc);
 
   // The parameters of each run from its three sums.

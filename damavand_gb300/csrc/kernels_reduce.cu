@@ -1708,14 +1708,6 @@ int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const doubl
   // Columns of the per-parameter partials: the widest grid of the sweep's kernels.
   const int grid = std::max(adjoint_grid(pairs_u), adjoint_window_grid(int64_t(1) << std::max(0, s->n - 12)));
   do {
-    rc = partial.reserve((size_t)num_params * grid * sizeof(double) + (size_t)num_params * sizeof(double));
-    if (rc != DMV_OK) break;
-    double* part = static_cast<double*>(partial.ptr);
-    double* out = part + (size_t)num_params * grid;
-    if (cudaMemsetAsync(part, 0, (size_t)num_params * grid * sizeof(double), s->stream) != cudaSuccess) {
-      rc = set_error(DMV_ERR_CUDA, "memset of gradient partials failed");
-      break;
-    }
     if (cudaMemcpyAsync(psi->amps, s->amps, s->amp_bytes(), cudaMemcpyDeviceToDevice, s->stream) != cudaSuccess) {
       rc = set_error(DMV_ERR_CUDA, "statevector copy failed");
       break;
@@ -1726,6 +1718,14 @@ int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const doubl
       bool swept = false;
       rc = adjoint_sweep_fix(s, psi, lam, gates, grads, &swept);
       if (rc != DMV_OK || swept) break;
+    }
+    rc = partial.reserve((size_t)num_params * grid * sizeof(double) + (size_t)num_params * sizeof(double));
+    if (rc != DMV_OK) break;
+    double* part = static_cast<double*>(partial.ptr);
+    double* out = part + (size_t)num_params * grid;
+    if (cudaMemsetAsync(part, 0, (size_t)num_params * grid * sizeof(double), s->stream) != cudaSuccess) {
+      rc = set_error(DMV_ERR_CUDA, "memset of gradient partials failed");
+      break;
     }
     // FP32-pair arithmetic: psi and lam are scratch, so they take the pair form
     // once and keep it for the whole sweep.
