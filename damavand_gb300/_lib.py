@@ -97,6 +97,7 @@ SIGNATURES = {
     "dmv_batch_copy_state": (ctypes.c_int, [_vp, _i32, _dp]),
     "dmv_batch_stats": (ctypes.c_int, [_vp, _i64p, _i64p, _i64p, _i32p, _dp]),
     "dmv_batch_debug_wait_limit": (ctypes.c_int, [_vp, _i64, _i32]),
+    "dmv_debug_batch_candidates": (ctypes.c_int, [_i32, _i32, _i32, _i32, _i32p, _i32p]),
     "dmv_debug_fail_allocations": (ctypes.c_int, [_i32]),
     "dmv_debug_tma_wait_limit": (ctypes.c_int, [_i64]),
     "dmv_debug_tc_convert": (ctypes.c_int, [_i32]),

@@ -590,6 +590,48 @@ int batch_run(dmv_batch_s* b, float* ms) {
 }  // namespace
 }  // namespace dmv
 
+namespace dmv {
+namespace {
+
+struct BatchConfig {
+  int32_t k, low, tpi;
+};
+
+// What the autotuner times: the configuration there is, first, then tile sizes,
+// low qubits and tiles per item around it. A rewritten batch has fixed-point
+// passes on tiles of 2^12 amplitudes only, so smaller ones are left out where a
+// circuit fills such a tile (64 circuits of 10 to 20 qubits: 6.6 ms, 12.9 and
+// 16.6 on tiles of 2^11 and 2^10), and its default of 4 low qubits is among
+// those tried (5: 6.7, 6: 6.9; with 1 tile per item 6.2, with 16 15.3).
+std::vector<BatchConfig> batch_candidates(int32_t precision, bool rewrite, int32_t max_qubits, const BatchConfig& now) {
+  std::vector<BatchConfig> c{now};
+  const bool full_only = rewrite && max_qubits >= 12;
+  for (int32_t k : {10, 11, 12, 13}) {
+    if (k > (precision == DMV_C128 ? 12 : 13) || (full_only && k < 12)) continue;
+    for (int32_t low : {4, 5, 6}) {
+      if (low == 4 && !rewrite) continue;
+      for (int32_t tpi : {1, 4, 16})
+        if (k != now.k || low != now.low || tpi != now.tpi) c.push_back({k, low, tpi});
+    }
+  }
+  return c;
+}
+
+// Planner settings of a new batch. The default arithmetic takes the single
+// states' rewrite and its tables (made once, on the device); the others apply
+// every fused 2x2 directly.
+bool batch_defaults(int32_t precision, int32_t arithmetic, PlanOptions& opt) {
+  const bool rewrite = precision == DMV_C128 && arithmetic == DMV_ARITH_FP64;
+  if (rewrite) {
+    opt.low_bits = 4;
+    opt.search_windows = true;
+  }
+  return rewrite;
+}
+
+}  // namespace
+}  // namespace dmv
+
 extern "C" int dmv_batch_create(int32_t num_circuits, const int32_t* num_qubits, const int64_t* gate_offsets,
                                 const dmv_gate_t* gates, int32_t precision, int32_t arithmetic, dmv_batch_t* out) {
   clear_error();
@@ -608,13 +650,7 @@ extern "C" int dmv_batch_create(int32_t num_circuits, const int32_t* num_qubits,
   dmv_batch_s* b = new dmv_batch_s();
   b->count = num_circuits;
   b->precision = precision;
-  // The default arithmetic takes the single states' rewrite and its tables (made
-  // once, on the device); the others apply every fused 2x2 directly.
-  b->rewrite = precision == DMV_C128 && arithmetic == DMV_ARITH_FP64;
-  if (b->rewrite) {
-    b->opt.low_bits = 4;
-    b->opt.search_windows = true;
-  }
+  b->rewrite = batch_defaults(precision, arithmetic, b->opt);
   b->arith = arithmetic == DMV_ARITH_FP64_DIRECT ? (int32_t)ARITH_FP64 : arithmetic;
   int64_t off = 0;
   for (int32_t c = 0; c < num_circuits; ++c) {
@@ -750,16 +786,12 @@ extern "C" int dmv_batch_autotune(dmv_batch_t b, int32_t* tile_bits, int32_t* lo
                                   double* best_ms) {
   clear_error();
   if (!b) return set_error(DMV_ERR_INVALID, "null batch");
-  const int max_tile = b->precision == DMV_C128 ? 12 : 13;
-  struct Cand { int k, low, tpi; };
-  std::vector<Cand> cands;
-  for (int k : {10, 11, 12, 13})
-    if (k <= max_tile)
-      for (int low : {5, 6})
-        for (int tpi : {1, 4, 16}) cands.push_back({k, low, tpi});
-  Cand best{b->opt.tile_bits, b->opt.low_bits, b->tiles_per_item};
+  const int32_t max_qubits = *std::max_element(b->n.begin(), b->n.end());
+  const std::vector<BatchConfig> cands =
+      batch_candidates(b->precision, b->rewrite, max_qubits, {b->opt.tile_bits, b->opt.low_bits, b->tiles_per_item});
+  BatchConfig best = cands[0];
   float best_t = 1e30f;
-  for (const Cand& c : cands) {
+  for (const BatchConfig& c : cands) {
     DMV_TRY(dmv_batch_configure(b, c.k, c.low, c.tpi));
     float t = 0.f;
     DMV_TRY(batch_run(b, &t));  // build + warm
@@ -774,6 +806,24 @@ extern "C" int dmv_batch_autotune(dmv_batch_t b, int32_t* tile_bits, int32_t* lo
   if (low_bits) *low_bits = best.low;
   if (tiles_per_item) *tiles_per_item = best.tpi;
   if (best_ms) *best_ms = best_t;
+  return DMV_OK;
+}
+
+extern "C" int dmv_debug_batch_candidates(int32_t precision, int32_t arithmetic, int32_t max_qubits, int32_t capacity,
+                                          int32_t* configs, int32_t* count) {
+  clear_error();
+  if (!configs || !count) return set_error(DMV_ERR_INVALID, "null output");
+  dmv_batch_s b;
+  const bool rewrite = batch_defaults(precision, arithmetic, b.opt);
+  const std::vector<BatchConfig> c =
+      batch_candidates(precision, rewrite, max_qubits, {b.opt.tile_bits, b.opt.low_bits, b.tiles_per_item});
+  if ((int32_t)c.size() > capacity) return set_error(DMV_ERR_INVALID, "room for %d of %zu", capacity, c.size());
+  *count = (int32_t)c.size();
+  for (size_t i = 0; i < c.size(); ++i) {
+    configs[3 * i] = c[i].k;
+    configs[3 * i + 1] = c[i].low;
+    configs[3 * i + 2] = c[i].tpi;
+  }
   return DMV_OK;
 }
 

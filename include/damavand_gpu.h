@@ -294,6 +294,12 @@ int dmv_batch_stats(dmv_batch_t b, int64_t* items, int64_t* passes, int64_t* ops
  * poison != 0, re-plans so one item waits for a count that never arrives; the
  * next run must then end with DMV_ERR_TIMEOUT instead of hanging. */
 int dmv_batch_debug_wait_limit(dmv_batch_t b, int64_t spin_limit, int32_t poison);
+/* Test hook (host only, no GPU): the configurations (tile bits, low bits,
+ * tiles per item; 3 values each, room for `capacity`) that dmv_batch_autotune
+ * times on a new batch whose largest circuit has max_qubits. No reference
+ * counterpart. */
+int dmv_debug_batch_candidates(int32_t precision, int32_t arithmetic, int32_t max_qubits, int32_t capacity,
+                               int32_t* configs, int32_t* count);
 /* Test hook: the next `count` device allocations of the library fail (as if
  * out of memory). */
 int dmv_debug_fail_allocations(int32_t count);
