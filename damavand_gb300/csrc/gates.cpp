@@ -249,6 +249,11 @@ Window next_window(const std::vector<SGate>& sg, const std::vector<int64_t>& pen
     if (!(first.local & qbit(q))) { first.local |= qbit(q); ++nlocal; }
   if (!search || k >= n) return first;
 
+  // A scan ends where every local qubit that a pending gate touches is blocked
+  // (one that none touches never is).
+  uint64_t touched = 0;
+  const uint64_t all = (uint64_t(1) << n) - 1;
+  for (size_t i = 0; i < pending.size() && touched != all; ++i) touched |= sg[(size_t)pending[i]].qs;
   const double pass_cost = n < kFewTilesQubits ? kPassCostFewTiles : kPassCost;
   Window best = first;
   double best_score = -1.0;
@@ -262,7 +267,7 @@ Window next_window(const std::vector<SGate>& sg, const std::vector<int64_t>& pen
     uint64_t blocked = 0;
     int32_t depth[64] = {};
     for (int64_t gi : pending) {
-      if (!(local & ~blocked)) break;  // every local qubit blocked
+      if (!(local & touched & ~blocked)) break;
       const SGate& g = sg[(size_t)gi];
       if ((g.qs & blocked) || !(local & g.target)) {
         blocked |= g.qs;
