@@ -272,3 +272,73 @@ bool build_fix_pass(const Op* ops, int64_t count, int32_t tile_bits, std::vector
 }
 
 }  // namespace dmv
+
+// ---------------------------------------------------------------------------
+// Host view of the scheduled passes (dmv_debug_fix_plan), for a test that runs
+// them next to the ops they come from.
+// ---------------------------------------------------------------------------
+extern "C" int dmv_debug_fix_plan(const dmv_gate_t* gates, int64_t num_gates, int32_t num_qubits, int32_t form,
+                                  int64_t capacity, int64_t* words, int64_t* count) {
+  using namespace dmv;
+  clear_error();
+  if (!words || !count || form < 0 || form > 2) return set_error(DMV_ERR_INVALID, "dmv_debug_fix_plan: bad arguments");
+  std::vector<Gate> g;
+  DMV_TRY(parse_gates(gates, num_gates, num_qubits, g));
+  dmv_state_s probe;
+  probe.n = num_qubits;
+  probe.precision = form == 2 ? DMV_C64 : DMV_C128;
+  PlanOptions opt = plan_options_for(&probe, DMV_FUSE_WINDOW, form == 1);
+  std::vector<int32_t> run_of, gen;
+  if (form == 1) {  // a gradient's windows, every gate's run measured
+    opt.tile_bits = 11;
+    opt.windows_only = true;
+    for (const Gate& x : g) gen.push_back(x.control < 0 ? 1 : 0);
+    opt.run_of = &run_of;
+    opt.generator_of = gen.data();
+  }
+  Plan plan;
+  DMV_TRY(build_plan(g, num_qubits, probe.precision, opt, plan));
+  std::vector<int64_t> w;
+  auto bits = [](double x) {
+    int64_t i;
+    std::memcpy(&i, &x, sizeof(i));
+    return i;
+  };
+  for (const Pass& ps : plan.passes) {
+    const int32_t k = ps.low_bits + ps.num_high;
+    if (ps.kind != 1 || k != opt.tile_bits) continue;
+    RewrittenPass r;
+    rewrite_pass_rotations(plan.ops.data() + ps.op_begin, ps.op_count, k, true, r.ops, r.tab, &r.scale, form == 2);
+    std::vector<FixOp> fops;
+    int32_t shifts = 0;
+    const bool taken = build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), k, fops, &shifts, nullptr, form == 2);
+    w.insert(w.end(), {ps.low_bits, ps.num_high});
+    w.insert(w.end(), ps.high, ps.high + ps.num_high);
+    w.insert(w.end(), {ps.op_count, taken ? 1 : 0, (int64_t)fops.size(), (int64_t)r.tab.tables.size(),
+                       (int64_t)r.tab.terms.size(), shifts, bits(r.scale.hi)});
+    for (int64_t o = 0; o < ps.op_count; ++o) {
+      const Op& op = plan.ops[(size_t)(ps.op_begin + o)];
+      w.insert(w.end(), {op.target, op.ctrl, op.ctrl_kind, op.param, op.generator});
+      for (double x : op.m) w.push_back(bits(x));
+    }
+    const size_t at = w.size();
+    w.push_back(0);  // measurements: the run of each (a FIX_GRAD's slot) and its frame
+    for (const Op& op : r.ops)
+      if (op.cls == OP_GRAD) {
+        int64_t frame;
+        std::memcpy(&frame, op.fh, sizeof(frame));
+        w.insert(w.end(), {op.param, frame});
+        ++w[at];
+      }
+    for (const FixOp& f : fops) {
+      w.push_back(f.kind);
+      w.insert(w.end(), f.a, f.a + 11);
+    }
+    for (const PhaseTable& t : r.tab.tables) w.insert(w.end(), {t.entry, t.c, t.first_term, t.num_terms, t.k, t.g});
+    for (const PhaseTerm& t : r.tab.terms) w.insert(w.end(), {(int64_t)t.mask, t.turn});
+  }
+  *count = (int64_t)w.size();
+  if (*count > capacity) return set_error(DMV_ERR_INVALID, "dmv_debug_fix_plan: %lld words", (long long)*count);
+  std::copy(w.begin(), w.end(), words);
+  return DMV_OK;
+}

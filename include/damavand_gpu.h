@@ -327,6 +327,20 @@ int dmv_debug_tma_wait_limit(int64_t polls);
  * reference counterpart. */
 int dmv_debug_check_fp64_rewrite(const dmv_gate_t* gates, int64_t num_gates, int32_t num_qubits, uint64_t seed,
                                  double* max_err, int64_t* counts);
+/* Test hook (host only, no GPU): the register-phase form of every full window
+ * pass of a gate list, as the kernels get it: form 0 complex128 fixed point
+ * (2^12 amplitudes), 1 the windows of a gradient (2^11, `gates` as the reversed
+ * list), 2 complex64 from 20 qubits. Per pass, in 64-bit words: low bits, number
+ * of high qubits, the high qubits; number of ops, 1 if the kernel takes the
+ * pass, numbers of register-phase ops, tables and terms, halvings, the factor
+ * product (double bits); the ops (target, control, its kind, run, generator, 8
+ * matrix entries as double bits); the number of measurements and for each its
+ * run and frame; the register-phase ops (12 words each); the tables (first
+ * entry, constant, first term, number of terms, tile bits, global bits); the
+ * terms (mask, turn). DMV_ERR_INVALID with *count set when `capacity` words do
+ * not hold it. No reference counterpart. */
+int dmv_debug_fix_plan(const dmv_gate_t* gates, int64_t num_gates, int32_t num_qubits, int32_t form, int64_t capacity,
+                       int64_t* words, int64_t* count);
 /* Test hook (host only, no GPU): plans the reverse sweep of an adjoint
  * gradient over `gates` (reversed, each gate's adjoint, unmerged, ops tagged
  * with parameter slots and generators, 2^12-amplitude windows) and writes 6
