@@ -34,6 +34,14 @@ constexpr int kAdjThreads = 256;
 constexpr int kAdjThreadBits = 8;
 constexpr int kAdjAmps = 8;
 constexpr int kAdjWarps = kAdjThreads / 32;
+// A tile is taken when a sixteenth of either state is within 2^kAdjSpread of its
+// largest component. The forward's stricter lines (FixScan) guard the norm of
+// the error, which 2^12 components of a concentrated tile share out; a gradient
+// is an inner product with the other state, and what 2^-57 M in every component
+// adds to it is that times the other's norm, however M is shared out. On states
+// around a product state, also with weights that vanish at its largest
+// amplitude, the gradients' errors against 64 bits are 0.3 to 1 times those of
+// the sweep in FP64 gate by gate.
 constexpr int kAdjSpread = 6;  // binary orders
 constexpr int kAdjGrads = 48;  // measurements per launch (a longer window runs as several launches)
 
