@@ -218,7 +218,7 @@ k_batch_fix(double2* __restrict__ arena, const BatchPass* __restrict__ passes, c
         r[2 * u] = v.x;
         r[2 * u + 1] = v.y;
       }
-      const FixScan scan = fix_scan(r, s_scan);
+      const FixScan scan = fix_scan<true>(r, s_scan);
       if (num_fix > 0 && scan.fixed(ps.sparse) && scan.heavy()) {
         fix_put(r, smem_raw, scan.emax());
         const int renorm = fix_run(r, smem_raw, stage, fops, num_fix, fix_tab, base, s_top);

@@ -217,6 +217,8 @@ struct FixScan {
 };
 
 // Over the CTA, of amplitudes raw (double bits); s: 5 x 8 words of shared memory.
+// MASS: for heavy(); the registers it needs cost the FP32-pair kernel 5 %.
+template <bool MASS>
 __device__ __forceinline__ FixScan fix_scan(const long long (&raw)[2 * kFixAmps], uint32_t (*s)[kFixThreads / 32]) {
   uint32_t mx = 0, mn = ~0u, any = 0, cnt = 0;
 #pragma unroll
@@ -234,23 +236,25 @@ __device__ __forceinline__ FixScan fix_scan(const long long (&raw)[2 * kFixAmps]
   mn = __reduce_min_sync(0xffffffffu, mn);
   any = __reduce_or_sync(0xffffffffu, any);
   cnt = __reduce_add_sync(0xffffffffu, cnt);
-  // the squares, in units of the warp's largest exponent: floats in [0, 2)
-  float q = 0.f;
-  const int unit = ((int)(mx >> 20) - 127) << 20;
+  uint32_t mass = 0;
+  if constexpr (MASS) {  // the squares, in units of the warp's largest exponent: floats in [0, 2)
+    float q = 0.f;
+    const int unit = ((int)(mx >> 20) - 127) << 20;
 #pragma unroll
-  for (int u = 0; u < kFixAmps; ++u) {
-    const int h = max((int)(raw[2 * u] >> 32) & 0x7FFFFFFF, (int)(raw[2 * u + 1] >> 32) & 0x7FFFFFFF);
-    const float f = __int_as_float(max(h - unit, 0) << 3);
-    q = fmaf(f, f, q);
+    for (int u = 0; u < kFixAmps; ++u) {
+      const int h = max((int)(raw[2 * u] >> 32) & 0x7FFFFFFF, (int)(raw[2 * u + 1] >> 32) & 0x7FFFFFFF);
+      const float f = __int_as_float(max(h - unit, 0) << 3);
+      q = fmaf(f, f, q);
+    }
+    mass = __reduce_add_sync(0xffffffffu, (uint32_t)(q * 65536.f));  // 2^9 2^2 2^16 at most
   }
-  uint32_t mass = __reduce_add_sync(0xffffffffu, (uint32_t)(q * 65536.f));  // 2^9 2^2 2^16 at most
   if ((threadIdx.x & 31) == 0) {
     const int w = (int)threadIdx.x >> 5;
     s[0][w] = mx;
     s[1][w] = mn;
     s[2][w] = any;
     s[3][w] = cnt;
-    s[4][w] = mass;
+    if constexpr (MASS) s[4][w] = mass;
   }
   __syncthreads();
   cnt = 0;
@@ -261,9 +265,11 @@ __device__ __forceinline__ FixScan fix_scan(const long long (&raw)[2 * kFixAmps]
     any |= s[2][w];
     cnt += s[3][w];
   }
-  mass = 0;
+  if constexpr (MASS) {
+    mass = 0;
 #pragma unroll
-  for (int w = 0; w < kFixThreads / 32; ++w) mass += s[4][w] >> min(2 * ((mx >> 20) - (s[0][w] >> 20)), 31u);
+    for (int w = 0; w < kFixThreads / 32; ++w) mass += s[4][w] >> min(2 * ((mx >> 20) - (s[0][w] >> 20)), 31u);
+  }
   return FixScan{mx, mn, any, cnt, mass};
 }
 

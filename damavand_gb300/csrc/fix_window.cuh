@@ -111,11 +111,11 @@ k_window_fix(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ F
       r[2 * u] = v.x;
       r[2 * u + 1] = v.y;
     }
-    const FixScan scan = fix_scan(r, s_scan);
+    constexpr bool MASS = std::is_same<FB, PolF64>::value;  // FP32 pairs round more coarsely than any fixed-point tile
+    const FixScan scan = fix_scan<MASS>(r, s_scan);
     const int emax = scan.emax();
     const bool zero = scan.zero();
-    // FP32 pairs round more coarsely than any fixed-point tile
-    const bool fixed = scan.fixed(fp.sparse) && (!std::is_same<FB, PolF64>::value || scan.heavy());
+    const bool fixed = scan.fixed(fp.sparse) && (!MASS || scan.heavy());
     int e_out = 0;
     const bool store = !zero;
     if (fixed) {
