@@ -409,6 +409,8 @@ k_window_phases(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   }
 }
 
+constexpr int kShallowOps = 8;  // the most that shallow_pass lets through
+
 template <typename P>
 __global__ void __launch_bounds__(kWindowThreads, 2)
 k_window_tma(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ TmaPassParams p) {
@@ -484,6 +486,17 @@ k_window_tma(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ T
       const G* tg = reinterpret_cast<const G*>(tile);
       for (int l = threadIdx.x; l < T; l += NT) tv[l] = cvt_in<P>(tg[l], e);
       __syncthreads();
+    } else if constexpr (!P::kBlockScaled) {
+      // A tile of zeros stays one. Looked for in passes of few ops, where that is
+      // most of the time on a state near |0...0>: in longer ones it costs 2 %.
+      if (num_ops <= kShallowOps) {
+        bool any = false;
+        for (int l = threadIdx.x; l < T; l += NT) any = any || any_bits(tv[l], tv[l]);
+        if (!__syncthreads_or(any)) {
+          if (mover && next < num_tiles) geom.load(&tmap, &s_bar, tile, next, boxes, tile_bytes, lane);
+          continue;
+        }
+      }
     }
     tile_apply_ops<P>(tv, T, ops, num_ops, base, p.phase_tab);
     if constexpr (P::kBlockScaled) tile_store_fx(tv, amps, base, T, t_off, s_slot, e);
@@ -859,6 +872,19 @@ int make_phase_tables(const PhaseTables& tabs, const std::vector<FixOp>& fix_ops
   return DMV_OK;
 }
 
+// A rewritten FP64 pass of so few ops that k_window_tma's arithmetic in FP64
+// fits into the time k_window_fix spends on a tile before its first op (reading,
+// scanning, converting and writing it: 640 us at 26 qubits, 320 of them HBM).
+// There a rotation or table takes 270 to 400 us in FP64 and 80 to 220 in fixed
+// point, an exchange 40 and nothing. Measured, FP64 against fixed point: one
+// table 570 and 860 us, two rotations 670 and 860, three 950 and 940, two
+// exchanges 370 and 640, eight 630 and 630; the same ratios from 13 qubits on.
+bool shallow_pass(const std::vector<Op>& ops) {
+  size_t cost = 0;
+  for (const Op& op : ops) cost += op.cls == OP_SWAP ? 3 : 10;
+  return cost <= 3 * kShallowOps;
+}
+
 // FP32-pair states: the least product of rotation factors a state or a pass
 // leaves out.
 constexpr double kPairScale = 0x1p-40;
@@ -918,7 +944,7 @@ int launch_plan_form(dmv_state_s* s, const Plan& plan, bool rewritten_form) {
       // complex64 states and FP32 pairs hold the unscaled values of a pass only to 2^40
       const bool in_range = (fix && rot_ops) || r.scale.hi >= kPairScale;
       const bool eligible = single ? tma_eligible<PolF32>(ps) : tma_eligible<PolF64>(ps);
-      fixed = in_range && eligible &&
+      fixed = in_range && eligible && !(!single && rot_ops && shallow_pass(r.ops)) &&
               build_fix_pass(r.ops.data(), (int64_t)r.ops.size(), 12, s->fix_ops, &shifts, &sparse, single);
       if (single && !fixed) rewritten_at[pi] = -1;  // its gates as complex 2x2s
       if (!single && !rot_ops && !fixed) {  // FP32 pairs outside the fixed-point kernel: rotations as real 2x2 ops
