@@ -283,8 +283,7 @@ int copy_in(dmv_state_s* s, const double* re, const double* im, const double* in
 
 int apply_gate_list(dmv_state_s* s, const std::vector<Gate>& gates, int32_t fusion) {
   Plan plan;
-  const PlanOptions opt = plan_options_for(s, fusion);
-  DMV_TRY(build_plan(gates, s->n, s->precision, opt, plan));
+  DMV_TRY(plan_for(s, gates, fusion, plan));
   return launch_plan(s, plan);
 }
 
@@ -603,7 +602,8 @@ extern "C" int dmv_plan_describe(int32_t num_qubits, int32_t precision, const dm
   PlanOptions opt = plan_options_for(&probe, fusion);
   if (tile_bits > 0) opt.tile_bits = tile_bits;
   Plan plan;
-  DMV_TRY(build_plan(parsed, num_qubits, precision, opt, plan));
+  if (tile_bits > 0) DMV_TRY(build_plan(parsed, num_qubits, precision, opt, plan));
+  else DMV_TRY(plan_for(&probe, parsed, fusion, plan));
   int64_t windows = 0;
   int32_t max_local = 0;
   for (const Pass& p : plan.passes) {

@@ -268,6 +268,7 @@ struct Plan {
   std::vector<Pass> passes;
   std::vector<Op> ops;
   int64_t num_gates = 0;
+  bool as_is = false;  // complex64: its passes run as 2x2 matrices, not rewritten
 };
 
 struct PlanOptions {
@@ -515,6 +516,34 @@ inline PlanOptions plan_options_for(const dmv_state_s* s, int32_t fusion, bool s
     opt.low_bits = 6;  // rows of 512 and 1024 bytes
   }
   return opt;
+}
+
+// complex64 lists of a few gates from kSearchQubits qubits on, if one pass over
+// the first targets' qubits holds them: a table among them costs a rewritten
+// pass a launch and a phase, and with rows of 128 bytes a pass moves the state
+// at 0.87 of the rate of rows of 512. Rewritten and as they are: four Hadamards
+// 19.2 and 14.0 us at 20 qubits, 67.7 and 57.8 at 24, 800 and 699 at 28; six
+// 19.6 and 15.5, 76.9 and 78.6, 959 and 1029.
+constexpr int64_t kFewGates = 4, kFewGatesSmall = 8;
+constexpr int32_t kFewGatesSmallQubits = 22;  // fewer: the launches decide
+// The plan of a gate list on a state.
+inline int plan_for(const dmv_state_s* s, const std::vector<Gate>& gates, int32_t fusion, Plan& plan) {
+  if (s->precision == DMV_C64 && s->n >= kSearchQubits && gates.size() <= 64) {
+    PlanOptions opt;
+    opt.fusion = fusion;
+    DMV_TRY(build_plan(gates, s->n, s->precision, opt, plan));
+    bool tables = false;
+    for (const Op& op : plan.ops) {  // exchanges and rotations [[c, -s], [s, c]], 0 < s <= c, leave none
+      const bool rotation = op.cls == OP_REAL && op.m[0] == op.m[6] && op.m[2] == -op.m[4] && op.m[4] > 0.0 &&
+                            op.m[0] >= op.m[4];
+      tables = tables || (op.cls != OP_SWAP && !rotation);
+    }
+    plan.as_is = plan.passes.size() == 1 && tables &&
+                 (int64_t)plan.ops.size() <= (s->n < kFewGatesSmallQubits ? kFewGatesSmall : kFewGates);
+    if (plan.as_is) return DMV_OK;
+  }
+  plan.as_is = false;
+  return build_plan(gates, s->n, s->precision, plan_options_for(s, fusion), plan);
 }
 
 // Kernel launchers (kernels_*.cu). All stream-ordered on s->stream.

@@ -907,7 +907,7 @@ int launch_plan_form(dmv_state_s* s, const Plan& plan, bool rewritten_form) {
   const bool rewrite = rewritten_form && c128 &&
                        ((s->arith == ARITH_FP64 && s->fp64_rewrite) || s->arith == ARITH_FP32X2 ||
                         s->arith == ARITH_INT64);
-  const bool single = rewritten_form && !c128 && s->n >= kSearchQubits;  // complex64 passes as rotations and tables
+  const bool single = rewritten_form && !c128 && !plan.as_is && s->n >= kSearchQubits;  // complex64 passes as rotations and tables
   const bool rot_ops = single || s->arith == ARITH_FP64;
   const bool fix = rewrite && s->arith != ARITH_INT64 && s->n >= 12;  // fixed-point passes where the kernel takes them
   s->phase_tabs = PhaseTables();

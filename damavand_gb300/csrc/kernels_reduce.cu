@@ -1677,8 +1677,7 @@ int adjoint_gradient(dmv_state_s* s, const std::vector<Gate>& gates, const doubl
   // Forward from |0...0> with the fused plan.
   DMV_TRY(launch_set_zero(s));
   Plan plan;
-  const PlanOptions opt = plan_options_for(s, DMV_FUSE_WINDOW);
-  DMV_TRY(build_plan(gates, s->n, s->precision, opt, plan));
+  DMV_TRY(plan_for(s, gates, DMV_FUSE_WINDOW, plan));
   DMV_TRY(launch_plan(s, plan));
   std::vector<double> ez((size_t)s->n);
   DMV_TRY(launch_expect_z(s, ez.data(), nullptr));

@@ -73,3 +73,28 @@ def test_non_finite_tile_stays_apart(built_lib, oracle_mod):
     assert fp64 and not np.all(np.isfinite(got[:part]))
     assert np.count_nonzero(got[part:2 * part]) == 0
     assert np.max(np.abs(got[2 * part:] - want[2 * part:])) <= 4 * 2.0 ** -53 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("n,count,as_is", [(20, 4, True), (20, 8, True), (20, 9, False), (21, 8, True), (22, 4, True),
+                                           (22, 5, False), (24, 4, True)])
+@pytest.mark.parametrize("kind", ["h", "rz"])
+def test_complex64_lists_of_few_gates(built_lib, oracle_mod, n, count, as_is, kind):
+    """On both sides of the line between a rewritten pass (it has tables) and the gates as they are."""
+    q = [n - 1, 0, n - 2, 7, n - 3, 1, n // 2, 2, 3]
+    gates = [(H if kind == "h" else RZ, q[i], -1, False, 0.0 if kind == "h" else 0.3 + 0.1 * i) for i in range(count)]
+    if count > 4:
+        gates = gates[:-1] + [(CNOT, q[1], q[0], False, 0.0)]
+    psi = random_state(n, np.random.default_rng(n))
+    st = new_state(n, 1)
+    try:
+        load_state(st, psi)
+        from damavand_gb300._lib import check, lib
+        apply_gates(st, gates, 1)
+        total, terms = ctypes.c_int64(), ctypes.c_int64()
+        check(lib.dmv_last_upload_bytes(st.handle, ctypes.byref(total), ctypes.byref(terms)))
+        got = st.numpy().astype(np.complex128)
+    finally:
+        free_state(st)
+    assert (terms.value == 0) == as_is
+    want = oracle_forward_any_control(oracle_mod, n, gates, psi)
+    assert np.max(np.abs(got - want)) <= 2 * len(gates) * 2.0 ** -24 * np.max(np.abs(want))
