@@ -281,9 +281,11 @@ struct dmv_batch_s {
   cudaStream_t stream = nullptr;
   DeviceBuffer passes_dev, items_dev, ops_dev, counters_dev, offsets_dev, reduce_dev;
   // Pauli-Z reductions: reduce_dev holds the sums (one column per circuit and qubit, and its total), then the
-  // partials; mass_dev the circuits' BatchMass and the circuit of each CTA and column.
+  // partials; mass_dev the BatchMass of the circuits that share a pass and the circuit of each CTA and column of theirs.
   DeviceBuffer mass_dev;
-  int32_t mass_ctas = 0, mass_columns = 0;
+  int32_t mass_count = 0, mass_ctas = 0, shared_columns = 0, mass_columns = 0;
+  std::vector<int32_t> first_column;              // of each circuit; those of the shared pass come first
+  std::vector<std::pair<int32_t, int64_t>> own_mass;  // circuits with a pass of their own, and its partials
   int64_t num_items = 0, num_passes = 0, num_ops = 0;
   int32_t max_k = 0;
   PlanOptions opt;
@@ -536,11 +538,17 @@ int batch_enqueue(dmv_batch_s* b) {
     else DMV_TRY(batch_launch_kernel<PolF64>(b));
   }
   double* red = static_cast<double*>(b->reduce_dev.ptr);
-  const char* md = static_cast<const char*>(b->mass_dev.ptr);
-  const int32_t* of_cta = reinterpret_cast<const int32_t*>(md + (size_t)b->count * sizeof(BatchMass));
-  DMV_TRY(launch_batch_mass(reinterpret_cast<const BatchMass*>(md), of_cta, b->mass_ctas, of_cta + b->mass_ctas,
-                            b->mass_columns, b->arena, b->precision == DMV_C128 ? 0 : 1, red + b->mass_columns, red,
+  const int kind = b->precision == DMV_C128 ? 0 : 1;
+  for (const auto& own : b->own_mass)
+    DMV_TRY(launch_own_mass(static_cast<const char*>(b->arena) + (size_t)b->offsets[(size_t)own.first] * b->amp_size(),
+                            kind, b->n[(size_t)own.first], red + own.second, red + b->first_column[(size_t)own.first],
                             b->stream));
+  if (b->mass_count > 0) {
+    const char* md = static_cast<const char*>(b->mass_dev.ptr);
+    const int32_t* of_cta = reinterpret_cast<const int32_t*>(md + (size_t)b->mass_count * sizeof(BatchMass));
+    DMV_TRY(launch_batch_mass(reinterpret_cast<const BatchMass*>(md), of_cta, b->mass_ctas, of_cta + b->mass_ctas,
+                              b->shared_columns, b->arena, kind, red + b->mass_columns, red, b->stream));
+  }
   return DMV_OK;
 }
 
@@ -592,6 +600,12 @@ int batch_run(dmv_batch_s* b, float* ms) {
 
 namespace dmv {
 namespace {
+
+// Circuits of this many qubits have a Pauli-Z mass pass of their own, staged by
+// bulk copies: they fill the chip, and the shared pass's plain loads are slower.
+// One circuit of one gate in complex64, shared and own pass: 104 and 112 us at
+// 23 qubits, 188 and 172 at 24, 1238 and 973 at 27.
+constexpr int32_t kOwnMassQubits = 24;
 
 struct BatchConfig {
   int32_t k, low, tpi;
@@ -696,24 +710,38 @@ extern "C" int dmv_batch_create(int32_t num_circuits, const int32_t* num_qubits,
       break;
     }
     std::vector<BatchMass> mass;
-    std::vector<int32_t> of;  // the circuit of each CTA, then of each column
-    int64_t red = 0;
+    std::vector<int32_t> of;  // of the shared pass: the circuit of each CTA, then of each column
+    int64_t red = 0;          // partials, after the sums
+    b->first_column.assign((size_t)num_circuits, 0);
     for (int32_t c = 0; c < num_circuits; ++c) {
       const int32_t n = b->n[(size_t)c];
+      if (n >= kOwnMassQubits) continue;
       const int32_t ctas = batch_mass_ctas(n);
+      b->first_column[(size_t)c] = b->mass_columns;
       mass.push_back(BatchMass{b->offsets[(size_t)c], red, n, b->mass_ctas, ctas, b->mass_columns});
       red += (int64_t)ctas * (n + 1);
       b->mass_ctas += ctas;
       b->mass_columns += n + 1;
-      of.insert(of.end(), (size_t)ctas, c);
+      of.insert(of.end(), (size_t)ctas, b->mass_count++);
     }
-    for (int32_t c = 0; c < num_circuits; ++c) of.insert(of.end(), (size_t)b->n[(size_t)c] + 1, c);
+    b->shared_columns = b->mass_columns;
+    for (int32_t m = 0; m < b->mass_count; ++m) of.insert(of.end(), (size_t)mass[(size_t)m].n + 1, m);
+    for (int32_t c = 0; c < num_circuits; ++c) {
+      const int32_t n = b->n[(size_t)c];
+      if (n < kOwnMassQubits) continue;
+      b->first_column[(size_t)c] = b->mass_columns;
+      b->mass_columns += n + 1;
+      b->own_mass.push_back({c, red});
+      red += own_mass_partials(precision == DMV_C128 ? 0 : 1, n);
+    }
+    for (auto& own : b->own_mass) own.second += b->mass_columns;
     if ((rc = b->reduce_dev.reserve((size_t)(red + b->mass_columns) * sizeof(double))) != DMV_OK) break;
     const size_t mb = mass.size() * sizeof(BatchMass);
     if ((rc = b->mass_dev.reserve(mb + of.size() * sizeof(int32_t))) != DMV_OK) break;
-    if (cudaMemcpy(b->mass_dev.ptr, mass.data(), mb, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(static_cast<char*>(b->mass_dev.ptr) + mb, of.data(), of.size() * sizeof(int32_t),
-                   cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (b->mass_count > 0 &&
+        (cudaMemcpy(b->mass_dev.ptr, mass.data(), mb, cudaMemcpyHostToDevice) != cudaSuccess ||
+         cudaMemcpy(static_cast<char*>(b->mass_dev.ptr) + mb, of.data(), of.size() * sizeof(int32_t),
+                    cudaMemcpyHostToDevice) != cudaSuccess)) {
       rc = set_error(DMV_ERR_CUDA, "reduction plan upload failed");
       break;
     }
@@ -831,14 +859,15 @@ extern "C" int dmv_batch_expect_z(dmv_batch_t b, double* out) {
   clear_error();
   if (!b || !out) return set_error(DMV_ERR_INVALID, "null batch or output");
   DMV_CUDA_TRY(cudaStreamSynchronize(b->stream));
+  if (!b->own_mass.empty()) DMV_TRY(check_window_status());  // a mass pass whose chunk load wait gave up
   std::vector<double> h((size_t)b->mass_columns);
   DMV_CUDA_TRY(cudaMemcpy(h.data(), b->reduce_dev.ptr, h.size() * sizeof(double), cudaMemcpyDeviceToHost));
-  int64_t pos = 0, col = 0;
+  int64_t pos = 0;
   for (int32_t c = 0; c < b->count; ++c) {
     const int n = b->n[(size_t)c];
-    for (int q = 0; q < n; ++q) out[pos + q] = h[(size_t)(col + n)] - 2.0 * h[(size_t)(col + q)];
+    const double* m = h.data() + b->first_column[(size_t)c];
+    for (int q = 0; q < n; ++q) out[pos + q] = m[n] - 2.0 * m[q];
     pos += n;
-    col += n + 1;
   }
   return DMV_OK;
 }

@@ -581,7 +581,12 @@ uint32_t tma_wait_limit();
 // The device word those waits set to 1 when they give up.
 int* tma_status_word();
 
-// Pauli-Z mass reduction of every circuit of a batch in one pass: circuit c's
+// The Pauli-Z mass pass of one state (bulk-staged) into caller-provided device
+// buffers: `partial` holds own_mass_partials doubles, `sums` the n + 1 sums. The
+// first call for a kind is not made inside a capture.
+int64_t own_mass_partials(int src_kind, int n);
+int launch_own_mass(const void* src, int src_kind, int n, double* partial, double* sums, cudaStream_t stream);
+// The same for many circuits of a batch in one pass: circuit c's
 // CTAs first_cta .. + ctas leave n + 1 sums each at `partial`, and columns
 // first_column .. + n of `sums` get the mass with bit q set (q < n), then the total.
 struct BatchMass {

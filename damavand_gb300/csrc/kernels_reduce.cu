@@ -1437,6 +1437,24 @@ int batch_mass_ctas(int n) {
   return (int)std::min<int64_t>(chunks, (int64_t)sm_count() * 8);
 }
 
+int64_t own_mass_partials(int src_kind, int n) {
+  if (src_kind == 0) mass_bulk_attributes<0>();
+  else mass_bulk_attributes<1>();
+  tma_status_word();
+  return (int64_t)mass_grid_for(src_kind, n, int64_t(1) << (n - mass_chunk_bits_for(n))) * (n + 1);
+}
+
+int launch_own_mass(const void* src, int src_kind, int n, double* partial, double* sums, cudaStream_t stream) {
+  const int cb = mass_chunk_bits_for(n);
+  const int64_t num_chunks = int64_t(1) << (n - cb);
+  const int grid = mass_grid_for(src_kind, n, num_chunks);
+  launch_mass_kernel(src, src_kind, n, cb, num_chunks, grid, partial, stream);
+  k_reduce_partials<<<n + 1, kPartialThreads, 0, stream>>>(partial, n + 1, grid, sums);
+  count_launch(2);
+  DMV_CUDA_TRY(cudaGetLastError());
+  return DMV_OK;
+}
+
 int launch_batch_mass(const BatchMass* circuits, const int32_t* circuit_of_cta, int ctas, const int32_t* circuit_of_column,
                       int columns, const void* arena, int src_kind, double* partial, double* sums,
                       cudaStream_t stream) {
