@@ -58,10 +58,11 @@ enum { DMV_C128 = 0, DMV_C64 = 1 };
  *   a scaled matrix (the product of the scale factors is multiplied back into
  *   the state once per forward) and collect the diagonals of a pass into a few
  *   per-amplitude phase tables. Tiles of 2^12 amplitudes within 2^12 of one
- *   another run in 64-bit fixed point, 57 bits for the tile's largest
- *   component, one rounding per output; every other tile (and pass, and state
- *   below 12 qubits) in IEEE FP64. Measured errors against 64-bit values are
- *   below those of FP64 throughout.
+ *   another, and not dominated by a few, run in 64-bit fixed point, 57 bits for
+ *   the tile's largest component, one rounding per output (zeros stay exact
+ *   zeros); every other tile (and pass with other ops or with very few, and
+ *   state below 12 qubits) in IEEE FP64. Measured errors against 64-bit values
+ *   are below those of FP64 throughout.
  * DMV_ARITH_FP64_DIRECT: IEEE FP64 with every fused 2x2 applied as a full
  *   complex multiply-add (8 per amplitude for a general matrix).
  * The FP32-pair and int64 arithmetics below take the same rewrite of their
@@ -69,8 +70,8 @@ enum { DMV_C128 = 0, DMV_C64 = 1 };
  * DMV_ARITH_FP32X2: the FP64 amplitudes are split into FP32 pairs (about 48
  *   significant bits) inside each kernel and combined with error-free
  *   transformations, then stored back as FP64; GB300 runs FP32 ~71x faster
- *   than FP64. Tiles that DMV_ARITH_FP64 would run in fixed point do so here
- *   as well. Where all passes of a gate list are in pairs the state keeps that
+ *   than FP64. Tiles of 2^12 amplitudes within 2^12 of one another run in the
+ *   fixed point of DMV_ARITH_FP64. Where all passes of a gate list are in pairs the state keeps that
  *   form between them (the same 16 bytes per amplitude); it is IEEE complex128
  *   again when the call returns. Measured error on deep circuits below 1e-13
  *   normwise.
