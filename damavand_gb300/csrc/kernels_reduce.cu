@@ -842,7 +842,9 @@ __global__ void k_chunk_guide(const double* __restrict__ incl, int64_t num_chunk
 // The levels' sums round differently. Where no segment of the chunk reaches
 // u*total, the last one of nonzero mass is taken (the chunk has some: its prefix
 // is above its predecessor's); where no element of nonzero probability of the
-// segment does, the last such element.
+// segment does, the last such element. Compared by bits (scan_less; a total that
+// is not a number has left before): on the FP64 pipe the 16 comparisons of a
+// lane's elements made 2^17 samples 599 us instead of 452.
 template <int SRC>
 __global__ void __launch_bounds__(kRedThreads)
 k_sample_warp(const void* src, int seg_bits, int chunk_bits, int64_t num_chunks, const double* __restrict__ chunk_incl,
@@ -878,8 +880,8 @@ k_sample_warp(const void* src, int seg_bits, int chunk_bits, int64_t num_chunks,
     const double* sp = seg_incl + lo * spc;
     const double mine_sp = sp[lane < spc ? lane : 0];
     const double prev_sp = __shfl_up_sync(0xffffffffu, mine_sp, 1);
-    const unsigned segs = __ballot_sync(0xffffffffu, lane < spc && xsi <= before + mine_sp);
-    const unsigned some = __ballot_sync(0xffffffffu, lane < spc && mine_sp > (lane > 0 ? prev_sp : 0.));
+    const unsigned segs = __ballot_sync(0xffffffffu, lane < spc && !scan_less(before + mine_sp, xsi));
+    const unsigned some = __ballot_sync(0xffffffffu, lane < spc && scan_less(lane > 0 ? prev_sp : 0., mine_sp));
     const int sg = segs ? __ffs((int)segs) - 1 : some ? 31 - __clz((int)some) : spc - 1;
     const double sbefore = sg > 0 ? before + sp[sg - 1] : before;
     const int64_t base = ((lo * spc + sg) << seg_bits) + (int64_t)lane * E;
@@ -904,8 +906,9 @@ k_sample_warp(const void* src, int seg_bits, int chunk_bits, int64_t num_chunks,
     for (int e = 0; e < 8; ++e) {
       if (e < mine) {
         run += p[e];
-        if (p[e] > 0.) last_nz = e;
-        if (hit < 0 && p[e] > 0. && xsi <= run) hit = e;
+        const bool nz = scan_less(0., p[e]);
+        if (nz) last_nz = e;
+        if (hit < 0 && nz && !scan_less(run, xsi)) hit = e;
       }
     }
     const unsigned hits = __ballot_sync(0xffffffffu, hit >= 0);
